@@ -1,245 +1,245 @@
-// Batched complex FP64 GEMM (plain form).  B200 has no FP64 tcgen05 path, and
-// its FP64 DMMA rate equals its DFMA rate, so this kernel register-tiles the
-// complex multiply-adds on the FP64 pipe: each thread owns a TMxTN block of
-// the output, operand tiles are staged through shared memory (double
-// buffered), and column-major stores are coalesced along the row index.
+// Batched complex FP64 GEMM (plain form) on the FP64 matrix instruction
+// (mma.sync.m8n8k4.f64).  tcgen05 has no FP64 kind; the warp-level FP64
+// product runs at the rate of the FP64 pipe (37.0 TFLOP/s measured, against
+// 33.9 for a bare chain of DFMAs), and its fragments take each operand value
+// from shared memory once per warp: a 32 x 16 complex warp tile reads 3 KB
+// per 512 matrix-pipe cycles, where the register-tiled DFMA form before it was
+// bound by its fragment loads.  One B200, before and after: M-build (16384 x
+// 2048 x 640, real A) 4.14 -> 2.83 ms (30.3 TFLOP/s), exchange of n = 128, 32
+// electrons, 640 vectors and 2048 walkers 17.1 -> 10.7 ms, one-body product
+// of 1024 128 x 56 walkers 0.465 -> 0.27 ms.
 #include "zgemm.cuh"
-
-#include <cuda_bf16.h>
 
 #include <atomic>
 #include <map>
 #include <mutex>
 #include <tuple>
 
+#include "dmma.cuh"
+#include "once.cuh"
+
 extern std::atomic<long long> g_launch_count;
 
 namespace {
 
-constexpr int BK = 8;
+template <bool REAL> struct Elem { typedef zd T; };
+template <> struct Elem<true> { typedef double T; };
 
-template <int OP>
-__device__ __forceinline__ zd load_op(const void *P, long long ld, int i, int l, int kind,
-                                      long long plane)
-{
-    // element (i, l) of op(P) where P is column-major with leading dimension ld
-    long long idx = (OP == OP_N) ? (long long)i + (long long)l * ld : (long long)l + (long long)i * ld;
-    zd v;
-    if (kind == ST_R64) v = make_double2(__ldg((const double *)P + idx), 0.0);
-    else if (kind == ST_C32P) v = make_double2((double)__ldg((const float *)P + idx),
-                                               (double)__ldg((const float *)P + plane + idx));
-    else v = __ldg((const zd *)P + idx);
-    if (OP == OP_C) v.y = -v.y;
-    return v;
-}
+// One operand's tile: R rows (its m or n extent) by BK of the contraction.
+// KC: the contraction index is the contiguous one in memory.  The shared
+// layout keeps memory's order, so that neighbouring threads copy neighbouring
+// elements, and its leading dimension makes a fragment load (8 rows x 4 k)
+// touch every bank once: 4 mod 8 (complex) or 4 / 12 mod 16 (real) elements
+// with k contiguous, 2 mod 8 or 4 mod 16 with the rows contiguous.
+template <int R, int BK, bool KC, bool REAL>
+struct TileLayout {
+    typedef typename Elem<REAL>::T T;
+    static constexpr int LD = KC ? BK + 4 : R + (REAL ? 4 : 2);
+    static constexpr int COUNT = KC ? R * LD : BK * LD;
+    static constexpr size_t BYTES = (COUNT * sizeof(T) + 15) / 16 * 16;
+    static __device__ __forceinline__ int at(int r, int k) { return KC ? r * LD + k : k * LD + r; }
+};
 
-// REAL: 0 both operands complex (a real operand is loaded as complex with a
-// zero imaginary part), 1 A real, 2 B real, 3 both real; a real operand
-// takes one FP64 multiply-add per real product instead of the complex four.
-template <int BM, int BN, int TM, int TN, int OPA, int OPB, int REAL>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN), TM * TN > 16 ? 1 : 2)
+// REAL: 0 both operands complex, 1 A real, 2 B real, 3 both real; a real
+// operand takes two real products per complex one in place of four.
+template <int BM_, int BN_, int WM_, int WN_, int BK_, int STAGES_, int MINB_>
+struct Tile {
+    static constexpr int BM = BM_, BN = BN_, WM = WM_, WN = WN_, BK = BK_, STAGES = STAGES_, MINB = MINB_;
+    static constexpr int NT = 32 * (BM / WM) * (BN / WN);
+};
+
+template <class TL, int OPA, int OPB, int REAL>
+struct GemmShape {
+    typedef TileLayout<TL::BM, TL::BK, OPA != OP_N, (REAL & 1) != 0> LA;
+    typedef TileLayout<TL::BN, TL::BK, OPB == OP_N, (REAL & 2) != 0> LB;
+    static constexpr size_t STAGE = LA::BYTES + LB::BYTES;
+    static constexpr size_t SMEM = STAGE * TL::STAGES;
+};
+
+template <int R, int BK, int NT, bool KC, bool REAL>
+struct Loader {
+    typedef TileLayout<R, BK, KC, REAL> L;
+    typedef typename L::T T;
+    static constexpr int N = R * BK / NT;   // elements per thread
+    static_assert(R * BK % NT == 0 && (KC ? NT % BK == 0 : (NT % R == 0 || R % NT == 0)), "tile split");
+    const T *base;
+    const T *safe;
+    long long ld;
+    int r0, k0, rows, K;
+
+    __device__ __forceinline__ Loader(const void *P, long long ld_, int tile, int ext, int K_)
+    {
+        const int t = threadIdx.x;
+        // thread t's first element; the t-th of its N is rstep / kstep further
+        k0 = KC ? t % BK : t / R;
+        r0 = KC ? t / BK : t % R;
+        ld = ld_;
+        rows = ext - tile;
+        K = K_;
+        safe = (const T *)P;
+        base = (const T *)P + (KC ? (long long)(tile + r0) * ld + k0 : (long long)k0 * ld + tile + r0);
+    }
+    // tile number kt of the contraction into the stage at `dst`
+    __device__ __forceinline__ void load(unsigned dst, int kt) const
+    {
+        const T *p = base + (KC ? (long long)kt * BK : (long long)kt * BK * ld);
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const int dr = KC ? i * (NT / BK) : (R > NT ? (i % (R / NT)) * NT : 0);
+            const int dk = KC ? 0 : (R > NT ? i / (R / NT) : i * (NT / R));
+            const bool ok = r0 + dr < rows && kt * BK + k0 + dk < K;
+            const T *q = p + (KC ? (long long)dr * ld : (long long)dk * ld + dr);
+            cp_async_elem<(int)sizeof(T)>(dst + (unsigned)(L::at(r0 + dr, k0 + dk) * sizeof(T)), ok ? q : safe, ok);
+        }
+    }
+};
+
+// C_b = alpha op(A_b) op(B_b) + beta C_b, one BM x BN tile per CTA, BK columns
+// of the contraction per stage, STAGES cp.async stages in flight.  Each warp
+// owns a WM x WN block as 8 x 8 accumulator fragments; a fragment row or
+// column that lies outside C takes no products, so a ragged edge costs its
+// 8-row granule only.
+template <class TL, int OPA, int OPB, int REAL>
+__global__ void __launch_bounds__(TL::NT, TL::MINB)
 zgemm_kernel(ZGemmArgs a)
 {
-    constexpr int NTX = BM / TM;           // threads along rows
-    constexpr int NT = (BM / TM) * (BN / TN);
+    constexpr int BM = TL::BM, BN = TL::BN, WM = TL::WM, WN = TL::WN, BK = TL::BK, ST = TL::STAGES, NT = TL::NT;
+    constexpr int MI = WM / 8, NI = WN / 8;
+    constexpr bool RA = (REAL & 1) != 0, RB = (REAL & 2) != 0;
+    typedef GemmShape<TL, OPA, OPB, REAL> SH;
+    typedef typename SH::LA LA;
+    typedef typename SH::LB LB;
     const int b = blockIdx.z;
     if (a.mask && a.mask[b] == 0) return;
-    if (a.skip && a.skip[b] != 0) return;
     const int tileM = blockIdx.x * BM, tileN = blockIdx.y * BN;
-    if (tileM >= a.m || tileN >= a.n) return;
     if (a.lower && tileM + BM <= tileN) return;
 
-    const size_t esA = a.a_real == ST_R64 ? sizeof(double) : a.a_real == ST_C32P ? sizeof(float) : sizeof(zd);
-    const size_t esB = a.b_real == ST_R64 ? sizeof(double) : a.b_real == ST_C32P ? sizeof(float) : sizeof(zd);
-    const char *Ab = (const char *)a.A + (size_t)b * a.strideA * esA;
-    const char *Bb = (const char *)a.B + (size_t)b * a.strideB * esB;
-    zd *Cb = a.C ? a.C + (size_t)b * a.strideC : nullptr;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const unsigned smem0 = (unsigned)__cvta_generic_to_shared(smem);
+    const char *Ab = (const char *)a.A + (size_t)b * a.strideA * sizeof(typename LA::T);
+    const char *Bb = (const char *)a.B + (size_t)b * a.strideB * sizeof(typename LB::T);
+    const Loader<BM, BK, NT, OPA != OP_N, RA> la(Ab, a.lda, tileM, a.m, a.k);
+    const Loader<BN, BK, NT, OPB == OP_N, RB> lb(Bb, a.ldb, tileN, a.n, a.k);
 
-    __shared__ zd As[2][BK][BM];
-    __shared__ zd Bs[2][BK][BN];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int wm = (warp % (BM / WM)) * WM, wn = (warp / (BM / WM)) * WN;
+    const int fr = lane >> 2, fk = lane & 3;
+    // fragments of this warp that meet C
+    const int mb = (a.m - tileM - wm + 7) / 8, nb = (a.n - tileN - wn + 7) / 8;
 
-    const int tid = threadIdx.x;
-    // a warp covers 8 row and 4 column positions of the 16 x 16 thread grid,
-    // so each operand fragment load touches 8 (A) or 4 (B) distinct 16-byte
-    // words: one shared-memory wavefront each
-    static_assert(NTX == 16 && NT == 256, "16 x 16 thread grid");
-    const int warp = tid >> 5, lane = tid & 31;
-    const int tx = (warp & 1) * 8 + (lane & 7), ty = (warp >> 1) * 4 + (lane >> 3);
+    double cr[MI][NI][2], ci[MI][NI][2];
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NI; ++j) cr[i][j][0] = cr[i][j][1] = ci[i][j][0] = ci[i][j][1] = 0.0;
 
-    zd acc[TM][TN];
+    const int KT = (a.k + BK - 1) / BK;
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = make_double2(0.0, 0.0);
-
-    // real-operand forms (half the multiply-adds per K-step) fetch the next
-    // K-step's tiles into registers before this step's products and store them
-    // to shared memory after, so the global loads' latency overlaps the
-    // multiply-adds; the complex form has the registers for neither and
-    // stores them before its products
-    constexpr bool STAGE = REAL != 0;
-    constexpr int LA = (BM * BK + NT - 1) / NT, LB = (BN * BK + NT - 1) / NT;
-    zd pa[LA], pb[LB];
-    auto fetch = [&](int k0) {
-#pragma unroll
-        for (int t = 0; t < LA; ++t) {
-            const int e = tid + t * NT;
-            int i, l;
-            if (OPA == OP_N) { i = e % BM; l = e / BM; } else { l = e % BK; i = e / BK; }
-            const int gi = tileM + i, gl = k0 + l;
-            zd v = make_double2(0.0, 0.0);
-            if (e < BM * BK && gi < a.m && gl < a.k) v = load_op<OPA>(Ab, a.lda, gi, gl, a.a_real, a.planeA);
-            pa[t] = v;
+    for (int s = 0; s < ST - 1; ++s) {
+        if (s < KT) {
+            la.load(smem0 + s * (unsigned)SH::STAGE, s);
+            lb.load(smem0 + s * (unsigned)SH::STAGE + (unsigned)LA::BYTES, s);
         }
-#pragma unroll
-        for (int t = 0; t < LB; ++t) {
-            const int e = tid + t * NT;
-            int l, j;
-            if (OPB == OP_N) { l = e % BK; j = e / BK; } else { j = e % BN; l = e / BN; }
-            const int gl = k0 + l, gj = tileN + j;
-            zd v = make_double2(0.0, 0.0);
-            if (e < BN * BK && gl < a.k && gj < a.n) v = load_op<OPB>(Bb, a.ldb, gl, gj, a.b_real, a.planeB);
-            pb[t] = v;
-        }
-    };
-    auto commit = [&](int buf) {
-#pragma unroll
-        for (int t = 0; t < LA; ++t) {
-            const int e = tid + t * NT;
-            int i, l;
-            if (OPA == OP_N) { i = e % BM; l = e / BM; } else { l = e % BK; i = e / BK; }
-            if (e < BM * BK) As[buf][l][i] = pa[t];
-        }
-#pragma unroll
-        for (int t = 0; t < LB; ++t) {
-            const int e = tid + t * NT;
-            int l, j;
-            if (OPB == OP_N) { l = e % BK; j = e / BK; } else { j = e % BN; l = e / BN; }
-            if (e < BN * BK) Bs[buf][l][j] = pb[t];
-        }
-    };
-
-    auto load_tiles = [&](int buf, int k0) {
-        for (int e = tid; e < BM * BK; e += NT) {
-            int i, l;
-            if (OPA == OP_N) { i = e % BM; l = e / BM; } else { l = e % BK; i = e / BK; }
-            int gi = tileM + i, gl = k0 + l;
-            zd v = make_double2(0.0, 0.0);
-            if (gi < a.m && gl < a.k) v = load_op<OPA>(Ab, a.lda, gi, gl, a.a_real, a.planeA);
-            As[buf][l][i] = v;
-        }
-        for (int e = tid; e < BN * BK; e += NT) {
-            int l, j;
-            if (OPB == OP_N) { l = e % BK; j = e / BK; } else { j = e % BN; l = e / BN; }
-            int gl = k0 + l, gj = tileN + j;
-            zd v = make_double2(0.0, 0.0);
-            if (gl < a.k && gj < a.n) v = load_op<OPB>(Bb, a.ldb, gl, gj, a.b_real, a.planeB);
-            Bs[buf][l][j] = v;
-        }
-    };
-
-    int buf = 0;
-    if (STAGE) {
-        fetch(0);
-        commit(0);
-    } else {
-        load_tiles(0, 0);
+        cp_async_commit();
     }
-    __syncthreads();
-    for (int k0 = 0; k0 < a.k; k0 += BK) {
-        const bool more = k0 + BK < a.k;
-        if (STAGE && more) fetch(k0 + BK);
-        if (!STAGE && more) load_tiles(buf ^ 1, k0 + BK);
-#pragma unroll
-        for (int l = 0; l < BK; ++l) {
-            zd ra[TM], rb[TN];
-#pragma unroll
-            for (int i = 0; i < TM; ++i) ra[i] = As[buf][l][tx + i * NTX];
-#pragma unroll
-            for (int j = 0; j < TN; ++j) rb[j] = Bs[buf][l][ty + j * (BN / TN)];
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) {
-                    if (REAL == 0) {
-                        zfma(acc[i][j], ra[i], rb[j]);
-                    } else if (REAL == 1) {
-                        acc[i][j].x = fma(ra[i].x, rb[j].x, acc[i][j].x);
-                        acc[i][j].y = fma(ra[i].x, rb[j].y, acc[i][j].y);
-                    } else if (REAL == 2) {
-                        acc[i][j].x = fma(ra[i].x, rb[j].x, acc[i][j].x);
-                        acc[i][j].y = fma(ra[i].y, rb[j].x, acc[i][j].y);
-                    } else {
-                        acc[i][j].x = fma(ra[i].x, rb[j].x, acc[i][j].x);
-                    }
-                }
-        }
-        if (STAGE && more) commit(buf ^ 1);
+    int slot = 0, fill = ST - 1;
+    for (int kt = 0; kt < KT; ++kt) {
+        cp_async_wait<ST - 2>();
         __syncthreads();
-        buf ^= 1;
+        if (kt + ST - 1 < KT) {
+            la.load(smem0 + fill * (unsigned)SH::STAGE, kt + ST - 1);
+            lb.load(smem0 + fill * (unsigned)SH::STAGE + (unsigned)LA::BYTES, kt + ST - 1);
+        }
+        cp_async_commit();
+        const typename LA::T *As = (const typename LA::T *)(smem + slot * SH::STAGE);
+        const typename LB::T *Bs = (const typename LB::T *)(smem + slot * SH::STAGE + LA::BYTES);
+#pragma unroll
+        for (int k4 = 0; k4 < BK; k4 += 4) {
+            double ar[MI], ai[MI], an[MI];
+#pragma unroll
+            for (int i = 0; i < MI; ++i) {
+                if constexpr (RA) {
+                    ar[i] = As[LA::at(wm + 8 * i + fr, k4 + fk)];
+                } else {
+                    const zd v = As[LA::at(wm + 8 * i + fr, k4 + fk)];
+                    ar[i] = v.x;
+                    ai[i] = OPA == OP_C ? -v.y : v.y;
+                    an[i] = OPA == OP_C ? v.y : -v.y;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < NI; ++j) {
+                if (j >= nb) continue;
+                double br, bi = 0.0;
+                if constexpr (RB) {
+                    br = Bs[LB::at(wn + 8 * j + fr, k4 + fk)];
+                } else {
+                    const zd v = Bs[LB::at(wn + 8 * j + fr, k4 + fk)];
+                    br = v.x;
+                    bi = OPB == OP_C ? -v.y : v.y;
+                }
+#pragma unroll
+                for (int i = 0; i < MI; ++i) {
+                    if (i >= mb) continue;
+                    dmma(cr[i][j][0], cr[i][j][1], ar[i], br);
+                    if constexpr (!RB) dmma(ci[i][j][0], ci[i][j][1], ar[i], bi);
+                    if constexpr (!RA && !RB) dmma(cr[i][j][0], cr[i][j][1], an[i], bi);
+                    if constexpr (!RA) dmma(ci[i][j][0], ci[i][j][1], ai[i], br);
+                }
+            }
+        }
+        slot = slot + 1 == ST ? 0 : slot + 1;
+        fill = fill + 1 == ST ? 0 : fill + 1;
     }
 
+    zd *Cb = a.C + (size_t)b * a.strideC;
     const bool beta0 = (a.beta.x == 0.0 && a.beta.y == 0.0);
 #pragma unroll
-    for (int j = 0; j < TN; ++j) {
-        int gj = tileN + ty + j * (BN / TN);
-        if (gj >= a.n) continue;
+    for (int j = 0; j < NI; ++j) {
 #pragma unroll
-        for (int i = 0; i < TM; ++i) {
-            int gi = tileM + tx + i * NTX;
-            if (gi >= a.m) continue;
-            zd v = zmul(a.alpha, acc[i][j]);
-            if (Cb) {
+        for (int h = 0; h < 2; ++h) {
+            const int gj = tileN + wn + 8 * j + 2 * fk + h;
+            if (gj >= a.n) continue;
+#pragma unroll
+            for (int i = 0; i < MI; ++i) {
+                const int gi = tileM + wm + 8 * i + fr;
+                if (gi >= a.m) continue;
+                zd v = zmul(a.alpha, make_double2(cr[i][j][h], ci[i][j][h]));
                 zd *c = Cb + gi + (size_t)gj * a.ldc;
                 if (!beta0) zfma(v, a.beta, *c);
                 *c = v;
             }
-            if (a.outMode & OUT_BF16P) {
-                __nv_bfloat16 *c2 = (__nv_bfloat16 *)a.C2 + (size_t)b * a.strideC2 + gi + (size_t)gj * a.ldc2;
-                c2[0] = __double2bfloat16(v.x);
-                c2[a.plane2] = __double2bfloat16(v.y);
-            }
-            if (a.outMode & OUT_C32P) {
-                float *c3 = a.C3 + (size_t)b * a.strideC3 + gi + (size_t)gj * a.ldc3;
-                c3[0] = (float)v.x;
-                c3[a.plane3] = (float)v.y;
-            }
         }
     }
 }
 
-template <int BM, int BN, int TM, int TN, int OPA, int OPB, int REAL = 0>
+template <class TL, int OPA, int OPB, int REAL = 0>
 cudaError_t launch3(const ZGemmArgs &a, cudaStream_t s)
 {
-    dim3 grid((a.m + BM - 1) / BM, (a.n + BN - 1) / BN, a.batch);
-    dim3 block((BM / TM) * (BN / TN));
-    zgemm_kernel<BM, BN, TM, TN, OPA, OPB, REAL><<<grid, block, 0, s>>>(a);
+    typedef GemmShape<TL, OPA, OPB, REAL> SH;
+    dim3 grid((a.m + TL::BM - 1) / TL::BM, (a.n + TL::BN - 1) / TL::BN, a.batch);
+    static std::atomic<unsigned long long> attr{0};
+    const cudaError_t r = each_device_once(attr, [] {
+        return cudaFuncSetAttribute(zgemm_kernel<TL, OPA, OPB, REAL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)SH::SMEM);
+    });
+    if (r != cudaSuccess) return r;
+    zgemm_kernel<TL, OPA, OPB, REAL><<<grid, TL::NT, SH::SMEM, s>>>(a);
     return cudaGetLastError();
 }
 
-template <int BM, int BN, int TM, int TN, int OPA, int OPB>
-cudaError_t launch_real(const ZGemmArgs &a, cudaStream_t s)
-{
-    const int real = (a.a_real == ST_R64 ? 1 : 0) | (a.b_real == ST_R64 ? 2 : 0);
-    if (real == 1) return launch3<BM, BN, TM, TN, OPA, OPB, 1>(a, s);
-    if (real == 2) return launch3<BM, BN, TM, TN, OPA, OPB, 2>(a, s);
-    if (real == 3) return launch3<BM, BN, TM, TN, OPA, OPB, 3>(a, s);
-    return launch3<BM, BN, TM, TN, OPA, OPB, 0>(a, s);
-}
-
-template <int BM, int BN, int TM, int TN>
+// The operator pairs and real operands that the engine's products have.
+template <class TL>
 cudaError_t launch2(const ZGemmArgs &a, cudaStream_t s)
 {
-    // the operator pairs that real operands come with take the real forms
-    if (a.opA == OP_N && a.opB == OP_N) return launch_real<BM, BN, TM, TN, OP_N, OP_N>(a, s);
-    if (a.opA == OP_N && a.opB == OP_T) return launch_real<BM, BN, TM, TN, OP_N, OP_T>(a, s);
-    if (a.opA == OP_C && a.opB == OP_N) return launch_real<BM, BN, TM, TN, OP_C, OP_N>(a, s);
-    if (a.opA == OP_T && a.opB == OP_N) return launch_real<BM, BN, TM, TN, OP_T, OP_N>(a, s);
-#define ZG_CASE(OA, OB) \
-    if (a.opA == OA && a.opB == OB) return launch3<BM, BN, TM, TN, OA, OB>(a, s);
-    ZG_CASE(OP_N, OP_N) ZG_CASE(OP_N, OP_T) ZG_CASE(OP_N, OP_C)
-    ZG_CASE(OP_T, OP_N) ZG_CASE(OP_T, OP_T) ZG_CASE(OP_T, OP_C)
-    ZG_CASE(OP_C, OP_N) ZG_CASE(OP_C, OP_T) ZG_CASE(OP_C, OP_C)
+    const int real = (a.a_real ? 1 : 0) | (a.b_real ? 2 : 0);
+#define ZG_CASE(OA, OB, R) \
+    if (a.opA == OA && a.opB == OB && real == R) return launch3<TL, OA, OB, R>(a, s);
+    ZG_CASE(OP_N, OP_N, 0) ZG_CASE(OP_N, OP_N, 1) ZG_CASE(OP_N, OP_N, 2)
+    ZG_CASE(OP_N, OP_T, 0) ZG_CASE(OP_N, OP_T, 1) ZG_CASE(OP_N, OP_T, 3)
+    ZG_CASE(OP_C, OP_N, 0) ZG_CASE(OP_C, OP_N, 2)
+    ZG_CASE(OP_T, OP_N, 0) ZG_CASE(OP_T, OP_N, 1)
+    ZG_CASE(OP_T, OP_T, 0) ZG_CASE(OP_T, OP_C, 0)
 #undef ZG_CASE
     return cudaErrorInvalidValue;
 }
@@ -253,50 +253,48 @@ cudaError_t launch2(const ZGemmArgs &a, cudaStream_t s)
 // outside stream capture; captured launches reuse the cached choice.
 namespace {
 
-constexpr int NCAND = 5;
-
-int real_form(const ZGemmArgs &a)
-{
-    if (a.opA != OP_N || (a.opB != OP_N && a.opB != OP_T)) return 0;
-    return (a.a_real == ST_R64 ? 1 : 0) | (a.b_real == ST_R64 ? 2 : 0);
-}
-
-// Wide thread tiles for one real operand: a thread's A (B) values cost four
-// shared-memory wavefronts per complex and two per real value and K-column,
-// so 4 x 8 (complex A, real B) and 8 x 4 (real A, complex B) give 64 FP64
-// FMAs per 32 wavefronts, twice the 4 x 4 form's 32 per 24.
-cudaError_t launch_wide_real(const ZGemmArgs &a, cudaStream_t s)
-{
-    const int real = real_form(a);
-    if (real == 2) {
-        if (a.opB == OP_N) return launch3<64, 128, 4, 8, OP_N, OP_N, 2>(a, s);
-        return launch3<64, 128, 4, 8, OP_N, OP_T, 2>(a, s);
-    }
-    if (real == 1) {
-        if (a.opB == OP_N) return launch3<128, 64, 8, 4, OP_N, OP_N, 1>(a, s);
-        return launch3<128, 64, 8, 4, OP_N, OP_T, 1>(a, s);
-    }
-    return launch2<64, 64, 4, 4>(a, s);
-}
+// Measured on one B200, TFLOP/s of the three tiles (32 x 32 | 64 x 32 | 64 x 64):
+// M-build 16384 x 2048 x 640, real A: - | - | 30.4; 128 x 32 x 128 x 2048
+// walkers: 30.3 | 30.6 | 26.9; 56 x 56 x 128 x 1024: 23.8 | 23.4 | 20.8;
+// 32 x 32 x 128 x 2048: 28.2 | 15.4 | 9.3; 14 x 14 x 32 x 100: 6.5 us each.
+constexpr int NCAND = 3;
+typedef Tile<32, 32, 16, 16, 8, 4, 4> TileS;
+typedef Tile<64, 32, 32, 16, 8, 4, 3> TileM;
+typedef Tile<64, 64, 32, 16, 16, 3, 2> TileL;
 
 cudaError_t launch_cand(int c, const ZGemmArgs &a, cudaStream_t s)
 {
     switch (c) {
-    case 0: return launch2<32, 32, 2, 2>(a, s);
-    case 1: return launch2<32, 64, 2, 4>(a, s);
-    case 2: return launch2<64, 64, 4, 4>(a, s);
-    case 3: return launch2<128, 32, 8, 2>(a, s);
-    default: return launch_wide_real(a, s);
+    case 0: return launch2<TileS>(a, s);
+    case 1: return launch2<TileM>(a, s);
+    default: return launch2<TileL>(a, s);
     }
+}
+
+// Time of the last-finishing SM in units of products: waves of CTAs (148 SMs,
+// MINB CTAs each) times the whole tile, over the tile's measured rate on
+// shapes that fill it (the smaller tiles pay more fragment loads and barriers
+// per product).  A tile counts in full where C covers part of it: the warps
+// outside C leave their SM quadrant's matrix pipe idle (32 x 32 outputs: 0.076
+// ms in 32 x 32 tiles, 0.140 in 64 x 32, 0.232 in 64 x 64).
+template <class TL>
+double tile_cost(const ZGemmArgs &a, double rate)
+{
+    const double tm = (a.m + TL::BM - 1) / TL::BM, tn = (a.n + TL::BN - 1) / TL::BN;
+    const double tiles = tm * tn * a.batch * (a.lower ? 0.5 : 1.0);
+    double waves = tiles / (148.0 * TL::MINB);
+    // beyond a few waves the ragged last one overlaps the stragglers
+    waves = waves < 4.0 ? (double)(long long)(waves + 0.999999) : waves + 0.5;
+    return waves * TL::MINB * TL::BM * TL::BN / rate;
 }
 
 int default_cand(const ZGemmArgs &a)
 {
-    if (a.m <= 32 && a.n <= 32) return 0;
-    if (a.m <= 32) return 1;
-    const int real = real_form(a);
-    if ((real == 1 || real == 2) && a.m >= 128 && a.n >= 128) return 4;
-    return 2;
+    const double c[NCAND] = {tile_cost<TileS>(a, 0.93), tile_cost<TileM>(a, 0.95), tile_cost<TileL>(a, 1.0)};
+    int best = 0;
+    for (int i = 1; i < NCAND; ++i)
+        if (c[i] < c[best]) best = i;
+    return best;
 }
 
 std::mutex g_tune_mu;
