@@ -24,6 +24,7 @@
 #include "engine_internal.cuh"
 #include "exchange_f64.cuh"
 #include "mixed.cuh"
+#include "taylor_f64.cuh"
 #include "tc_gemm.cuh"
 #include "walker_kernels.cuh"
 #include "zgemm.cuh"
@@ -295,10 +296,25 @@ int xbar_gemm(afqmc_engine *e, const Blocks &bl)
 // dst = exp(M) src via the dynamicOrder Taylor series
 // (LogHop2isSD2isOperation::applyToRight, logHop2isSD2isOperation.cpp:38-45,159-195).
 // Mstride = 0 for a shared matrix (one-body LogHop2is), n*n per walker otherwise.
+// With `post` (n x n) given, dst = post exp(M) src.  Shapes beyond the fused
+// kernel (n > 256 or more than 128 columns) run one GEMM and one accumulation
+// per order; dst must then differ from src, and post is not taken.
 int taylor_apply(afqmc_engine *e, const zd *M, long long Mstride, const zd *src, zd *dst,
-                 const int *mask, bool stats)
+                 const int *mask, bool stats, const zd *post = nullptr)
 {
     const int W = e->W;
+    if (taylor_f64_supported(e->n, e->ncol)) {
+        TaylorF64 t;
+        t.n = e->n; t.N = e->ncol; t.W = W;
+        t.M = M; t.Mstride = Mstride; t.src = src; t.dst = dst; t.mask = mask;
+        t.order = e->order; t.status = e->status;
+        t.kmax = TAYLOR_KMAX; t.checkFrom = TAYLOR_BASE + 1; t.acc = TAYLOR_ACC;
+        t.postZ = post;
+        const cudaError_t r = taylor_f64(t, e->stream);
+        if (r != cudaSuccess) return fail(AFQMC_ERR_CUDA, std::string("Taylor kernel: ") + cudaGetErrorString(r));
+        if (stats) launch_taylor_stats(W, mask, e->order, e->tstats, e->stream);
+        return check_launch();
+    }
     launch_copy_masked(W, e->wsize, src, dst, mask, e->stream);
     CUDA_TRY(cudaMemsetAsync(e->done, 0, sizeof(int) * W, e->stream));
     const zd *old = src;
@@ -402,11 +418,14 @@ int project_dtk_dtv(afqmc_engine *e)
             g.alpha = make_double2(0.0, e->cdv.sqrtMinusDtIm);
             TRY(gemm(g, s));
         }
+        // the dense one-body product runs inside the Taylor kernel
+        const bool fused = !e->useLog && taylor_f64_supported(e->n, e->ncol);
         {
             PHASE(AFQMC_PH_TAYLOR);
-            TRY(taylor_apply(e, e->M, (long long)e->n * e->n, e->wf, e->wfTmp, e->surv, true));
+            TRY(taylor_apply(e, e->M, (long long)e->n * e->n, e->wf, fused ? e->wf : e->wfTmp, e->surv, true,
+                             fused ? e->expK[0] : nullptr));
         }
-        { PHASE(AFQMC_PH_ONEBODY); TRY(one_body(e, 0, e->wfTmp, e->wf, e->surv)); }
+        if (!fused) { PHASE(AFQMC_PH_ONEBODY); TRY(one_body(e, 0, e->wfTmp, e->wf, e->surv)); }
     }
     return check_launch();
 }

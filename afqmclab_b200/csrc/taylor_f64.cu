@@ -1,0 +1,280 @@
+// exp(M) phi of every walker by the dynamicOrder Taylor series
+// (LogHop2isSD2isOperation::applyToRight, logHop2isSD2isOperation.cpp:38-45,
+// 159-195), FP64, one kernel for the whole series and, where asked, the
+// one-body product that follows it.
+//
+// A CTA holds 16 columns of one walker and all n rows: the current term in
+// shared memory (the right operand of the next order), the running sum in
+// the registers that also define the accumulator layout (a warp owns 16 rows
+// by 16 columns).  M is streamed through four cp.async stages of 8 columns,
+// once per order; the walkers in flight (148 SMs times n^2 16 bytes per walker,
+// 39 MB at n = 128) stay in L2, so memory sees M once.  The CTAs of one
+// walker form a cluster: the stopping test is the walker's largest term, so
+// each order from `checkFrom` on ends with one exchange of maxima over
+// distributed shared memory.
+//
+// Bound: the FP64 matrix rate.  Per order 8 n^2 N flops per walker against
+// n^2 16 bytes of M from L2 (16 bytes per cycle and SM at n = 256, 8 at 128) and
+// 32 bytes per cycle and SM of fragment loads, both far below their limits.
+// Measured, series and one-body product, against one GEMM and one accumulation
+// launch per order up to the cap: n = 128, N = 32, 2048 walkers 7.44 -> 2.49 ms;
+// n = 64, N = 16, 512 walkers 0.761 -> 0.113; n = 90, N = 21, 300 walkers 1.17 ->
+// 0.338; n = 256, N = 64, 512 walkers 7.37 -> 5.59.
+#include <cooperative_groups.h>
+#include <math_constants.h>
+
+#include <algorithm>
+#include <atomic>
+
+#include "dmma.cuh"
+#include "once.cuh"
+#include "taylor_f64.cuh"
+
+namespace cg = cooperative_groups;
+
+extern std::atomic<long long> g_launch_count;
+
+namespace {
+
+constexpr int TF_COLS = 16;      // columns of phi per CTA
+constexpr int TF_BK = 8;         // columns of M per stage
+constexpr int TF_STAGES = 4;
+constexpr int TF_MAXN = 256;     // 16 rows per warp, 16 warps
+constexpr int TF_MAXCL = 8;      // CTAs per walker (portable cluster size)
+
+__host__ __device__ constexpr int tf_rows(int n) { return (n + 15) / 16 * 16; }
+// leading dimensions (elements) that keep fragment loads conflict-free: rows
+// contiguous 2 mod 8 (complex) or 4 mod 16 (real); contraction contiguous 4 mod 8
+__host__ __device__ constexpr int tf_lda(int n) { return tf_rows(n) + 2; }
+__host__ __device__ constexpr int tf_ldt(int n) { return tf_rows(n) + 4; }
+__host__ __device__ constexpr size_t tf_stage(int n) { return (size_t)TF_BK * tf_lda(n) * sizeof(zd); }
+__host__ __device__ constexpr size_t tf_smem(int n)
+{
+    return TF_STAGES * tf_stage(n) + (size_t)TF_COLS * tf_ldt(n) * sizeof(zd);
+}
+
+struct TfAcc {
+    double r[2][2][2], i[2][2][2];   // 8-row block, 8-column block, column parity
+};
+
+// One n x n matrix times the term in shared memory, accumulated into c.  The
+// stream of M stages is cyclic: stage `it` of the stream is tile it % KT, so
+// that the next order's first tiles are already on their way at an order's
+// end.  REAL: the matrix is real (its tile is 8-byte elements, leading
+// dimension rows + 4).
+template <bool REAL>
+struct TfStream {
+    const void *base;
+    int n, npad, KT, it;
+    unsigned st0;
+    size_t stage;
+    int r, k0;                 // this thread's row and first column of a tile
+
+    __device__ __forceinline__ void start(const void *m, int n_, unsigned st0_, size_t stage_)
+    {
+        base = m; n = n_; npad = tf_rows(n_); KT = (n_ + TF_BK - 1) / TF_BK; it = 0; st0 = st0_; stage = stage_;
+        r = threadIdx.x % npad;
+        k0 = threadIdx.x / npad;   // 0 or 1: the CTA has 2 npad threads
+#pragma unroll
+        for (int s = 0; s < TF_STAGES - 1; ++s) fill(s);
+    }
+    __device__ __forceinline__ void fill(int at)
+    {
+        constexpr int E = REAL ? 8 : 16;
+        const int kt = at % KT, slot = at % TF_STAGES;
+        const int ld = REAL ? npad + 4 : npad + 2;
+        const unsigned dst = st0 + (unsigned)(slot * stage);
+#pragma unroll
+        for (int t = 0; t < TF_BK / 2; ++t) {
+            const int kk = k0 + 2 * t, k = kt * TF_BK + kk;
+            const bool ok = r < n && k < n;
+            const char *p = (const char *)base + (ok ? ((size_t)k * n + r) * E : 0);
+            cp_async_elem<E>(dst + (unsigned)((kk * ld + r) * E), p, ok);
+        }
+        cp_async_commit();
+    }
+    __device__ __forceinline__ void product(const unsigned char *smem, const zd *T, int ldt, int wr, int fr, int fk,
+                                            int nb, TfAcc &c)
+    {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) c.r[i][j][0] = c.r[i][j][1] = c.i[i][j][0] = c.i[i][j][1] = 0.0;
+        for (int kt = 0; kt < KT; ++kt, ++it) {
+            cp_async_wait<TF_STAGES - 2>();
+            __syncthreads();
+            fill(it + TF_STAGES - 1);
+            const unsigned char *sp = smem + (it % TF_STAGES) * stage;
+#pragma unroll
+            for (int k4 = 0; k4 < TF_BK; k4 += 4) {
+                double ar[2], ai[2], an[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    if constexpr (REAL) {
+                        ar[i] = ((const double *)sp)[(k4 + fk) * (npad + 4) + wr + 8 * i + fr];
+                    } else {
+                        const zd v = ((const zd *)sp)[(k4 + fk) * (npad + 2) + wr + 8 * i + fr];
+                        ar[i] = v.x; ai[i] = v.y; an[i] = -v.y;
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    if (j >= nb) continue;
+                    const zd b = T[(size_t)(8 * j + fr) * ldt + kt * TF_BK + k4 + fk];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        dmma(c.r[i][j][0], c.r[i][j][1], ar[i], b.x);
+                        dmma(c.i[i][j][0], c.i[i][j][1], ar[i], b.y);
+                        if constexpr (!REAL) {
+                            dmma(c.r[i][j][0], c.r[i][j][1], an[i], b.y);
+                            dmma(c.i[i][j][0], c.i[i][j][1], ai[i], b.x);
+                        }
+                    }
+                }
+            }
+        }
+    }
+};
+
+__global__ void __launch_bounds__(2 * TF_MAXN, 1)
+taylor_f64_kernel(TaylorF64 a)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ double wmax[16], cmax[2][TF_MAXCL];
+    const int n = a.n, N = a.N;
+    const int cs = (N + TF_COLS - 1) / TF_COLS, w = blockIdx.x / cs, rank = blockIdx.x % cs;
+    if (a.mask && !a.mask[w]) return;   // the whole cluster
+    const int col0 = rank * TF_COLS, ncols = min(TF_COLS, N - col0), nb = (ncols + 7) / 8;
+    const int ldt = tf_ldt(n);
+    const size_t stage = tf_stage(n);
+    zd *T = (zd *)(smem + TF_STAGES * stage);
+    const unsigned st0 = (unsigned)__cvta_generic_to_shared(smem);
+    const int tid = threadIdx.x, NT = blockDim.x, lane = tid & 31, warp = tid >> 5;
+    const int wr = warp * 16, fr = lane >> 2, fk = lane & 3;
+
+    TfStream<false> ms;
+    ms.start(a.M + (size_t)w * a.Mstride, n, st0, stage);
+    const zd *src = a.src + ((size_t)w * N + col0) * n;
+    for (int e = tid; e < TF_COLS * tf_rows(n); e += NT) {
+        const int r = e % tf_rows(n), c = e / tf_rows(n);
+        T[(size_t)c * ldt + r] = (r < n && c < ncols) ? src[(size_t)c * n + r] : make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+    TfAcc sum, c;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const zd v = T[(size_t)(8 * j + 2 * fk + h) * ldt + wr + 8 * i + fr];
+                sum.r[i][j][h] = v.x;
+                sum.i[i][j][h] = v.y;
+            }
+
+    int k = 1;
+    for (;; ++k) {
+        ms.product(smem, T, ldt, wr, fr, fk, nb, c);
+        const double inv = 1.0 / k;
+        double mx = 0.0;   // largest |term|^2
+        __syncthreads();   // every warp is done with the previous term
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const double x = c.r[i][j][h] * inv, y = c.i[i][j][h] * inv;
+                    sum.r[i][j][h] += x;
+                    sum.i[i][j][h] += y;
+                    T[(size_t)(8 * j + 2 * fk + h) * ldt + wr + 8 * i + fr] = make_double2(x, y);
+                    double s = fma(x, x, y * y);
+                    // |z| of an infinity with a NaN is infinite
+                    if (!(s <= 1e300) && (isinf(x) || isinf(y))) s = CUDART_INF;
+                    mx = fmax(mx, s);
+                }
+        if (k < a.checkFrom) continue;
+        mx = warp_max(mx);
+        if (lane == 0) wmax[warp] = mx;
+        __syncthreads();
+        double all = 0.0;
+        for (int q = 0; q < NT / 32; ++q) all = fmax(all, wmax[q]);
+        if (cs > 1) {
+            cg::cluster_group cl = cg::this_cluster();
+            if (tid < cs) cl.map_shared_rank(&cmax[k & 1][0], tid)[rank] = all;
+            cl.sync();
+            for (int q = 0; q < cs; ++q) all = fmax(all, cmax[k & 1][q]);
+        }
+        const bool done = all <= a.acc * a.acc;
+        if (!done && k < a.kmax) continue;
+        if (rank == 0 && tid == 0) {
+            if (a.order) a.order[w] = k;
+            if (!done) atomicOr(a.status + w, (int)ST_TAYLOR_CAP);
+        }
+        break;
+    }
+
+    if (a.postZ || a.postR) {
+        cp_async_wait<0>();
+        __syncthreads();   // the series' stages and the last term are free
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    T[(size_t)(8 * j + 2 * fk + h) * ldt + wr + 8 * i + fr] =
+                        make_double2(sum.r[i][j][h], sum.i[i][j][h]);
+        if (a.postR) {
+            TfStream<true> ps;
+            ps.start(a.postR, n, st0, stage);
+            ps.product(smem, T, ldt, wr, fr, fk, nb, sum);
+        } else {
+            ms.start(a.postZ, n, st0, stage);
+            ms.product(smem, T, ldt, wr, fr, fk, nb, sum);
+        }
+    }
+    zd *dst = a.dst + ((size_t)w * N + col0) * n;
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int cc = 8 * j + 2 * fk + h;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int r = wr + 8 * i + fr;
+                if (cc < ncols && r < n) dst[(size_t)cc * n + r] = make_double2(sum.r[i][j][h], sum.i[i][j][h]);
+            }
+        }
+    cp_async_wait<0>();
+}
+
+}  // namespace
+
+bool taylor_f64_supported(int n, int N) { return n <= TF_MAXN && N <= TF_COLS * TF_MAXCL; }
+
+cudaError_t taylor_f64(const TaylorF64 &a, cudaStream_t s)
+{
+    g_launch_count++;
+    static std::atomic<unsigned long long> attr{0};
+    cudaError_t r = each_device_once(attr, [] {
+        return cudaFuncSetAttribute(taylor_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)tf_smem(TF_MAXN));
+    });
+    if (r != cudaSuccess) return r;
+    const int cs = (a.N + TF_COLS - 1) / TF_COLS;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)cs * (unsigned)a.W);
+    cfg.blockDim = dim3((unsigned)(2 * tf_rows(a.n)));
+    cfg.dynamicSmemBytes = tf_smem(a.n);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)cs;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    r = cudaLaunchKernelEx(&cfg, taylor_f64_kernel, a);
+    return r != cudaSuccess ? r : cudaGetLastError();
+}
