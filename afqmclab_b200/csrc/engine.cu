@@ -695,7 +695,7 @@ int engine_pl_local_energy(afqmc_engine *e, int exchange)
         bool first = true;
         for (int b = 0; b < nb; ++b) {
             if (e->bl.Ns[b] == 0) continue;
-            TRY(exf64_walker_totals(e, exf64_block(e, b), !first, mult));
+            TRY(exf64_walker_totals(e, exf64_block(e, b), !first, mult, true));
             first = false;
         }
         launch_pl_energy(W, e->G, e->Ktot, e->wfDaggerT, e->thetaT, e->xbar, e->ex, e->alive, e->logov,

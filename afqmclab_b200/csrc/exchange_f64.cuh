@@ -34,8 +34,10 @@ int exf64_run(afqmc_engine *e, const ExF64 &x, bool accumulate, int mult);
 // The operands of spin block b (block 0's X and V when restricted, which are
 // block 1's too: both blocks carry the same trial).
 ExF64 exf64_block(const afqmc_engine *e, int b);
-// Z = V U (Z(b + Ns i, w) = sum_g (D_gw A_g)(b, i)) and exTot[w] (+)= mult u_w^T Z_w.
-int exf64_walker_totals(afqmc_engine *e, const ExF64 &x, bool accumulate, int mult);
+// exTot[w] (+)= mult u_w^T V u_w.  With wantZ the scratch then holds Z = V U
+// (Z(b + Ns i, w) = sum_g (D_gw A_g)(b, i)); without it, half the products are
+// done and Z is of no use.
+int exf64_walker_totals(afqmc_engine *e, const ExF64 &x, bool accumulate, int mult, bool wantZ);
 // M = Uden Um^T (K x K) and its exchange permutation R, R(a + Ns i, b + Ns j) =
 // M(b + Ns i, a + Ns j); Uden, Um are K x W with leading dimension K.
 int exf64_pair_matrix(afqmc_engine *e, const ExF64 &x, const zd *Uden, const zd *Um);

@@ -10,6 +10,7 @@
 // of 1024 128 x 56 walkers 0.465 -> 0.27 ms.
 #include "zgemm.cuh"
 
+#include <algorithm>
 #include <atomic>
 #include <map>
 #include <mutex>
@@ -109,23 +110,28 @@ zgemm_kernel(ZGemmArgs a)
     typedef GemmShape<TL, OPA, OPB, REAL> SH;
     typedef typename SH::LA LA;
     typedef typename SH::LB LB;
-    const int b = blockIdx.z;
+    const int b = blockIdx.z / a.parts;
+    const bool second = blockIdx.z % a.parts != 0;
     if (a.mask && a.mask[b] == 0) return;
-    const int tileM = blockIdx.x * BM, tileN = blockIdx.y * BN;
+    const int m = second ? a.m1 : a.m, n = second ? a.n1 : a.n;
+    // a quadratic form's rows get longer downwards: the longest start first
+    const int tileM = (a.quad ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * BM, tileN = blockIdx.y * BN;
+    if (tileM >= m || tileN >= n) return;
     if (a.lower && tileM + BM <= tileN) return;
+    const int k = a.quad ? min(a.k, tileM + BM) : second ? a.k1 : a.k;
 
     extern __shared__ __align__(16) unsigned char smem[];
     const unsigned smem0 = (unsigned)__cvta_generic_to_shared(smem);
-    const char *Ab = (const char *)a.A + (size_t)b * a.strideA * sizeof(typename LA::T);
-    const char *Bb = (const char *)a.B + (size_t)b * a.strideB * sizeof(typename LB::T);
-    const Loader<BM, BK, NT, OPA != OP_N, RA> la(Ab, a.lda, tileM, a.m, a.k);
-    const Loader<BN, BK, NT, OPB == OP_N, RB> lb(Bb, a.ldb, tileN, a.n, a.k);
+    const char *Ab = (const char *)a.A + ((size_t)b * a.strideA + (second ? a.offA1 : 0)) * sizeof(typename LA::T);
+    const char *Bb = (const char *)a.B + ((size_t)b * a.strideB + (second ? a.offB1 : 0)) * sizeof(typename LB::T);
+    const Loader<BM, BK, NT, OPA != OP_N, RA> la(Ab, a.lda, tileM, m, k);
+    const Loader<BN, BK, NT, OPB == OP_N, RB> lb(Bb, a.ldb, tileN, n, k);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wm = (warp % (BM / WM)) * WM, wn = (warp / (BM / WM)) * WN;
     const int fr = lane >> 2, fk = lane & 3;
     // fragments of this warp that meet C
-    const int mb = (a.m - tileM - wm + 7) / 8, nb = (a.n - tileN - wn + 7) / 8;
+    const int mb = (m - tileM - wm + 7) / 8, nb = (n - tileN - wn + 7) / 8;
 
     double cr[MI][NI][2], ci[MI][NI][2];
 #pragma unroll
@@ -133,7 +139,9 @@ zgemm_kernel(ZGemmArgs a)
 #pragma unroll
         for (int j = 0; j < NI; ++j) cr[i][j][0] = cr[i][j][1] = ci[i][j][0] = ci[i][j][1] = 0.0;
 
-    const int KT = (a.k + BK - 1) / BK;
+    const int KT = (k + BK - 1) / BK;
+    const int ktDiag = a.quad && tileM > 0 ? tileM / BK : -1;   // first stage of the diagonal block
+    static_assert(BM % BK == 0, "a diagonal block starts a stage");
 #pragma unroll
     for (int s = 0; s < ST - 1; ++s) {
         if (s < KT) {
@@ -151,6 +159,14 @@ zgemm_kernel(ZGemmArgs a)
             lb.load(smem0 + fill * (unsigned)SH::STAGE + (unsigned)LA::BYTES, kt + ST - 1);
         }
         cp_async_commit();
+        if (kt == ktDiag) {
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int j = 0; j < NI; ++j)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) { cr[i][j][h] *= 2.0; ci[i][j][h] *= 2.0; }
+        }
         const typename LA::T *As = (const typename LA::T *)(smem + slot * SH::STAGE);
         const typename LB::T *Bs = (const typename LB::T *)(smem + slot * SH::STAGE + LA::BYTES);
 #pragma unroll
@@ -192,18 +208,18 @@ zgemm_kernel(ZGemmArgs a)
         fill = fill + 1 == ST ? 0 : fill + 1;
     }
 
-    zd *Cb = a.C + (size_t)b * a.strideC;
+    zd *Cb = a.C + (size_t)b * a.strideC + (second ? a.offC1 : 0);
     const bool beta0 = (a.beta.x == 0.0 && a.beta.y == 0.0);
 #pragma unroll
     for (int j = 0; j < NI; ++j) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int gj = tileN + wn + 8 * j + 2 * fk + h;
-            if (gj >= a.n) continue;
+            if (gj >= n) continue;
 #pragma unroll
             for (int i = 0; i < MI; ++i) {
                 const int gi = tileM + wm + 8 * i + fr;
-                if (gi >= a.m) continue;
+                if (gi >= m) continue;
                 zd v = zmul(a.alpha, make_double2(cr[i][j][h], ci[i][j][h]));
                 zd *c = Cb + gi + (size_t)gj * a.ldc;
                 if (!beta0) zfma(v, a.beta, *c);
@@ -217,7 +233,8 @@ template <class TL, int OPA, int OPB, int REAL = 0>
 cudaError_t launch3(const ZGemmArgs &a, cudaStream_t s)
 {
     typedef GemmShape<TL, OPA, OPB, REAL> SH;
-    dim3 grid((a.m + TL::BM - 1) / TL::BM, (a.n + TL::BN - 1) / TL::BN, a.batch);
+    const int m = a.parts > 1 ? std::max(a.m, a.m1) : a.m, n = a.parts > 1 ? std::max(a.n, a.n1) : a.n;
+    dim3 grid((m + TL::BM - 1) / TL::BM, (n + TL::BN - 1) / TL::BN, a.batch * a.parts);
     static std::atomic<unsigned long long> attr{0};
     const cudaError_t r = each_device_once(attr, [] {
         return cudaFuncSetAttribute(zgemm_kernel<TL, OPA, OPB, REAL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -280,8 +297,9 @@ cudaError_t launch_cand(int c, const ZGemmArgs &a, cudaStream_t s)
 template <class TL>
 double tile_cost(const ZGemmArgs &a, double rate)
 {
-    const double tm = (a.m + TL::BM - 1) / TL::BM, tn = (a.n + TL::BN - 1) / TL::BN;
-    const double tiles = tm * tn * a.batch * (a.lower ? 0.5 : 1.0);
+    double tiles = (double)((a.m + TL::BM - 1) / TL::BM) * ((a.n + TL::BN - 1) / TL::BN);
+    if (a.parts > 1) tiles += (double)((a.m1 + TL::BM - 1) / TL::BM) * ((a.n1 + TL::BN - 1) / TL::BN);
+    tiles *= a.batch * (a.lower || a.quad ? 0.5 : 1.0);
     double waves = tiles / (148.0 * TL::MINB);
     // beyond a few waves the ragged last one overlaps the stragglers
     waves = waves < 4.0 ? (double)(long long)(waves + 0.999999) : waves + 0.5;
@@ -298,7 +316,12 @@ int default_cand(const ZGemmArgs &a)
 }
 
 std::mutex g_tune_mu;
-std::map<std::tuple<int, int, int, int, int, int, int, int>, int> g_tuned;
+typedef std::tuple<int, int, int, int, int, int, int, int, int> TuneKey;
+TuneKey tune_key(const ZGemmArgs &a)
+{
+    return TuneKey(a.m, a.n, a.k, a.opA, a.opB, a.a_real, a.b_real, a.batch, a.lower + 2 * a.quad + 4 * a.parts);
+}
+std::map<TuneKey, int> g_tuned;
 std::atomic<int> g_autotune{0};
 
 }  // namespace
@@ -307,7 +330,7 @@ void zgemm_set_autotune(int on) { g_autotune = on; }
 
 int zgemm_tuned_choice(const ZGemmArgs &a)
 {
-    auto key = std::make_tuple(a.m, a.n, a.k, a.opA, a.opB, a.a_real, a.b_real, a.batch);
+    const TuneKey key = tune_key(a);
     std::lock_guard<std::mutex> lock(g_tune_mu);
     auto it = g_tuned.find(key);
     return it == g_tuned.end() ? -1 : it->second;
@@ -318,7 +341,7 @@ cudaError_t zgemm_batched(const ZGemmArgs &a, cudaStream_t stream)
     g_launch_count++;
     if (a.m <= 0 || a.n <= 0 || a.batch <= 0) return cudaSuccess;
     if (a.k <= 0) return cudaErrorInvalidValue;
-    const auto key = std::make_tuple(a.m, a.n, a.k, a.opA, a.opB, a.a_real, a.b_real, a.batch);
+    const TuneKey key = tune_key(a);
     int choice = -1;
     {
         std::lock_guard<std::mutex> lock(g_tune_mu);

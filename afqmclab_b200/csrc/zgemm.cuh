@@ -25,6 +25,16 @@ struct ZGemmArgs {
     // symmetric product (m = n): only output tiles that meet the lower
     // triangle (row >= column) are computed; tiles above it are not written
     int lower = 0;
+    // A symmetric (m = k) and C wanted only through sum_i x_i C_i with the
+    // columns x of B, x^T A x: row block I takes its diagonal block of A once
+    // and the blocks left of it twice, half the products.  Only A's entries
+    // with row >= column and its 64 x 64 diagonal blocks are read.
+    int quad = 0;
+    // A second product in the same launch and batch (parts = 2), of its own
+    // sizes and at these element offsets from A, B and C: the two spins of
+    // operators that do not mix them
+    int parts = 1, m1 = 0, n1 = 0, k1 = 0;
+    long long offA1 = 0, offB1 = 0, offC1 = 0;
 };
 
 // Launches on `stream`; returns cudaGetLastError() (cudaErrorInvalidValue for an
