@@ -50,6 +50,16 @@ struct afqmc_engine {
     zd expLogw[3] = {{0, 0}, {0, 0}, {0, 0}};
     bool useLog = false;
     zd *logK = nullptr;
+    // FP64 form: real copies of the one-body operators and of the trial where
+    // every imaginary part is zero (null otherwise).  Constrained path: n0 > 0
+    // when the trial's first n0 columns live on the spin-up rows and the
+    // others on the spin-down rows; spinDiag[k] when expK[k] has no entries
+    // between the spins
+    double *expKr[3] = {nullptr, nullptr, nullptr}, *realBuf[3] = {nullptr, nullptr, nullptr};
+    double *phiTr[2] = {nullptr, nullptr};
+    int *realFlag = nullptr;
+    int n0 = 0;
+    bool spinDiag[3] = {false, false, false};
     // propagator rebuild on the GPU: K (n x n), scratch Kp and three Taylor
     // matrices (n x n each), the 1-norm of Kp and sum bg^2
     double *kin = nullptr, *propNorms = nullptr;
@@ -64,6 +74,7 @@ struct afqmc_engine {
     // phaseless
     CholDev cdv{};
     double *chol = nullptr, *bg = nullptr, *tdev = nullptr;
+    double *cholP = nullptr;   // symmetric L_g in panel storage (taylor_panel_size(n) x G)
     zd *Aall = nullptr, *wfDaggerT = nullptr, *xbar = nullptr, *forcePL = nullptr, *aux = nullptr,
        *M = nullptr, *ex = nullptr, *constForcePL = nullptr;
     long long Ktot = 0;

@@ -19,7 +19,10 @@
 // Measured, series and one-body product, against one GEMM and one accumulation
 // launch per order up to the cap: n = 128, N = 32, 2048 walkers 7.44 -> 2.49 ms;
 // n = 64, N = 16, 512 walkers 0.761 -> 0.113; n = 90, N = 21, 300 walkers 1.17 ->
-// 0.338; n = 256, N = 64, 512 walkers 7.37 -> 5.59.
+// 0.338; n = 256, N = 64, 512 walkers 7.37 -> 5.59.  From the panels of a
+// symmetric M (and a real one-body operator): 2.57, 0.116, 0.336 and 6.19; the
+// mirrored rows cost loads here, and the M-build that writes them loses half
+// its products (2.87 -> 1.58, 0.117 -> 0.064, 0.123 -> 0.083, 5.68 -> 2.96 ms).
 #include <cooperative_groups.h>
 #include <math_constants.h>
 
@@ -61,8 +64,11 @@ struct TfAcc {
 // stream of M stages is cyclic: stage `it` of the stream is tile it % KT, so
 // that the next order's first tiles are already on their way at an order's
 // end.  REAL: the matrix is real (its tile is 8-byte elements, leading
-// dimension rows + 4).
-template <bool REAL>
+// dimension rows + 4).  PACKED: the matrix is complex symmetric, its lower
+// triangle packed by columns; a tile's rows above the diagonal block come from
+// the mirrored entries, 8 neighbouring threads taking one row's 8 columns (128
+// contiguous bytes).
+template <bool REAL, bool PACKED>
 struct TfStream {
     const void *base;
     int n, npad, KT, it;
@@ -84,12 +90,35 @@ struct TfStream {
         const int kt = at % KT, slot = at % TF_STAGES;
         const int ld = REAL ? npad + 4 : npad + 2;
         const unsigned dst = st0 + (unsigned)(slot * stage);
+        const int c0 = kt * TF_BK;
+        if (!PACKED) {
 #pragma unroll
-        for (int t = 0; t < TF_BK / 2; ++t) {
-            const int kk = k0 + 2 * t, k = kt * TF_BK + kk;
-            const bool ok = r < n && k < n;
-            const char *p = (const char *)base + (ok ? ((size_t)k * n + r) * E : 0);
-            cp_async_elem<E>(dst + (unsigned)((kk * ld + r) * E), p, ok);
+            for (int t = 0; t < TF_BK / 2; ++t) {
+                const int kk = k0 + 2 * t, k = c0 + kk;
+                const bool ok = r < n && k < n;
+                cp_async_elem<E>(dst + (unsigned)((kk * ld + r) * E), (const char *)base + (ok ? (k * n + r) * E : 0), ok);
+            }
+        } else {
+            const int n8 = (n + 7) / 8 * 8;
+            if (r >= c0) {
+                const int e0 = c0 * n8 - c0 * (c0 - 8) / 2 + (r - c0), len = n8 - c0;
+                const bool ok = r < n8;
+#pragma unroll
+                for (int t = 0; t < TF_BK / 2; ++t) {
+                    const int kk = k0 + 2 * t;
+                    cp_async_elem<E>(dst + (unsigned)((kk * ld + r) * E),
+                                     (const char *)base + (ok ? (e0 + kk * len) * E : 0), ok);
+                }
+            }
+            const int kk = threadIdx.x % TF_BK, dr = npad / 4;   // 2 npad / TF_BK rows a pass
+            int rr = threadIdx.x / TF_BK;
+#pragma unroll
+            for (int t = 0; t < 4; ++t, rr += dr)
+                if (rr < c0) {
+                    const int j0 = rr & ~7;
+                    const int e = j0 * n8 - j0 * (j0 - 8) / 2 + (rr - j0) * (n8 - j0) + (c0 - j0) + kk;
+                    cp_async_elem<E>(dst + (unsigned)((kk * ld + rr) * E), (const char *)base + e * E, true);
+                }
         }
         cp_async_commit();
     }
@@ -136,6 +165,7 @@ struct TfStream {
     }
 };
 
+template <bool PACKED>
 __global__ void __launch_bounds__(2 * TF_MAXN, 1)
 taylor_f64_kernel(TaylorF64 a)
 {
@@ -152,7 +182,7 @@ taylor_f64_kernel(TaylorF64 a)
     const int tid = threadIdx.x, NT = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const int wr = warp * 16, fr = lane >> 2, fk = lane & 3;
 
-    TfStream<false> ms;
+    TfStream<false, PACKED> ms;
     ms.start(a.M + (size_t)w * a.Mstride, n, st0, stage);
     const zd *src = a.src + ((size_t)w * N + col0) * n;
     for (int e = tid; e < TF_COLS * tf_rows(n); e += NT) {
@@ -226,12 +256,13 @@ taylor_f64_kernel(TaylorF64 a)
                     T[(size_t)(8 * j + 2 * fk + h) * ldt + wr + 8 * i + fr] =
                         make_double2(sum.r[i][j][h], sum.i[i][j][h]);
         if (a.postR) {
-            TfStream<true> ps;
+            TfStream<true, false> ps;
             ps.start(a.postR, n, st0, stage);
             ps.product(smem, T, ldt, wr, fr, fk, nb, sum);
         } else {
-            ms.start(a.postZ, n, st0, stage);
-            ms.product(smem, T, ldt, wr, fr, fk, nb, sum);
+            TfStream<false, false> ps;
+            ps.start(a.postZ, n, st0, stage);
+            ps.product(smem, T, ldt, wr, fr, fk, nb, sum);
         }
     }
     zd *dst = a.dst + ((size_t)w * N + col0) * n;
@@ -253,12 +284,12 @@ taylor_f64_kernel(TaylorF64 a)
 
 bool taylor_f64_supported(int n, int N) { return n <= TF_MAXN && N <= TF_COLS * TF_MAXCL; }
 
-cudaError_t taylor_f64(const TaylorF64 &a, cudaStream_t s)
+template <bool PACKED>
+static cudaError_t launch(const TaylorF64 &a, cudaStream_t s)
 {
-    g_launch_count++;
     static std::atomic<unsigned long long> attr{0};
     cudaError_t r = each_device_once(attr, [] {
-        return cudaFuncSetAttribute(taylor_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        return cudaFuncSetAttribute(taylor_f64_kernel<PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)tf_smem(TF_MAXN));
     });
     if (r != cudaSuccess) return r;
@@ -275,6 +306,12 @@ cudaError_t taylor_f64(const TaylorF64 &a, cudaStream_t s)
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    r = cudaLaunchKernelEx(&cfg, taylor_f64_kernel, a);
+    r = cudaLaunchKernelEx(&cfg, taylor_f64_kernel<PACKED>, a);
     return r != cudaSuccess ? r : cudaGetLastError();
+}
+
+cudaError_t taylor_f64(const TaylorF64 &a, cudaStream_t s)
+{
+    g_launch_count++;
+    return a.packed ? launch<true>(a, s) : launch<false>(a, s);
 }

@@ -1027,17 +1027,12 @@ __global__ void cp_force_kernel(int W, HubbardDev h, const zd *thetaT, long long
             f = h.constForce[i];
         } else {
             zd a = make_double2(0.0, 0.0), b = make_double2(0.0, 0.0);
-            if (h.decomp <= 1) {
-                for (int j = 0; j < N; ++j) {
-                    zfma(a, zconj(h.phiT[i + (size_t)n * j]), th[j + (size_t)N * i]);
-                    zfma(b, zconj(h.phiT[i + L + (size_t)n * j]), th[j + (size_t)N * (i + L)]);
-                }
-            } else {
-                for (int j = 0; j < N; ++j) {
-                    zfma(a, zconj(h.phiT[i + (size_t)n * j]), th[j + (size_t)N * (i + L)]);
-                    zfma(b, zconj(h.phiT[i + L + (size_t)n * j]), th[j + (size_t)N * i]);
-                }
-            }
+            // a trial that keeps the spins apart has its zeros skipped (and only
+            // the other blocks of thetaT are current then)
+            const int ja = h.n0 > 0 ? h.n0 : N, jb = h.n0;
+            const zd *ta = th + (size_t)N * (h.decomp <= 1 ? i : i + L), *tb = th + (size_t)N * (h.decomp <= 1 ? i + L : i);
+            for (int j = 0; j < ja; ++j) zfma(a, zconj(h.phiT[i + (size_t)n * j]), ta[j]);
+            for (int j = jb; j < N; ++j) zfma(b, zconj(h.phiT[i + L + (size_t)n * j]), tb[j]);
             zd bgv;
             if (h.decomp == 0) bgv = make_double2(a.x + b.x - 1.0, a.y + b.y);
             else if (h.decomp == 1) bgv = zsub(a, b);

@@ -45,6 +45,7 @@ struct HubbardDev {
     double dtUSum, forceCap;
     const double *constForce;  // non-null for constForce
     const zd *phiT;
+    int n0;   // > 0: columns [0, n0) of phiT live on the spin-up rows, the others on the spin-down rows
 };
 void launch_cp_force(int W, const HubbardDev &h, const zd *thetaT, long long tStride,
                      const int *surv, double *force, cudaStream_t s);
