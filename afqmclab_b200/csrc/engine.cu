@@ -445,21 +445,60 @@ __global__ void chol_pack_kernel(int n, int G, const double *chol, double *cholP
     }
 }
 
-// A real copy of `src` in *buf (allocated on the first call) and in *out when
-// every imaginary part is zero; *out is null otherwise.
-int real_copy(afqmc_engine *e, const zd *src, size_t count, double **buf, double **out)
+// Real copies of the dense one-body operators after an update, in the slots
+// that real_operators laid out.
+int refresh_real_operators(afqmc_engine *e)
 {
-    if (!*buf) TRY(dalloc(e, buf, count));
-    if (!e->realFlag) TRY(dalloc(e, &e->realFlag, 1));
-    int flag = 0;
-    CUDA_TRY(cudaMemsetAsync(e->realFlag, 0, sizeof(int), e->stream));
-    g_launch_count++;
-    real_parts_kernel<<<(int)std::min<size_t>(592, (count + 255) / 256), 256, 0, e->stream>>>((long long)count, src,
-                                                                                              *buf, e->realFlag);
+    if (e->precision != AFQMC_FP64) return AFQMC_OK;
+    const size_t n2 = (size_t)e->n * e->n;
+    int flags[3] = {0, 0, 0};
+    CUDA_TRY(cudaMemsetAsync(e->realFlag, 0, sizeof(flags), e->stream));
+    for (int k = 0; k < 3; ++k) {
+        e->expKr[k] = nullptr;
+        if (!e->expK[k]) continue;
+        g_launch_count++;
+        real_parts_kernel<<<(int)std::min<size_t>(592, (n2 + 255) / 256), 256, 0, e->stream>>>(
+            (long long)n2, e->expK[k], e->realBuf[k], e->realFlag + k);
+    }
     TRY(check_launch());
-    CUDA_TRY(cudaMemcpyAsync(&flag, e->realFlag, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+    CUDA_TRY(cudaMemcpyAsync(flags, e->realFlag, sizeof(flags), cudaMemcpyDeviceToHost, e->stream));
     CUDA_TRY(cudaStreamSynchronize(e->stream));
-    *out = flag ? nullptr : *buf;
+    for (int k = 0; k < 3; ++k)
+        if (e->expK[k] && !flags[k] && !(e->useLog && e->kind == KIND_PL)) e->expKr[k] = e->realBuf[k];
+    return AFQMC_OK;
+}
+
+// At creation, from the caller's arrays: real copies of the one-body operators
+// and of the trial blocks that have no imaginary part, in one allocation.
+int real_operators(afqmc_engine *e, const double *const op[3], const double *const trial[2])
+{
+    if (e->precision != AFQMC_FP64) return AFQMC_OK;
+    const size_t n2 = (size_t)e->n * e->n;
+    const size_t cnt[5] = {n2, n2, n2, (size_t)e->n * e->bl.Ns[0], (size_t)e->n * e->bl.Ns[1]};
+    const double *src[5] = {op[0], op[1], op[2], trial[0], trial[1]};
+    std::vector<double> host(cnt[0] + cnt[1] + cnt[2] + cnt[3] + cnt[4], 0.0);
+    bool real[5];
+    size_t at = 0;
+    for (int k = 0; k < 5; ++k) {
+        real[k] = src[k] != nullptr && cnt[k] > 0;
+        for (size_t i = 0; real[k] && i < cnt[k]; ++i) {
+            real[k] = src[k][2 * i + 1] == 0.0;
+            host[at + i] = src[k][2 * i];
+        }
+        at += cnt[k];
+    }
+    double *dev = nullptr;
+    TRY(dupload(e, &dev, host.data(), host.size()));
+    TRY(dalloc(e, &e->realFlag, 3));
+    for (int k = 0; k < 5; ++k) {
+        if (k < 3) {
+            e->realBuf[k] = dev;
+            if (real[k] && !(e->useLog && e->kind == KIND_PL)) e->expKr[k] = dev;
+        } else if (real[k]) {
+            e->phiTr[k - 3] = dev;
+        }
+        dev += cnt[k];
+    }
     return AFQMC_OK;
 }
 
@@ -467,7 +506,6 @@ int real_copy(afqmc_engine *e, const zd *src, size_t count, double **buf, double
 int pack_chol(afqmc_engine *e)
 {
     const int n = e->n, G = e->G;
-    if (!e->realFlag) TRY(dalloc(e, &e->realFlag, 1));
     int flag = 0;
     CUDA_TRY(cudaMemsetAsync(e->realFlag, 0, sizeof(int), e->stream));
     g_launch_count++;
@@ -480,28 +518,6 @@ int pack_chol(afqmc_engine *e)
     g_launch_count++;
     chol_pack_kernel<<<1184, 256, 0, e->stream>>>(n, G, e->chol, e->cholP);
     return check_launch();
-}
-
-// Real copies of the dense one-body operators, after they were set.
-int refresh_real_operators(afqmc_engine *e)
-{
-    if (e->precision != AFQMC_FP64) return AFQMC_OK;
-    for (int k = 0; k < 3; ++k) {
-        e->expKr[k] = nullptr;
-        if (e->expK[k] && !(e->useLog && e->kind == KIND_PL))
-            TRY(real_copy(e, e->expK[k], (size_t)e->n * e->n, &e->realBuf[k], &e->expKr[k]));
-    }
-    return AFQMC_OK;
-}
-
-int refresh_real_trial(afqmc_engine *e)
-{
-    if (e->precision != AFQMC_FP64) return AFQMC_OK;
-    for (int b = 0; b < e->bl.nblk; ++b) {
-        double *buf = nullptr;
-        if (e->bl.Ns[b] > 0) TRY(real_copy(e, e->phiT[b], (size_t)e->n * e->bl.Ns[b], &buf, &e->phiTr[b]));
-    }
-    return AFQMC_OK;
 }
 
 // Constrained path: whether the trial's columns split into spin-up ones
@@ -1024,9 +1040,9 @@ int afqmc_cp_create(int L, int N, int W, int decomp, int force_type, double dt, 
         CK(gemm(g, e->stream));
     }
     if (precision == AFQMC_MIXED) CK(mixed_create(e));
-    CK(refresh_real_operators(e));
-    CK(refresh_real_trial(e));
     const double *const ops[3] = {expMinusDtK, expHalfDtK, expMinusHalfDtK ? expMinusHalfDtK : expHalfDtK};
+    const double *const trials[2] = {phiT, nullptr};
+    CK(real_operators(e, ops, trials));
     find_spin_blocks(e, phiT, ops);
     e->hd.n0 = e->n0;
     cudaError_t ce = cudaStreamSynchronize(e->stream);
@@ -1110,8 +1126,9 @@ int afqmc_pl_create(int n, int Nup, int Ndn, int G, int W, int force_type, doubl
     CK(dalloc(e, &e->ex, (size_t)G * W));
     CK(dalloc(e, &e->bgNum, G));
     CK(dalloc(e, &e->exNum, G));
-    CK(refresh_real_operators(e));
-    CK(refresh_real_trial(e));
+    const double *const ops[3] = {expMinusDtK, expHalfDtK, expMinusHalfDtK ? expMinusHalfDtK : expHalfDtK};
+    const double *const trials[2] = {phiTUp, Ndn > 0 ? phiTDn : nullptr};
+    CK(real_operators(e, ops, trials));
     if (precision == AFQMC_FP64) {
         if (taylor_f64_supported(n, e->ncol)) CK(pack_chol(e));
         CK(dalloc(e, &e->M, (size_t)m_rows(e) * W));

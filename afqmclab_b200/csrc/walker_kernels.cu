@@ -1,5 +1,7 @@
 // AFQMC walker-step kernels other than the GEMMs (plain FP64 form).
 // Each kernel cites the reference function it replaces.
+#include "lu_block.cuh"
+#include "lu_common.cuh"
 #include "walker_kernels.cuh"
 
 #include <atomic>
@@ -435,169 +437,8 @@ gj_cta_kernel(int W, Blocks bl, const zd *S, zd *Sinv, const int *active, const 
 }
 
 // ---------------------------------------------------------------------------
-// Same contract as lu_kernel for blocks of at most 32 columns, one warp per
-// walker: Gauss-Jordan elimination with the zgetf2 pivot choice (first row
-// of maximal |re|+|im| in the current column), in place in a padded shared
-// tile (lane i owns row i), then the column unscrambling of the recorded row
-// interchanges.  The pivots are the U diagonal of the LU factorisation, so
-// the log-determinant follows logDeterminant (tensor_2d_common_fun.cpp:75-105).
-// ---------------------------------------------------------------------------
-constexpr int GJ_WARPS = 4;
-constexpr int GJ_LD = 33;
-
-__global__ void __launch_bounds__(GJ_WARPS * 32)
-gj_warp_kernel(int W, Blocks bl, const zd *S, zd *Sinv, const int *active, const zd *logw,
-               zd logwAdd, zd logwT, zd *logov, int *alive, int *surv, zd *logwOut, double *weight,
-               int *status, int mode, int wantInverse)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int w = blockIdx.x * GJ_WARPS + warp;
-    if (w >= W) return;
-    zd *A = (zd *)smem_raw + (size_t)warp * 32 * GJ_LD;
-    const bool act = (active == nullptr) || active[w] != 0;
-    if (!act) {
-        if (lane == 0) {
-            if (mode == LU_PROJECT) surv[w] = 0;
-            if (mode == LU_POPWEIGHT) { weight[w] = 0.0; alive[w] = 1; }
-        }
-        return;
-    }
-    bool singular = false;
-    zd logdetSum = make_double2(0.0, 0.0);
-    const bool inv = wantInverse && Sinv;
-    for (int b = 0; b < bl.nblk; ++b) {
-        const int Ns = bl.Ns[b];
-        if (Ns == 0) continue;
-        const zd *Sg = S + (size_t)w * bl.sStride + bl.sOff[b];
-        for (int e = lane; e < Ns * Ns; e += 32) A[(e % Ns) * GJ_LD + e / Ns] = Sg[e];
-        __syncwarp();
-        double lognorm = 0.0;
-        zd phase = make_double2(1.0, 0.0);
-        int myPartner = lane;  // lane k keeps the row interchanged at step k
-        bool sing = false;
-        for (int k = 0; k < Ns; ++k) {
-            double v = (lane >= k && lane < Ns) ? zcabs1(A[lane * GJ_LD + k]) : -1.0;
-            if (!(v == v)) v = INFINITY;   // a NaN row wins: the comparisons below stay a total order
-            int idx = lane;
-            for (int o = 16; o > 0; o >>= 1) {
-                double ov = __shfl_xor_sync(0xffffffffu, v, o);
-                int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-                if (ov > v || (ov == v && oi < idx)) { v = ov; idx = oi; }
-            }
-            // the pivot row steers the warp-wide branches below (each with a
-            // full-mask __syncwarp): every lane takes lane 0's choice
-            const int p = __shfl_sync(0xffffffffu, idx, 0);
-            if (lane == k) myPartner = p;
-            if (p != k) {
-                for (int j = lane; j < Ns; j += 32) {
-                    zd t = A[k * GJ_LD + j];
-                    A[k * GJ_LD + j] = A[p * GJ_LD + j];
-                    A[p * GJ_LD + j] = t;
-                }
-                __syncwarp();
-            }
-            const zd piv = A[k * GJ_LD + k];
-            if (zeq0(piv)) {
-                sing = true;
-                __syncwarp();
-                continue;
-            }
-            const double a = zabs(piv);
-            lognorm += log(a);
-            const zd f = (p != k) ? zneg(piv) : piv;
-            phase = zmul(phase, make_double2(f.x / a, f.y / a));
-            const zd pinv = zdiv(make_double2(1.0, 0.0), piv);
-            __syncwarp();
-            // normalise the pivot row; its column-k entry becomes 1/piv
-            for (int j = lane; j < Ns; j += 32)
-                A[k * GJ_LD + j] = (j == k) ? pinv : zmul(A[k * GJ_LD + j], pinv);
-            __syncwarp();
-            // eliminate column k from every other row (lane i owns row i);
-            // without the inverse only the trailing block below and right of
-            // the pivot (the LU elimination) is needed
-            // (columns in chunks of 8: the chunk's loads are issued before its
-            // stores, which the compiler cannot reorder across the shared tile)
-            const bool elim = inv ? (lane < Ns && lane != k) : (lane > k && lane < Ns);
-            if (elim) {
-                zd *row = A + lane * GJ_LD;
-                const zd *prow = A + k * GJ_LD;
-                const zd dum = row[k];
-                if (inv) row[k] = make_double2(0.0, 0.0);
-                const int j1 = inv ? 0 : k + 1;
-                for (int j0 = j1; j0 < Ns; j0 += 8) {
-                    zd pv[8], r[8];
-#pragma unroll
-                    for (int t = 0; t < 8; ++t)
-                        if (j0 + t < Ns) { pv[t] = prow[j0 + t]; r[t] = row[j0 + t]; }
-#pragma unroll
-                    for (int t = 0; t < 8; ++t)
-                        if (j0 + t < Ns) {
-                            r[t].x -= pv[t].x * dum.x - pv[t].y * dum.y;
-                            r[t].y -= pv[t].x * dum.y + pv[t].y * dum.x;
-                            row[j0 + t] = r[t];
-                        }
-                }
-            }
-            __syncwarp();
-        }
-        // undo the row interchanges as column swaps, last first
-        for (int k = Ns - 1; k >= 0 && inv; --k) {
-            const int p = __shfl_sync(0xffffffffu, myPartner, k);
-            if (p != k && lane < Ns) {
-                zd t = A[lane * GJ_LD + k];
-                A[lane * GJ_LD + k] = A[lane * GJ_LD + p];
-                A[lane * GJ_LD + p] = t;
-            }
-        }
-        __syncwarp();
-        // a singular block adds lognorm -1e300 with phase 1
-        // (lognormPhaseDeterminant, tensor_2d_common_fun.cpp:75-84)
-        if (sing) {
-            singular = true;
-            logdetSum = zadd(logdetSum, make_double2(-1e300, 0.0));
-        } else {
-            zd ld = zadd(make_double2(lognorm, 0.0), zlog(phase));
-            logdetSum = zadd(logdetSum, ld);
-        }
-        if (wantInverse && Sinv) {
-            zd *Xg = Sinv + (size_t)w * bl.sStride + bl.sOff[b];
-            for (int e = lane; e < Ns * Ns; e += 32) Xg[e] = A[(e % Ns) * GJ_LD + e / Ns];
-        }
-        __syncwarp();
-    }
-    if (lane == 0) {
-        zd lwR = zadd(logwAdd, logw[w]);
-        if (bl.mult == 2) logdetSum = zadd(logdetSum, logdetSum);
-        zd lo = zadd(zadd(zconj(logwT), lwR), logdetSum);
-        logov[w] = lo;
-        if (singular && status) atomicOr(status + w, (int)ST_SINGULAR);
-        if (!(isfinite(lo.x) && isfinite(lo.y)) && status && !singular) atomicOr(status + w, (int)ST_NONFINITE);
-        if (mode == LU_PROJECT) {
-            double ph = lo.y;
-            double c = cos(ph);
-            if (c <= 0.0) {
-                alive[w] = 0; surv[w] = 0;
-            } else {
-                logwOut[w] = zadd(logw[w], make_double2(log(c), -ph));
-                surv[w] = 1;
-            }
-        } else if (mode == LU_POPWEIGHT) {
-            zd e = zexp(lo);
-            if (e.x <= 0.0) {
-                weight[w] = 0.0;
-            } else {
-                weight[w] = e.x;
-                logwOut[w] = zsub(logw[w], lo);
-            }
-            alive[w] = 1;
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
 // Gauss-Jordan with the matrix in registers (gj_regw_kernel below), same
-// contract as gj_warp_kernel for one or two blocks of 17..64 columns: each
+// contract as lu_kernel for one or two blocks of 17..32 columns: each
 // row lives in registers (padded with zeros to the window; only Ns steps
 // run, after which the last Ns window slots hold the inverse columns).  The
 // column loop is not unrolled; instead every row rotates by one slot per
@@ -626,99 +467,10 @@ __device__ __forceinline__ zd zrcp(zd b)
     return make_double2(r * d, -d);
 }
 
-// A rank that orders candidates like the pivot search: for values >= +0 the
-// IEEE bits are monotonic; NaN ranks as infinity; ineligible rows rank 0.
-__device__ __forceinline__ unsigned long long gr_rank(zd a0, bool eligible)
-{
-    double v = zcabs1(a0);
-    if (!(v == v)) v = INFINITY;
-    return eligible ? (unsigned long long)__double_as_longlong(v) + 1ull : 0ull;
-}
-
-// 1 / b without a division, so that it schedules between other arithmetic:
-// b is scaled by a power of two (exact) so that max(|re|, |im|) lies in
-// [1, 2), the real reciprocal y of d = |b|^2 in [1, 8) starts from the
-// single-precision approximation and takes two Newton-Raphson steps
-// y <- y + y (1 - d y), each of which doubles the correct bits (about 21 ->
-// 42 -> full precision), and 1/b = s conj(b s) y.  Within a few ulp of the
-// rounded quotient; a NaN or infinite b gives NaN (callers test zero first).
-__device__ __forceinline__ zd zrcp_nr(zd b)
-{
-    const double m = fmax(fabs(b.x), fabs(b.y));
-    const long long e = (__double_as_longlong(m) >> 52) & 0x7ff;
-    const double s = __longlong_as_double((2046 - e) << 52);   // 2^(1023 - e)
-    const double xs = b.x * s, ys = b.y * s;
-    const double d = fma(xs, xs, ys * ys);
-    double y = (double)__fdividef(1.0f, (float)d);
-    y = fma(y, fma(-d, y, 1.0), y);
-    y = fma(y, fma(-d, y, 1.0), y);
-    const double t = y * s;
-    return make_double2(xs * t, -ys * t);
-}
-
-// Position of the warp's best candidate: largest rank, then lowest position.
-__device__ __forceinline__ int gr_warp_best(unsigned long long u, int pos)
-{
-    const unsigned hi = (unsigned)(u >> 32), lo = (unsigned)u;
-    const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
-    const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
-    const unsigned key = (hi == mhi && lo == mlo) ? (unsigned)pos : 0xffffffffu;
-    return (int)__reduce_min_sync(0xffffffffu, key);
-}
-
-// Per-walker finish of the block log-determinants: the overlap's log and,
-// by mode, the constraint or the population weight.  ldB/sgB hold the
-// walker's nb block log-determinants and singular flags.
-__device__ void lu_walker_finish(int w, bool act, int nb, int mult, const zd *ldB, const int *sgB,
-                                 const zd *logw, zd logwAdd, zd logwT, zd *logov, int *alive, int *surv,
-                                 zd *logwOut, double *weight, int *status, int mode)
-{
-    if (!act) {
-        if (mode == LU_PROJECT) surv[w] = 0;
-        if (mode == LU_POPWEIGHT) { weight[w] = 0.0; alive[w] = 1; }
-        return;
-    }
-    bool singular = false;
-    zd logdetSum = make_double2(0.0, 0.0);
-    // a singular block adds lognorm -1e300 with phase 1
-    // (lognormPhaseDeterminant, tensor_2d_common_fun.cpp:75-84)
-    for (int t = 0; t < nb; ++t) {
-        const bool sb = sgB[t] != 0;
-        singular = singular || sb;
-        logdetSum = zadd(logdetSum, sb ? make_double2(-1e300, 0.0) : ldB[t]);
-    }
-    const zd lwR = zadd(logwAdd, logw[w]);
-    if (mult == 2) logdetSum = zadd(logdetSum, logdetSum);
-    const zd lo = zadd(zadd(zconj(logwT), lwR), logdetSum);
-    logov[w] = lo;
-    if (singular && status) atomicOr(status + w, (int)ST_SINGULAR);
-    if (!(isfinite(lo.x) && isfinite(lo.y)) && status && !singular) atomicOr(status + w, (int)ST_NONFINITE);
-    if (mode == LU_PROJECT) {
-        const double ph = lo.y;
-        const double c = cos(ph);
-        if (c <= 0.0) {
-            alive[w] = 0; surv[w] = 0;
-        } else {
-            logwOut[w] = zadd(logw[w], make_double2(log(c), -ph));
-            surv[w] = 1;
-        }
-    } else if (mode == LU_POPWEIGHT) {
-        const zd e = zexp(lo);
-        if (e.x <= 0.0) {
-            weight[w] = 0.0;
-        } else {
-            weight[w] = e.x;
-            logwOut[w] = zsub(logw[w], lo);
-        }
-        alive[w] = 1;
-    }
-}
-
 // ---------------------------------------------------------------------------
 // The same rotated Gauss-Jordan with the window split between two column
-// halves, one CTA per matrix: RH row halves x 2 column halves of SL slots
-// (RH = 2, SL = 32 for blocks of 33-64 columns, four warps; RH = 1, SL = 16
-// for 17-32 columns, two warps).  Warp (rh, ch) holds rows rh*32+lane and
+// halves of SL = 16 slots, one warp each, one CTA per matrix.  Warp ch holds rows
+// 0..31 and
 // half ch of a 2 SL-column window that moves by one column per step.  The half-0 warps hold
 // the current column in slot 0; while they update step k they already search
 // the pivot of step k+1 in their new slot 0 (max |re|+|im|, ties to the lower
@@ -728,8 +480,7 @@ __device__ void lu_walker_finish(int w, bool act, int nb, int mult, const zd *ld
 //     slot of every row (and of the pivot row) is the updated slot 0 of half
 //     1 from the step before, passed through shared memory;
 //   - half 1 takes its factor f = a_k * (1/piv) from the published column k,
-//     the pivot row's lane writes its half-1 row, a barrier of the half-1
-//     warps, then half 1 updates and takes the new inverse column in its last
+//     the pivot row's lane writes its half-1 row, then half 1 updates and takes the new inverse column in its last
 //     slot.
 // Shared buffers alternate between even and odd steps, so the only CTA-wide
 // barrier per step is the one that publishes step k+1's inputs.
@@ -745,39 +496,33 @@ __device__ void lu_walker_finish(int w, bool act, int nb, int mult, const zd *ld
 struct GR64Cand {
     unsigned long long u;   // rank of the candidate: bits of |re|+|im| plus one, 0 if not eligible
     int key;                // its position
-    int row;                // its row (rh*32+lane)
+    int row;                // its row
     zd a0;                  // its value in the current column
     zd q;                   // 1 / a0, zero when a0 is zero
 };
 
-// named barrier 1 of the column groups other than 0
-__device__ __forceinline__ void upper_groups_bar(int threads)
-{
-    asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
-}
-
-template <int NB, int SL, int RH, int NQ>
-__global__ void __launch_bounds__(32 * RH * NQ, SL == 16 ? 65536 / (32 * RH * NQ * 128) : 2)
+template <int NB>
+__global__ void __launch_bounds__(64, 8)
 gj_regw_kernel(int W, Blocks bl, const zd *S, zd *Sinv, float *Sinv32, long long s32, const int *active,
                 const zd *logw, zd logwAdd, zd logwT, zd *logov, int *alive, int *surv, zd *logwOut,
                 double *weight, int *status, int mode, int wantInverse)
 {
-    constexpr int NR = 32 * RH;                      // rows of the window
-    __shared__ __align__(16) zd prowC[2][RH][SL];   // [step parity][rh]: half 0 of each warp's candidate
-    __shared__ __align__(16) zd prowQ[NQ][SL];      // [cq >= 1]: column group cq of the pivot row
+    constexpr int SL = 16, NR = 32;                 // slots per half, rows of the window
+    __shared__ __align__(16) zd prowC[2][SL];       // [step parity]: half 0 of the candidate
+    __shared__ __align__(16) zd prowQ[SL];          // half 1 of the pivot row
     __shared__ __align__(16) zd colS[2][NR];        // [step parity][row]: the current column
-    __shared__ __align__(16) zd xS[NQ][2][NR];      // [cq >= 1][step parity][row]: group cq's updated slot 0
-    __shared__ __align__(16) GR64Cand cand[2][RH];  // [step parity][rh]
+    __shared__ __align__(16) zd xS[2][NR];          // [step parity][row]: half 1's updated slot 0
+    __shared__ __align__(16) GR64Cand cand[2];   // [step parity]
     __shared__ __align__(16) zd pivS[NR];
-    __shared__ __align__(16) zd phS[RH];
-    __shared__ double lnS[RH];
+    __shared__ zd phS;
+    __shared__ double lnS;
     __shared__ int pvS[NR];
     __shared__ int jxS[NR];
     __shared__ zd ldS;
     __shared__ int sgS;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rh = warp / NQ, ch = warp % NQ;   // ch: the column group
-    const int r = rh * 32 + lane;
+    const int ch = warp;   // the column half
+    const int r = lane;
     const int w = NB == 1 ? (int)blockIdx.x : (int)(blockIdx.x >> 1);
     const int b = NB == 1 ? 0 : (int)(blockIdx.x & 1);
     const bool act = (active == nullptr) || active[w] != 0;
@@ -795,9 +540,9 @@ gj_regw_kernel(int W, Blocks bl, const zd *S, zd *Sinv, float *Sinv32, long long
             a[s] = (r < Ns && c < Ns) ? Sg[r + (size_t)Ns * c] : make_double2(0.0, 0.0);
         }
         int pos = r;
-        // step 0's inputs, as if a step -1 had produced them: each group's
-        // last slot as the next group's "updated slot 0"
-        if (ch < NQ - 1) xS[ch + 1][1][r] = a[SL - 1];
+        // step 0's inputs, as if a step -1 had produced them: half 0's last slot as
+        // half 1's "updated slot 0"
+        if (ch == 0) xS[1][r] = a[SL - 1];
         if (ch == 0) {
             colS[0][r] = a[0];
             const unsigned long long u = gr_rank(a[0], true);
@@ -805,25 +550,19 @@ gj_regw_kernel(int W, Blocks bl, const zd *S, zd *Sinv, float *Sinv32, long long
                 GR64Cand c;
                 c.u = u; c.key = pos; c.row = r; c.a0 = a[0];
                 c.q = zeq0(a[0]) ? make_double2(0.0, 0.0) : zrcp_nr(a[0]);
-                cand[0][rh] = c;
+                cand[0] = c;
 #pragma unroll
-                for (int s = 0; s < SL - 1; ++s) prowC[0][rh][s] = a[s];
+                for (int s = 0; s < SL - 1; ++s) prowC[0][s] = a[s];
             }
         }
 #pragma unroll 1
         for (int k = 0; k < Ns; ++k) {
             __syncthreads();   // step k's candidates, column, half-0 rows and half 1's last slots
             const int cb = k & 1, pb = cb ^ 1;
-            int second = 0;
-            if constexpr (RH == 2) {
-                const unsigned long long u0 = cand[cb][0].u, u1 = cand[cb][1].u;
-                const int k0 = cand[cb][0].key, k1 = cand[cb][1].key;
-                second = (u1 > u0 || (u1 == u0 && k1 < k0)) ? 1 : 0;
-            }
-            const int p = cand[cb][second].key;
-            const zd q = cand[cb][second].q;
+            const int p = cand[cb].key;
+            const zd q = cand[cb].q;
             if (threadIdx.x == 0) {
-                const zd piv = cand[cb][second].a0;
+                const zd piv = cand[cb].a0;
                 pvS[k] = p;
                 pivS[k] = piv;
                 sing = sing || zeq0(piv);
@@ -832,9 +571,9 @@ gj_regw_kernel(int W, Blocks bl, const zd *S, zd *Sinv, float *Sinv32, long long
             if (pos == k) pos = p;
             if (isP) pos = k;
             if (ch == 0) {
-                a[SL - 1] = xS[1][pb][r];
-                const zd *pr = prowC[cb][second];
-                const zd pLast = xS[1][pb][cand[cb][second].row];
+                a[SL - 1] = xS[pb][r];
+                const zd *pr = prowC[cb];
+                const zd pLast = xS[pb][cand[cb].row];
                 const zd f = isP ? make_double2(0.0, 0.0) : zmul(a[0], q);
                 {
                     const zd pv = pr[1];
@@ -859,40 +598,36 @@ gj_regw_kernel(int W, Blocks bl, const zd *S, zd *Sinv, float *Sinv32, long long
                     GR64Cand c;
                     c.u = u; c.key = pos; c.row = r; c.a0 = a[0];
                     c.q = qn;
-                    cand[pb][rh] = c;
+                    cand[pb] = c;
 #pragma unroll
-                    for (int s = 0; s < SL - 1; ++s) prowC[pb][rh][s] = a[s];
+                    for (int s = 0; s < SL - 1; ++s) prowC[pb][s] = a[s];
                 }
             } else {
-                // a middle group's last slot: its right neighbour's slot 0 of step k-1
-                if (ch < NQ - 1) a[SL - 1] = xS[ch + 1][pb][r];
                 const zd f = isP ? make_double2(0.0, 0.0) : zmul(colS[cb][r], q);
-                zd *pq = prowQ[ch];
+                zd *pq = prowQ;
                 if (isP) {
 #pragma unroll
                     for (int s = 0; s < SL; ++s) pq[s] = a[s];
                 }
-                if constexpr (RH * (NQ - 1) > 1) upper_groups_bar(32 * RH * (NQ - 1));
-                else __syncwarp();
+                __syncwarp();
                 zd x;
                 x.x = fma(-f.x, pq[0].x, fma(f.y, pq[0].y, a[0].x));
                 x.y = fma(-f.x, pq[0].y, fma(-f.y, pq[0].x, a[0].y));
-                xS[ch][cb][r] = x;
+                xS[cb][r] = x;
 #pragma unroll
                 for (int s = 1; s < SL; ++s) {
                     const zd pv = pq[s];
                     a[s - 1].x = fma(-f.x, pv.x, fma(f.y, pv.y, a[s].x));
                     a[s - 1].y = fma(-f.x, pv.y, fma(-f.y, pv.x, a[s].y));
                 }
-                // the last group takes the new inverse column; the others
-                // take their neighbour's slot 0 at the next step
-                if (ch == NQ - 1) a[SL - 1] = isP ? make_double2(1.0, 0.0) : zneg(f);
+                // the new inverse column; half 0 takes half 1's slot 0 at the next step
+                a[SL - 1] = isP ? make_double2(1.0, 0.0) : zneg(f);
             }
         }
         if (threadIdx.x == 0) sgS = sing ? 1 : 0;
         __syncthreads();   // last slots of step Ns-1, all pivots
         sing = sgS != 0;
-        if (ch < NQ - 1) a[SL - 1] = xS[ch + 1][(Ns - 1) & 1][r];
+        if (ch == 0) a[SL - 1] = xS[(Ns - 1) & 1][r];
         const bool real = r < Ns;   // padding rows keep positions >= Ns
         const zd myD = real ? pivS[pos] : make_double2(1.0, 0.0);
         if (ch == 0) {
@@ -913,18 +648,15 @@ gj_regw_kernel(int W, Blocks bl, const zd *S, zd *Sinv, float *Sinv32, long long
                 t.y = __shfl_xor_sync(0xffffffffu, ph.y, o);
                 ph = zmul(ph, t);
             }
-            if (lane == 0) { lnS[rh] = ln; phS[rh] = ph; }
+            if (lane == 0) { lnS = ln; phS = ph; }
             if (real) jxS[pos] = r;
         }
         __syncthreads();
-        if (threadIdx.x == 0 && !sing) {
-            if constexpr (RH == 2) ld = zadd(make_double2(lnS[0] + lnS[1], 0.0), zlog(zmul(phS[0], phS[1])));
-            else ld = zadd(make_double2(lnS[0], 0.0), zlog(phS[0]));
-        }
+        if (threadIdx.x == 0 && !sing) ld = zadd(make_double2(lnS, 0.0), zlog(phS));
         if (inv && real) {
-            // window slot t = SL ch + s holds interchanged column j = t - (NQ SL - Ns)
+            // window slot t = SL ch + s holds interchanged column j = t - (2 SL - Ns)
             const zd sc = sing ? make_double2(0.0, 0.0) : zrcp(myD);
-            const int j0 = ch * SL - (NQ * SL - Ns);
+            const int j0 = ch * SL - (2 * SL - Ns);
             if (Sinv32) {
                 // fp32 planes [re | im], each Ns x Ns column-major
                 float *Xr = Sinv32 + (size_t)w * s32 + 2 * sOff, *Xi = Xr + (size_t)Ns * Ns;
@@ -2110,20 +1842,18 @@ void launch_lu_logdet_inverse(int W, const Blocks &bl, zd *S, zd *Sinv, const in
 
 // the split-window register LU: one CTA per block, the two blocks of a
 // two-block walker as a cluster of two CTAs
-template <int SL, int RH, int NQ>
 static void launch_regw(int W, const Blocks &bl, zd *S, zd *X64, float *Sinv32, long long s32, const int *active,
                         const zd *logw, zd logwAdd, zd logwT, zd *logov, int *alive, int *surv, zd *logwOut,
                         double *weight, int *status, int mode, int inv, cudaStream_t s)
 {
-    constexpr int T = 32 * RH * NQ;
     if (bl.nblk == 1) {
-        gj_regw_kernel<1, SL, RH, NQ><<<W, T, 0, s>>>(W, bl, S, X64, Sinv32, s32, active, logw, logwAdd, logwT,
+        gj_regw_kernel<1><<<W, 64, 0, s>>>(W, bl, S, X64, Sinv32, s32, active, logw, logwAdd, logwT,
                                                       logov, alive, surv, logwOut, weight, status, mode, inv);
         return;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(2 * W));
-    cfg.blockDim = dim3(T);
+    cfg.blockDim = dim3(64);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -2132,7 +1862,7 @@ static void launch_regw(int W, const Blocks &bl, zd *S, zd *X64, float *Sinv32, 
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, gj_regw_kernel<2, SL, RH, NQ>, W, bl, (const zd *)S, X64, Sinv32, s32, active, logw,
+    cudaLaunchKernelEx(&cfg, gj_regw_kernel<2>, W, bl, (const zd *)S, X64, Sinv32, s32, active, logw,
                        logwAdd, logwT, logov, alive, surv, logwOut, weight, status, mode, inv);
 }
 
@@ -2144,14 +1874,19 @@ void launch_lu_logdet_inverse32(int W, const Blocks &bl, zd *S, zd *Sinv, float 
     int maxNs = 0;
     for (int b = 0; b < bl.nblk; ++b) maxNs = bl.Ns[b] > maxNs ? bl.Ns[b] : maxNs;
     const long long s32 = sinv32_stride(bl);
-    if (maxNs > 16 && maxNs <= 64 && (bl.nblk == 1 || bl.nblk == 2)) {
+    // 17 to 32 columns stay element-wise where many matrices share an SM: its two
+    // warps per matrix take 0.074 ms for 2048 blocks of 32 columns against 0.094,
+    // 0.045 for 1024 against 0.052; up to four matrices per SM the blocked kernel's
+    // shorter steps win (23 columns, 333 matrices: 20.9 us against 23.1)
+    if ((maxNs <= 16 || maxNs > 32 || (long long)W * bl.nblk <= 592) && lu_block_supported(bl)) {
+        lu_block(W, bl, S, Sinv32 ? nullptr : Sinv, Sinv32, active, logw, logwAdd, logwT, logov, alive, surv, logwOut,
+                 weight, status, mode, wantInverse, s);
+        return;
+    }
+    if (maxNs > 16 && maxNs <= 32) {
         g_launch_count++;
-        if (maxNs <= 32)
-            launch_regw<16, 1, 2>(W, bl, S, Sinv32 ? nullptr : Sinv, Sinv32, s32, active, logw, logwAdd, logwT, logov,
-                               alive, surv, logwOut, weight, status, mode, wantInverse ? 1 : 0, s);
-        else
-            launch_regw<32, 2, 2>(W, bl, S, Sinv32 ? nullptr : Sinv, Sinv32, s32, active, logw, logwAdd, logwT, logov,
-                               alive, surv, logwOut, weight, status, mode, wantInverse ? 1 : 0, s);
+        launch_regw(W, bl, S, Sinv32 ? nullptr : Sinv, Sinv32, s32, active, logw, logwAdd, logwT, logov, alive, surv,
+                    logwOut, weight, status, mode, wantInverse ? 1 : 0, s);
         return;
     }
     launch_lu_fp64(W, bl, S, Sinv, active, logw, logwAdd, logwT, logov, alive, surv, logwOut, weight, status,
@@ -2169,34 +1904,15 @@ static void launch_lu_fp64(int W, const Blocks &bl, zd *S, zd *Sinv, const int *
     g_launch_count++;
     int maxNs = 0;
     for (int b = 0; b < bl.nblk; ++b) maxNs = bl.Ns[b] > maxNs ? bl.Ns[b] : maxNs;
-    if (maxNs <= 32) {
-        const size_t smem = (size_t)GJ_WARPS * 32 * GJ_LD * sizeof(zd);
-        static std::atomic<unsigned long long> gattr{0};
-        if (first_on_device(gattr)) {
-            cudaFuncSetAttribute(gj_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        }
-        gj_warp_kernel<<<(W + GJ_WARPS - 1) / GJ_WARPS, GJ_WARPS * 32, smem, s>>>(
-            W, bl, S, Sinv, active, logw, logwAdd, logwT, logov, alive, surv, logwOut, weight, status,
-            mode, wantInverse ? 1 : 0);
-        return;
-    }
     if (maxNs <= GJ_CTA_MAX_NS) {
         const size_t smem = gj_cta_smem(maxNs);
         static std::atomic<unsigned long long> cattr{0};
         if (first_on_device(cattr)) {
-            cudaFuncSetAttribute(gj_cta_kernel<256, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)gj_cta_smem(64));
             cudaFuncSetAttribute(gj_cta_kernel<512, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)gj_cta_smem(GJ_CTA_MAX_NS));
         }
-        if (maxNs <= 64)
-            gj_cta_kernel<256, 2><<<W, 256, smem, s>>>(W, bl, S, Sinv, active, logw, logwAdd, logwT, logov,
-                                                        alive, surv, logwOut, weight, status, mode,
-                                                        wantInverse ? 1 : 0, maxNs);
-        else
-            gj_cta_kernel<512, 4><<<W, 512, smem, s>>>(W, bl, S, Sinv, active, logw, logwAdd, logwT, logov,
-                                                        alive, surv, logwOut, weight, status, mode,
-                                                        wantInverse ? 1 : 0, maxNs);
+        gj_cta_kernel<512, 4><<<W, 512, smem, s>>>(W, bl, S, Sinv, active, logw, logwAdd, logwT, logov, alive, surv,
+                                                    logwOut, weight, status, mode, wantInverse ? 1 : 0, maxNs);
         return;
     }
     if (maxNs <= LU_SMEM_MAX_NS) {
