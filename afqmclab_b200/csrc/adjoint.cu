@@ -55,22 +55,42 @@
 
 namespace {
 
+// Sums over walkers: a CTA takes 32 entries, its ADJ_Y rows of threads every
+// ADJ_Y-th walker each, and their partial sums meet in shared memory in a fixed
+// order.  One thread per entry left most of the SMs without work (n = 128, 512
+// walkers: 259 -> 24 us for adj_r_kernel, 156 -> 13 for adj_grad_kernel).
+constexpr int ADJ_X = 32, ADJ_Y = 16;
+
+__device__ __forceinline__ zd adj_sum_rows(zd v, zd (*part)[ADJ_X])
+{
+    __syncthreads();   // the last sum has been read
+    part[threadIdx.y][threadIdx.x] = v;
+    __syncthreads();
+    zd r = part[0][threadIdx.x];
+    for (int y = 1; y < ADJ_Y; ++y) r = zadd(r, part[y][threadIdx.x]);
+    return r;
+}
+
 // R^T_s += den_w thetaT_s, the unweighted sum (log-overlap) and
 // Et = sum_w den_w (E_w - E) thetaT_w
-__global__ void adj_r_kernel(int W, long long Ktot, long long tStride, const zd *thetaT,
-                             const int *alive, const zd *den, const zd *eloc, zd Emix, zd *Rt, zd *St,
-                             zd *Et)
+__global__ void __launch_bounds__(ADJ_X * ADJ_Y)
+adj_r_kernel(int W, long long Ktot, long long tStride, const zd *thetaT, const int *alive, const zd *den,
+             const zd *eloc, zd Emix, zd *Rt, zd *St, zd *Et)
 {
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < Ktot;
-         e += (long long)gridDim.x * blockDim.x) {
-        zd r = make_double2(0, 0), q = make_double2(0, 0), t = make_double2(0, 0);
-        for (int w = 0; w < W; ++w) {
-            if (!alive[w]) continue;
-            const zd x = thetaT[(size_t)w * tStride + e];
-            zfma(r, den[w], x);
-            q = zadd(q, x);
-            zfma(t, zmul(den[w], zsub(eloc[w], Emix)), x);
-        }
+    __shared__ zd part[ADJ_Y][ADJ_X];
+    const long long e = blockIdx.x * (long long)ADJ_X + threadIdx.x;
+    zd r = make_double2(0, 0), q = make_double2(0, 0), t = make_double2(0, 0);
+    for (int w = threadIdx.y; e < Ktot && w < W; w += ADJ_Y) {
+        if (!alive[w]) continue;
+        const zd x = thetaT[(size_t)w * tStride + e];
+        zfma(r, den[w], x);
+        q = zadd(q, x);
+        zfma(t, zmul(den[w], zsub(eloc[w], Emix)), x);
+    }
+    r = adj_sum_rows(r, part);
+    q = adj_sum_rows(q, part);
+    t = adj_sum_rows(t, part);
+    if (e < Ktot && threadIdx.y == 0) {
         Rt[e] = r;
         St[e] = q;
         Et[e] = t;
@@ -120,19 +140,24 @@ __global__ void adj_h_kernel(long long K, int W, const zd *Tt, const zd *Z, cons
 
 // gradT(b + Ns i) = [sum_s Vp_s + TR - sum_w P_w](i, b) + Et(b + Ns i); the
 // n x Ns matrices are column-major, the gradient in the thetaT layout
-__global__ void adj_grad_kernel(int n, int Ns, int S, const zd *Vp, const zd *TR, int W, const zd *Pw,
-                                const int *alive, const zd *Et, double *grad)
+__global__ void __launch_bounds__(ADJ_X * ADJ_Y)
+adj_grad_kernel(int n, int Ns, int S, const zd *Vp, const zd *TR, int W, const zd *Pw, const int *alive,
+                const zd *Et, double *grad)
 {
+    __shared__ zd part[ADJ_Y][ADJ_X];
     const long long cnt = (long long)n * Ns;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < cnt;
-         e += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(e % n), b = (int)(e / n);
-        zd v = TR[e];
-        for (int s = 0; s < S; ++s) v = zadd(v, Vp[(size_t)s * cnt + e]);
-        for (int w = 0; w < W; ++w)
+    const long long e = blockIdx.x * (long long)ADJ_X + threadIdx.x;
+    zd v = make_double2(0, 0);
+    if (e < cnt) {
+        for (int s = threadIdx.y; s < S; s += ADJ_Y) v = zadd(v, Vp[(size_t)s * cnt + e]);
+        for (int w = threadIdx.y; w < W; w += ADJ_Y)
             if (alive[w]) v = zsub(v, Pw[(size_t)w * cnt + e]);
+    }
+    v = adj_sum_rows(v, part);
+    if (e < cnt && threadIdx.y == 0) {
+        const int i = (int)(e % n), b = (int)(e / n);
         const size_t t = (size_t)b + (size_t)Ns * i;
-        v = zadd(v, Et[t]);
+        v = zadd(zadd(v, TR[e]), Et[t]);
         grad[2 * t] = v.x;
         grad[2 * t + 1] = v.y;
     }
@@ -195,15 +220,41 @@ __global__ void adj_conj_kernel(long long count, const zd *src, zd *dst)
         dst[e] = zconj(src[e]);
 }
 
-// Device scratch of one adjoint evaluation, freed on every return path
-// (cudaFree waits for the work in flight).
+// Device scratch of one adjoint evaluation: the engine's slots, in the order
+// of the requests, kept for its next evaluation and freed with it (about
+// (4 n max(Nup, Ndn) W + G W) complex numbers, 4 % of the engine at n = 256; a call
+// ends with the stream idle, so the next one may reuse them on any stream).
+// Allocated and freed on every call they cost more than the work: n = 128, 512
+// walkers, 11-280 ms a call of which 6.2 ms were kernels.  The staging copy of a
+// gradient that goes to host memory, as large as the gradient, is freed on
+// return (once).
 struct DevBufs {
+    afqmc_engine *e;
+    size_t next = 0;
     std::vector<void *> p;
+    explicit DevBufs(afqmc_engine *e_) : e(e_) {}
     ~DevBufs()
     {
-        for (void *q : p) cudaFree(q);
+        for (void *q : p) cudaFree(q);   // waits for the work in flight
     }
     template <class T> cudaError_t get(T **out, size_t count)
+    {
+        *out = nullptr;
+        const size_t bytes = sizeof(T) * std::max<size_t>(count, 1);
+        if (next == e->adjSlots.size()) e->adjSlots.push_back({nullptr, 0});
+        auto &s = e->adjSlots[next];
+        if (s.bytes < bytes) {
+            if (s.p) cudaFree(s.p);
+            s = {nullptr, 0};
+            cudaError_t c = cudaMalloc(&s.p, bytes);
+            if (c != cudaSuccess) { s.p = nullptr; return c; }
+            s.bytes = bytes;
+        }
+        ++next;
+        *out = (T *)s.p;
+        return cudaSuccess;
+    }
+    template <class T> cudaError_t once(T **out, size_t count)
     {
         *out = nullptr;
         cudaError_t c = cudaMalloc((void **)out, sizeof(T) * std::max<size_t>(count, 1));
@@ -484,7 +535,7 @@ int adjoint_gemm(AdjCtx &c, int nb, int mult)
             g.A = e->tdev; g.lda = n; g.B = c.Rt + tOff; g.ldb = Ns; g.C = TR; g.ldc = n;
             AGM(g);
         }
-        adj_grad_kernel<<<(int)std::min<long long>((K + 255) / 256, 1184), 256, 0, s>>>(
+        adj_grad_kernel<<<(unsigned)((K + ADJ_X - 1) / ADJ_X), dim3(ADJ_X, ADJ_Y), 0, s>>>(
             n, Ns, slots, Vp, TR, W, Pw, e->alive, c.Et + tOff, c.gradT + 2 * tOff);
         ACK(cudaGetLastError());
         first = false;
@@ -505,7 +556,7 @@ extern "C" int afqmc_pl_adjoint(afqmc_engine *e, double *energy, double *mean_lo
     if (!e || e->kind != KIND_PL) return engine_fail(AFQMC_ERR_ARG, "phaseless engine required");
     const int W = e->W, n = e->n, G = e->G;
     cudaStream_t s = e->stream;
-    DevBufs bufs;
+    DevBufs bufs(e);
 #define ACK(x) do { cudaError_t _c = (x); if (_c != cudaSuccess) return engine_fail(AFQMC_ERR_CUDA, cudaGetErrorString(_c)); } while (0)
     // the GEMM form for real half-rotated vectors; block 0 alone, counted
     // twice, for a spin-restricted trial (the walker's one orbital matrix
@@ -558,9 +609,9 @@ extern "C" int afqmc_pl_adjoint(afqmc_engine *e, double *energy, double *mean_lo
             cudaGetLastError();
         }
         if (cholDev) dchol = (zd *)dE_dchol;
-        else ACK(bufs.get(&dchol, (size_t)n * n * G));
+        else ACK(bufs.once(&dchol, (size_t)n * n * G));
     }
-    adj_r_kernel<<<256, 256, 0, s>>>(W, Ktot, e->bl.tStride, e->thetaT, e->alive, e->den, e->eloc, Emix,
+    adj_r_kernel<<<(unsigned)((Ktot + ADJ_X - 1) / ADJ_X), dim3(ADJ_X, ADJ_Y), 0, s>>>(W, Ktot, e->bl.tStride, e->thetaT, e->alive, e->den, e->eloc, Emix,
                                      Rt, St, Et);
     ACK(cudaGetLastError());
     AdjCtx c;

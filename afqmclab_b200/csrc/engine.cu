@@ -858,6 +858,7 @@ void free_engine(afqmc_engine *e)
     }
     if (e->upStream) cudaStreamDestroy(e->upStream);
     for (void *p : e->allocs) cudaFree(p);
+    for (auto &sl : e->adjSlots) cudaFree(sl.p);
     if (e->own) cudaStreamDestroy(e->own);
     delete e;
 }

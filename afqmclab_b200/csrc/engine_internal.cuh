@@ -112,6 +112,9 @@ struct afqmc_engine {
     cudaGraphExec_t graphExec[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     long long graphKernels[5] = {0, 0, 0, 0, 0};  // kernel nodes per graph
     std::vector<void *> allocs;
+    // device scratch of the adjoint, kept between evaluations (adjoint.cu)
+    struct Slot { void *p; size_t bytes; };
+    std::vector<Slot> adjSlots;
 };
 
 // Phase timing: record an event pair around a phase when profiling is on.
