@@ -20,9 +20,9 @@
 // launch per order up to the cap: n = 128, N = 32, 2048 walkers 7.44 -> 2.49 ms;
 // n = 64, N = 16, 512 walkers 0.761 -> 0.113; n = 90, N = 21, 300 walkers 1.17 ->
 // 0.338; n = 256, N = 64, 512 walkers 7.37 -> 5.59.  From the panels of a
-// symmetric M (and a real one-body operator): 2.57, 0.116, 0.336 and 6.19; the
+// symmetric M (and a real one-body operator): 2.49, 0.111, 0.314 and 6.01; the
 // mirrored rows cost loads here, and the M-build that writes them loses half
-// its products (2.87 -> 1.58, 0.117 -> 0.064, 0.123 -> 0.083, 5.68 -> 2.96 ms).
+// its products (2.87 -> 1.45, 0.117 -> 0.060, 0.123 -> 0.077, 5.68 -> 2.74 ms).
 #include <cooperative_groups.h>
 #include <math_constants.h>
 
@@ -129,6 +129,14 @@ struct TfStream {
         for (int i = 0; i < 2; ++i)
 #pragma unroll
             for (int j = 0; j < 2; ++j) c.r[i][j][0] = c.r[i][j][1] = c.i[i][j][0] = c.i[i][j][1] = 0.0;
+        // both 8-column blocks (no branch between the products), or the first alone
+        if (nb == 2) stages<true>(smem, T, ldt, wr, fr, fk, nb, c);
+        else stages<false>(smem, T, ldt, wr, fr, fk, nb, c);
+    }
+    template <bool FULL>
+    __device__ __forceinline__ void stages(const unsigned char *smem, const zd *T, int ldt, int wr, int fr, int fk,
+                                           int nb, TfAcc &c)
+    {
         for (int kt = 0; kt < KT; ++kt, ++it) {
             cp_async_wait<TF_STAGES - 2>();
             __syncthreads();
@@ -148,7 +156,7 @@ struct TfStream {
                 }
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
-                    if (j >= nb) continue;
+                    if (!FULL && j >= nb) continue;
                     const zd b = T[(size_t)(8 * j + fr) * ldt + kt * TF_BK + k4 + fk];
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {

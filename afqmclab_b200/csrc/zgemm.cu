@@ -7,7 +7,11 @@
 // bound by its fragment loads.  One B200, before and after: M-build (16384 x
 // 2048 x 640, real A) 4.14 -> 2.83 ms (30.3 TFLOP/s), exchange of n = 128, 32
 // electrons, 640 vectors and 2048 walkers 17.1 -> 10.7 ms, one-body product
-// of 1024 128 x 56 walkers 0.465 -> 0.27 ms.
+// of 1024 128 x 56 walkers 0.465 -> 0.27 ms.  Without a branch between the
+// products of a warp whose tile lies inside C, 10 % more: 8704 x 2048 x 640, real A,
+// 1.58 -> 1.45 ms (31.6 TFLOP/s); 4096 x 2048 x 4096, real A, 4.65 -> 4.24 (32.5); 4096
+// x 640 x 4096, real B, 1.67 -> 1.44 (29.9).  The matrix pipe is then busy 85 % of
+// the time; what is left is barriers and the copies' address arithmetic.
 #include "zgemm.cuh"
 
 #include <algorithm>
@@ -15,6 +19,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 
 #include "dmma.cuh"
 #include "once.cuh"
@@ -150,6 +155,47 @@ zgemm_kernel(ZGemmArgs a)
         }
         cp_async_commit();
     }
+    // FULL: every fragment of the warp meets C, so that no branch stands
+    // between the products
+    auto products = [&](auto full, const typename LA::T *As, const typename LB::T *Bs) {
+        constexpr bool FULL = decltype(full)::value;
+#pragma unroll
+        for (int k4 = 0; k4 < BK; k4 += 4) {
+            double ar[MI], ai[MI], an[MI];
+#pragma unroll
+            for (int i = 0; i < MI; ++i) {
+                if constexpr (RA) {
+                    ar[i] = As[LA::at(wm + 8 * i + fr, k4 + fk)];
+                } else {
+                    const zd v = As[LA::at(wm + 8 * i + fr, k4 + fk)];
+                    ar[i] = v.x;
+                    ai[i] = OPA == OP_C ? -v.y : v.y;
+                    an[i] = OPA == OP_C ? v.y : -v.y;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < NI; ++j) {
+                if (!FULL && j >= nb) continue;
+                double br, bi = 0.0;
+                if constexpr (RB) {
+                    br = Bs[LB::at(wn + 8 * j + fr, k4 + fk)];
+                } else {
+                    const zd v = Bs[LB::at(wn + 8 * j + fr, k4 + fk)];
+                    br = v.x;
+                    bi = OPB == OP_C ? -v.y : v.y;
+                }
+#pragma unroll
+                for (int i = 0; i < MI; ++i) {
+                    if (!FULL && i >= mb) continue;
+                    dmma(cr[i][j][0], cr[i][j][1], ar[i], br);
+                    if constexpr (!RB) dmma(ci[i][j][0], ci[i][j][1], ar[i], bi);
+                    if constexpr (!RA && !RB) dmma(cr[i][j][0], cr[i][j][1], an[i], bi);
+                    if constexpr (!RA) dmma(ci[i][j][0], ci[i][j][1], ai[i], br);
+                }
+            }
+        }
+    };
+    const bool full = mb >= MI && nb >= NI;
     int slot = 0, fill = ST - 1;
     for (int kt = 0; kt < KT; ++kt) {
         cp_async_wait<ST - 2>();
@@ -169,41 +215,8 @@ zgemm_kernel(ZGemmArgs a)
         }
         const typename LA::T *As = (const typename LA::T *)(smem + slot * SH::STAGE);
         const typename LB::T *Bs = (const typename LB::T *)(smem + slot * SH::STAGE + LA::BYTES);
-#pragma unroll
-        for (int k4 = 0; k4 < BK; k4 += 4) {
-            double ar[MI], ai[MI], an[MI];
-#pragma unroll
-            for (int i = 0; i < MI; ++i) {
-                if constexpr (RA) {
-                    ar[i] = As[LA::at(wm + 8 * i + fr, k4 + fk)];
-                } else {
-                    const zd v = As[LA::at(wm + 8 * i + fr, k4 + fk)];
-                    ar[i] = v.x;
-                    ai[i] = OPA == OP_C ? -v.y : v.y;
-                    an[i] = OPA == OP_C ? v.y : -v.y;
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < NI; ++j) {
-                if (j >= nb) continue;
-                double br, bi = 0.0;
-                if constexpr (RB) {
-                    br = Bs[LB::at(wn + 8 * j + fr, k4 + fk)];
-                } else {
-                    const zd v = Bs[LB::at(wn + 8 * j + fr, k4 + fk)];
-                    br = v.x;
-                    bi = OPB == OP_C ? -v.y : v.y;
-                }
-#pragma unroll
-                for (int i = 0; i < MI; ++i) {
-                    if (i >= mb) continue;
-                    dmma(cr[i][j][0], cr[i][j][1], ar[i], br);
-                    if constexpr (!RB) dmma(ci[i][j][0], ci[i][j][1], ar[i], bi);
-                    if constexpr (!RA && !RB) dmma(cr[i][j][0], cr[i][j][1], an[i], bi);
-                    if constexpr (!RA) dmma(ci[i][j][0], ci[i][j][1], ai[i], br);
-                }
-            }
-        }
+        if (full) products(std::true_type{}, As, Bs);
+        else products(std::false_type{}, As, Bs);
         slot = slot + 1 == ST ? 0 : slot + 1;
         fill = fill + 1 == ST ? 0 : fill + 1;
     }
