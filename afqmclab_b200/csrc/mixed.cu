@@ -164,92 +164,6 @@ __global__ void gather32_kernel(int W, long long ws32, const int *table, float *
     if (threadIdx.x == 0) logw[i] = logw[j];
 }
 
-// Gram-Schmidt (SD2is::stabilize, SD2is.cpp:48-76) on an fp32 walker: norms,
-// projections and updates in FP64, the columns kept in fp32 between updates
-// (the walker's own precision), which halves the shared memory per walker.
-// n <= 128 (the mixed form runs n = 64 or 128).
-__global__ void __launch_bounds__(256, 5)
-mgs32_kernel(int W, int n, int ncol, int nup, int ndn, float *w32, zd *logw, const int *alive,
-             int *status)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ double red[32];
-    const int w = blockIdx.x;
-    if (alive && !alive[w]) return;
-    float2 *A = (float2 *)smem_raw;   // the walker, fp32 (columns stored between FP64 updates)
-    float *g = w32 + (size_t)w * 2 * n * ncol;
-    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5, nw = nt >> 5;
-    const long long ws = (long long)n * ncol;
-    for (long long e = tid; e < ws; e += nt) A[e] = make_float2(g[e], g[ws + e]);
-    __syncthreads();
-    const int nmin = nup < ndn ? nup : ndn;
-    double logR = 0.0, logRmin = 0.0;
-    int bad = 0;
-    for (int j = 0; j < ncol; ++j) {
-        double s = 0.0;
-        for (int i = tid; i < n; i += nt) {
-            const float2 v = A[i + (size_t)n * j];
-            s += (double)v.x * v.x + (double)v.y * v.y;
-        }
-        s = block_sum(s, red);
-        double r = sqrt(s);
-        if (r == 0.0) bad = 1;
-        double inv = r > 0.0 ? 1.0 / r : 0.0;
-        for (int i = tid; i < n; i += nt) {
-            const float2 v = A[i + (size_t)n * j];
-            A[i + (size_t)n * j] = make_float2((float)(v.x * inv), (float)(v.y * inv));
-        }
-        if (tid == 0) {
-            double lr = log(r);
-            logR += lr;
-            if (j < nmin) logRmin += lr;
-        }
-        __syncthreads();
-        // This lane's rows i = lane + 32 r of column j (n <= 128: at most four),
-        // converted to FP64 once per column; each column c's rows are converted
-        // once and kept for both the projection and the update (the fp32 <->
-        // FP64 conversions, not the FMAs, bound this loop).
-        zd qv[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int i = lane + 32 * r;
-            const float2 q = i < n ? A[i + (size_t)n * j] : make_float2(0.f, 0.f);
-            qv[r] = make_double2(q.x, q.y);
-        }
-        for (int c = j + 1 + wid; c < ncol; c += nw) {
-            zd d = make_double2(0.0, 0.0);
-            zd vv[4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int i = lane + 32 * r;
-                const float2 v = i < n ? A[i + (size_t)n * c] : make_float2(0.f, 0.f);
-                vv[r] = make_double2(v.x, v.y);
-                if (i < n) zfma(d, make_double2(qv[r].x, -qv[r].y), vv[r]);
-            }
-            d.x = warp_sum(d.x);
-            d.y = warp_sum(d.y);
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int i = lane + 32 * r;
-                if (i < n) {
-                    const double vx = vv[r].x - (d.x * qv[r].x - d.y * qv[r].y);
-                    const double vy = vv[r].y - (d.x * qv[r].y + d.y * qv[r].x);
-                    A[i + (size_t)n * c] = make_float2((float)vx, (float)vy);
-                }
-            }
-        }
-        __syncthreads();
-    }
-    for (long long e = tid; e < ws; e += nt) { g[e] = A[e].x; g[ws + e] = A[e].y; }
-    if (tid == 0) {
-        zd lw = logw[w];
-        if (nup == ndn) lw.x += 2.0 * logR;
-        else lw.x += logR + logRmin;
-        logw[w] = lw;
-        if (bad && status) atomicOr(status + w, (int)ST_ZERO_NORM);
-    }
-}
-
 // Phaseless force from the tensor-core xbar partials, aux sampling, sample
 // log-weight and second cos projection (same arithmetic as the FP64 form),
 // writing y = sqrt(-dt) x as the bf16 operand of the two-body GEMM.  One warp
@@ -1467,18 +1381,9 @@ int mixed_project_dtk_dtv(afqmc_engine *e)
 int mixed_modify_gm(afqmc_engine *e)
 {
     if (e->kind == KIND_CP) return cp_mixed_modify_gm(e);
-    // columns in registers (FP64) where the shape fits one CTA of 512 lanes
-    if (launch_mgs_col(e->W, e->n, e->ncol, e->nup, e->ndn, 1, e->mx->wf32, true, e->logw, e->alive,
-                       e->status, e->stream))
-        return engine_check_launch();
-    const size_t bytes = (size_t)e->n * e->ncol * sizeof(float2);
-    static std::atomic<unsigned long long> attr{0};
-    if (first_on_device(attr)) {
-        cudaFuncSetAttribute(mgs32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-    }
-    if (bytes > 160 * 1024) return engine_fail(AFQMC_ERR_UNSUPPORTED, "walker too large for the fp32 stabiliser");
-    mgs32_kernel<<<e->W, 256, bytes, e->stream>>>(e->W, e->n, e->ncol, e->nup, e->ndn, e->mx->wf32,
-                                                  e->logw, e->alive, e->status);
+    if (!launch_mgs_block(e->W, e->n, e->ncol, e->nup, e->ndn, 1, e->mx->wf32, true, e->logw, e->alive, e->status,
+                          e->stream))
+        return engine_fail(AFQMC_ERR_UNSUPPORTED, "walker too large for the fp32 stabiliser");
     return engine_check_launch();
 }
 
