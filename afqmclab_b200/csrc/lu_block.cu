@@ -26,7 +26,7 @@
 // 1200.
 //
 // Against the element-wise kernels it replaces (us per launch, one B200): 14
-// columns, 100 matrices 35 -> 17; 16 columns, 512 matrices 31 -> 19; 56, 1024: 203
+// columns, 100 matrices 35 -> 17; 16 columns, 512 matrices 31 -> 17; 56, 1024: 203
 // -> 181; 64, 512: 131 -> 109; 80, 1024: 1459 -> 796; 120, 1024: 2867 -> 1413.
 #include <cooperative_groups.h>
 
@@ -42,9 +42,6 @@ namespace cg = cooperative_groups;
 extern std::atomic<long long> g_launch_count;
 
 namespace {
-
-constexpr int LB_NCB = 8;                 // block columns per CTA
-constexpr int LB_LDB = 8 * LB_NCB + 2;    // 2 mod 8: conflict-free fragment loads
 
 // A 32-bit rank for the pivot search, one warp reduction wide: the leading 25
 // bits of |re| + |im| (11 of exponent, 14 of mantissa; NaN ranks as infinity),
@@ -74,9 +71,12 @@ __device__ __noinline__ zd lb_rcp_any(zd b)
     return zeq0(b) ? make_double2(0.0, 0.0) : zdiv(make_double2(1.0, 0.0), b);
 }
 
-template <int C>
+// C: CTAs per block; NCB: block columns per CTA (8, or 4 for up to 32 columns, whose
+// fewer registers let six CTAs share an SM).
+template <int C, int NCB>
 struct LbShared {
-    static constexpr int ROWS = 64 * C, LDG = ROWS + 2;
+    static constexpr int ROWS = 8 * NCB * C, LDG = ROWS + 2;   // 2 mod 8: conflict-free fragment loads
+    static constexpr int LB_LDB = 8 * NCB + 2;
     zd G[2][8][LDG];        // [panel parity][column][row]
     zd B[8][LB_LDB];        // the pivot rows
     zd crow[2][2 * C][9];   // [step parity][warp]: the candidate's reciprocal, the rest of its panel row, its value
@@ -92,16 +92,16 @@ struct LbShared {
 __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
-// NBK: spin blocks per walker; C: CTAs per block (column halves).
-template <int NBK, int C>
-__global__ void __launch_bounds__(320 * C, C == 1 ? 2 : 1)
+// NBK: spin blocks per walker.
+template <int NBK, int C, int LB_NCB>
+__global__ void __launch_bounds__(LB_NCB == 4 ? 160 : 320 * C, LB_NCB == 4 ? 6 : C == 1 ? 2 : 1)
 lu_block_kernel(int nbw, Blocks bl, const zd *S, zd *Sinv, float *Sinv32, long long s32, const int *active, const zd *logw,
                 zd logwAdd, zd logwT, zd *logov, int *alive, int *surv, zd *logwOut, double *weight, int *status,
                 int mode, int wantInverse)
 {
     static_assert(NBK == 1 || C == 1, "two spin blocks are not split");
-    typedef LbShared<C> SH;
-    constexpr int LDG = SH::LDG;
+    typedef LbShared<C, LB_NCB> SH;
+    constexpr int LDG = SH::LDG, LB_LDB = SH::LB_LDB;
     extern __shared__ __align__(16) unsigned char smem[];
     SH &sh = *(SH *)smem;
     cg::cluster_group cl = cg::this_cluster();
@@ -401,22 +401,22 @@ lu_block_kernel(int nbw, Blocks bl, const zd *S, zd *Sinv, float *Sinv32, long l
     if constexpr (NBK * C > 1) cl.sync();   // rank 1's shared memory stays until rank 0 has read it
 }
 
-template <int NBK, int C>
+template <int NBK, int C, int NCB>
 cudaError_t launch(int W, int maxNs, const Blocks &bl, const zd *S, zd *Sinv, float *Sinv32, long long s32,
                    const int *active, const zd *logw, zd logwAdd, zd logwT, zd *logov, int *alive, int *surv,
                    zd *logwOut, double *weight, int *status, int mode, int inv, cudaStream_t s)
 {
     static std::atomic<unsigned long long> attr{0};
     cudaError_t r = each_device_once(attr, [] {
-        return cudaFuncSetAttribute(lu_block_kernel<NBK, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)sizeof(LbShared<C>));
+        return cudaFuncSetAttribute(lu_block_kernel<NBK, C, NCB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)sizeof(LbShared<C, NCB>));
     });
     if (r != cudaSuccess) return r;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(NBK * C) * (unsigned)W);
     const int nbw = (maxNs + 7) / 8;   // one warp per block row, then the panel warps
     cfg.blockDim = dim3(32u * (unsigned)(nbw + (maxNs + 31) / 32));
-    cfg.dynamicSmemBytes = sizeof(LbShared<C>);
+    cfg.dynamicSmemBytes = sizeof(LbShared<C, NCB>);
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -425,7 +425,7 @@ cudaError_t launch(int W, int maxNs, const Blocks &bl, const zd *S, zd *Sinv, fl
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = NBK * C > 1 ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, lu_block_kernel<NBK, C>, nbw, bl, S, Sinv, Sinv32, s32, active, logw, logwAdd,
+    return cudaLaunchKernelEx(&cfg, lu_block_kernel<NBK, C, NCB>, nbw, bl, S, Sinv, Sinv32, s32, active, logw, logwAdd,
                               logwT, logov, alive, surv, logwOut, weight, status, mode, inv);
 }
 
@@ -445,7 +445,8 @@ cudaError_t lu_block(int W, const Blocks &bl, const zd *S, zd *Sinv, float *Sinv
     const int maxNs = bl.nblk == 2 && bl.Ns[1] > bl.Ns[0] ? bl.Ns[1] : bl.Ns[0], inv = wantInverse ? 1 : 0;
     const long long s32 = sinv32_stride(bl);
 #define LB_ARGS W, maxNs, bl, S, Sinv, Sinv32, s32, active, logw, logwAdd, logwT, logov, alive, surv, logwOut, weight, status, mode, inv, s
-    if (bl.nblk == 2) return launch<2, 1>(LB_ARGS);
-    return maxNs <= 64 ? launch<1, 1>(LB_ARGS) : launch<1, 2>(LB_ARGS);
+    if (maxNs <= 32) return bl.nblk == 2 ? launch<2, 1, 4>(LB_ARGS) : launch<1, 1, 4>(LB_ARGS);
+    if (bl.nblk == 2) return launch<2, 1, 8>(LB_ARGS);
+    return maxNs <= 64 ? launch<1, 1, 8>(LB_ARGS) : launch<1, 2, 8>(LB_ARGS);
 #undef LB_ARGS
 }

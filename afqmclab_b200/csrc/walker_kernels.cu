@@ -1740,6 +1740,12 @@ static void launch_regw(int W, const Blocks &bl, zd *S, zd *X64, float *Sinv32, 
                        logwAdd, logwT, logov, alive, surv, logwOut, weight, status, mode, inv);
 }
 
+// 25 to 32 columns stay element-wise where more matrices come at once than the
+// blocked kernel has CTAs on the GPU (six per SM).  Measured, element-wise and
+// blocked, us: 32 columns, 2048 matrices 67 and 77; 1024: 45 and 50; 600: 37 and 33;
+// 24 columns, 2048: 58 and 49; 1024: 36 and 27; 600: 29 and 25.
+static bool lu_regw_faster(int maxNs, long long matrices) { return maxNs > 24 && maxNs <= 32 && matrices > 888; }
+
 void launch_lu_logdet_inverse32(int W, const Blocks &bl, zd *S, zd *Sinv, float *Sinv32, const int *active,
                                 const zd *logw, zd logwAdd, zd logwT, zd *logov, int *alive, int *surv,
                                 zd *logwOut, double *weight, int *status, int mode, bool wantInverse,
@@ -1748,11 +1754,7 @@ void launch_lu_logdet_inverse32(int W, const Blocks &bl, zd *S, zd *Sinv, float 
     int maxNs = 0;
     for (int b = 0; b < bl.nblk; ++b) maxNs = bl.Ns[b] > maxNs ? bl.Ns[b] : maxNs;
     const long long s32 = sinv32_stride(bl);
-    // 17 to 32 columns stay element-wise where many matrices share an SM: its two
-    // warps per matrix take 0.074 ms for 2048 blocks of 32 columns against 0.094,
-    // 0.045 for 1024 against 0.052; up to four matrices per SM the blocked kernel's
-    // shorter steps win (23 columns, 333 matrices: 20.9 us against 23.1)
-    if ((maxNs <= 16 || maxNs > 32 || (long long)W * bl.nblk <= 592) && lu_block_supported(bl)) {
+    if (lu_block_supported(bl) && !lu_regw_faster(maxNs, (long long)W * bl.nblk)) {
         lu_block(W, bl, S, Sinv32 ? nullptr : Sinv, Sinv32, active, logw, logwAdd, logwT, logov, alive, surv, logwOut,
                  weight, status, mode, wantInverse, s);
         return;

@@ -45,6 +45,6 @@ def test_walkers_equal_to_the_trial(N):
 
 
 def test_many_walkers_of_17_to_32_columns():
-    """Both sides of the rule that leaves 17 to 32 columns to the element-wise kernel."""
-    for W in (592, 593):
-        check(22, 18, 0, W, 0.05)
+    """Both sides of the rule that leaves 25 to 32 columns to the element-wise kernel."""
+    for N, W in ((24, 900), (25, 888), (25, 889)):
+        check(30, N, 0, W, 0.05)
