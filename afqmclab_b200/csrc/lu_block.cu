@@ -43,34 +43,6 @@ extern std::atomic<long long> g_launch_count;
 
 namespace {
 
-// A 32-bit rank for the pivot search, one warp reduction wide: the leading 25
-// bits of |re| + |im| (11 of exponent, 14 of mantissa; NaN ranks as infinity),
-// then the lower position.  The chosen pivot is within 2^-14 of zgetf2's, which
-// changes neither the bound on the growth nor any result beyond rounding.
-// Ineligible rows rank 0.
-__device__ __forceinline__ unsigned lb_rank(zd a, int pos, bool eligible)
-{
-    const unsigned hi = min((unsigned)__double2hiint(zcabs1(a)) & 0x7fffffffu, 0x7ff00000u);   // a NaN as infinity
-    return eligible ? (((hi >> 6) + 1u) << 7) | (unsigned)(127 - pos) : 0u;
-}
-
-// 1 / b: conj(b) / |b|^2 with the reciprocal of d = |b|^2 from the hardware's
-// approximation (20 bits) and two Newton-Raphson steps.  Good while d is
-// within 1e-280 .. 1e280; lb_rcp_any covers the rest (zero gives zero).
-__device__ __forceinline__ zd lb_rcp(zd b, double &d)
-{
-    d = fma(b.x, b.x, b.y * b.y);
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    y = fma(y, fma(-d, y, 1.0), y);
-    y = fma(y, fma(-d, y, 1.0), y);
-    return make_double2(b.x * y, -b.y * y);
-}
-__device__ __noinline__ zd lb_rcp_any(zd b)
-{
-    return zeq0(b) ? make_double2(0.0, 0.0) : zdiv(make_double2(1.0, 0.0), b);
-}
-
 // C: CTAs per block; NCB: block columns per CTA (8, or 4 for up to 32 columns, whose
 // fewer registers let six CTAs share an SM).
 template <int C, int NCB>

@@ -4,44 +4,32 @@
 
 #include "walker_kernels.cuh"
 
-// A rank that orders candidates like the pivot search: for values >= +0 the
-// IEEE bits are monotonic; NaN ranks as infinity; ineligible rows rank 0.
-__device__ __forceinline__ unsigned long long gr_rank(zd a0, bool eligible)
+// A 32-bit rank for the pivot search, one warp reduction wide: the leading 25
+// bits of |re| + |im| (11 of exponent, 14 of mantissa; NaN ranks as infinity),
+// then the lower position.  The chosen pivot is within 2^-14 of zgetf2's, which
+// changes neither the bound on the growth nor any result beyond rounding.
+// Ineligible rows rank 0.
+__device__ __forceinline__ unsigned lb_rank(zd a, int pos, bool eligible)
 {
-    double v = zcabs1(a0);
-    if (!(v == v)) v = CUDART_INF;
-    return eligible ? (unsigned long long)__double_as_longlong(v) + 1ull : 0ull;
+    const unsigned hi = min((unsigned)__double2hiint(zcabs1(a)) & 0x7fffffffu, 0x7ff00000u);   // a NaN as infinity
+    return eligible ? (((hi >> 6) + 1u) << 7) | (unsigned)(127 - pos) : 0u;
 }
 
-// 1 / b without a division, so that it schedules between other arithmetic:
-// b is scaled by a power of two (exact) so that max(|re|, |im|) lies in
-// [1, 2), the real reciprocal y of d = |b|^2 in [1, 8) starts from the
-// single-precision approximation and takes two Newton-Raphson steps
-// y <- y + y (1 - d y), each of which doubles the correct bits (about 21 ->
-// 42 -> full precision), and 1/b = s conj(b s) y.  Within a few ulp of the
-// rounded quotient; a NaN or infinite b gives NaN (callers test zero first).
-__device__ __forceinline__ zd zrcp_nr(zd b)
+// 1 / b: conj(b) / |b|^2 with the reciprocal of d = |b|^2 from the hardware's
+// approximation (20 bits) and two Newton-Raphson steps.  Good while d is
+// within 1e-280 .. 1e280; lb_rcp_any covers the rest (zero gives zero).
+__device__ __forceinline__ zd lb_rcp(zd b, double &d)
 {
-    const double m = fmax(fabs(b.x), fabs(b.y));
-    const long long e = (__double_as_longlong(m) >> 52) & 0x7ff;
-    const double s = __longlong_as_double((2046 - e) << 52);   // 2^(1023 - e)
-    const double xs = b.x * s, ys = b.y * s;
-    const double d = fma(xs, xs, ys * ys);
-    double y = (double)__fdividef(1.0f, (float)d);
+    d = fma(b.x, b.x, b.y * b.y);
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
     y = fma(y, fma(-d, y, 1.0), y);
     y = fma(y, fma(-d, y, 1.0), y);
-    const double t = y * s;
-    return make_double2(xs * t, -ys * t);
+    return make_double2(b.x * y, -b.y * y);
 }
-
-// Position of the warp's best candidate: largest rank, then lowest position.
-__device__ __forceinline__ int gr_warp_best(unsigned long long u, int pos)
+static __device__ __noinline__ zd lb_rcp_any(zd b)
 {
-    const unsigned hi = (unsigned)(u >> 32), lo = (unsigned)u;
-    const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
-    const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
-    const unsigned key = (hi == mhi && lo == mlo) ? (unsigned)pos : 0xffffffffu;
-    return (int)__reduce_min_sync(0xffffffffu, key);
+    return zeq0(b) ? make_double2(0.0, 0.0) : zdiv(make_double2(1.0, 0.0), b);
 }
 
 // Per-walker finish of the block log-determinants: the overlap's log and,

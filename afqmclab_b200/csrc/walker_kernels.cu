@@ -494,8 +494,7 @@ __device__ __forceinline__ zd zrcp(zd b)
 // memory.
 // ---------------------------------------------------------------------------
 struct GR64Cand {
-    unsigned long long u;   // rank of the candidate: bits of |re|+|im| plus one, 0 if not eligible
-    int key;                // its position
+    int key;                // the candidate's position
     int row;                // its row
     zd a0;                  // its value in the current column
     zd q;                   // 1 / a0, zero when a0 is zero
@@ -545,12 +544,10 @@ gj_regw_kernel(int W, Blocks bl, const zd *S, zd *Sinv, float *Sinv32, long long
         if (ch == 0) xS[1][r] = a[SL - 1];
         if (ch == 0) {
             colS[0][r] = a[0];
-            const unsigned long long u = gr_rank(a[0], true);
-            if (pos == gr_warp_best(u, pos)) {
-                GR64Cand c;
-                c.u = u; c.key = pos; c.row = r; c.a0 = a[0];
-                c.q = zeq0(a[0]) ? make_double2(0.0, 0.0) : zrcp_nr(a[0]);
-                cand[0] = c;
+            const unsigned u = lb_rank(a[0], pos, r < Ns);
+            const unsigned best = __reduce_max_sync(0xffffffffu, u);
+            if (u != 0 && u == best) {
+                cand[0] = {pos, r, a[0], lb_rcp_any(a[0])};
 #pragma unroll
                 for (int s = 0; s < SL - 1; ++s) prowC[0][s] = a[s];
             }
@@ -584,10 +581,11 @@ gj_regw_kernel(int W, Blocks bl, const zd *S, zd *Sinv, float *Sinv32, long long
                 // the last step, where nothing reads it, so the step stays
                 // one straight-line block the compiler can interleave)
                 colS[pb][r] = a[0];
-                const unsigned long long u = gr_rank(a[0], pos > k);
-                const bool win = (pos == gr_warp_best(u, pos));
-                const zd qr = zrcp_nr(a[0]);
-                const zd qn = zeq0(a[0]) ? make_double2(0.0, 0.0) : qr;
+                const unsigned u = lb_rank(a[0], pos, r < Ns && pos > k);
+                const unsigned best = __reduce_max_sync(0xffffffffu, u);
+                const bool win = u != 0 && u == best;
+                double d;
+                const zd qr = lb_rcp(a[0], d);
 #pragma unroll
                 for (int s = 2; s < SL; ++s) {
                     const zd pv = s < SL - 1 ? pr[s] : pLast;
@@ -595,10 +593,9 @@ gj_regw_kernel(int W, Blocks bl, const zd *S, zd *Sinv, float *Sinv32, long long
                     a[s - 1].y = fma(-f.x, pv.y, fma(-f.y, pv.x, a[s].y));
                 }
                 if (win) {
-                    GR64Cand c;
-                    c.u = u; c.key = pos; c.row = r; c.a0 = a[0];
-                    c.q = qn;
-                    cand[pb] = c;
+                    GR64Cand &c = cand[pb];
+                    c.key = pos; c.row = r; c.a0 = a[0];
+                    c.q = (d > 1e-280 && d < 1e280) ? qr : lb_rcp_any(a[0]);
 #pragma unroll
                     for (int s = 0; s < SL - 1; ++s) prowC[pb][s] = a[s];
                 }
