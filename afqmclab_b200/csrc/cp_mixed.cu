@@ -502,14 +502,16 @@ __device__ __forceinline__ zd zexp_d(zd z)
 // NiupNidnSampleSDOperation::applyToRight, NiupNidnSDOperation.cpp:15-41;
 // HubbardSOCMeasureFixedSDSD force, HubbardSOCMeasureFixedSDSD.cpp:95-130).
 __global__ void __launch_bounds__(256)
-cpm_sample_apply_kernel(int W, HubbardDev h, const float2 *gd, const int *surv, const unsigned long long *offs,
-                        uint64_t seed, const float *hi, const float *lo, float *thi, float *tlo, zd *logw,
+cpm_sample_apply_kernel(int W, HubbardDev h, const float2 *gd, const int *surv, RngPlace rng, uint64_t seed,
+                        const float *hi, const float *lo, float *thi, float *tlo, zd *logw,
                         double dtET, zd hopLogw, int *auxOut)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int scratch[33];
     const int w = blockIdx.x;
-    if (!surv[w]) return;
     const int L = h.L, N = h.N, n = h.n;
+    const unsigned long long place = rng_place(rng, W, w, surv, L, scratch);
+    if (!surv[w]) return;
     // layout: 16-byte entries first, so every array is aligned for any L
     zd *gxS = (zd *)smem_raw;                        // per site: gamma x
     float2 *d = (float2 *)(gxS + L);                 // 4 L entries: d00, d01, d10, d11
@@ -529,7 +531,7 @@ cpm_sample_apply_kernel(int W, HubbardDev h, const float2 *gd, const int *surv, 
             f = fmin(fmax(f, -h.forceCap), h.forceCap);
         }
         const double em = exp(-f), ep = exp(f);
-        const int x = (rng_uniform(seed, offs[w] + (unsigned long long)i) < em / (em + ep)) ? -1 : 1;
+        const int x = (rng_uniform(seed, place + (unsigned long long)i) < em / (em + ep)) ? -1 : 1;
         aux[i] = x;
         if (auxOut) auxOut[(size_t)w * L + i] = x;
         lpS[i] = x * f - log(ep + em);
@@ -883,11 +885,11 @@ int cp_mixed_project_dtk_dtv(afqmc_engine *e)
     }
     {
         PHASE(AFQMC_PH_SAMPLE);
-        launch_rng_scan(W, e->surv, e->L, e->counter, e->offs, s);
+        const RngPlace rng = engine_rng_place(e, e->L);
         const int L = e->L;
         const size_t smem = sizeof(float2) * 4 * L + sizeof(int) * (L + (L & 1)) + sizeof(double) * L + sizeof(zd) * L;
         g_launch_count++;
-        cpm_sample_apply_kernel<<<W, 256, smem, s>>>(W, e->hd, m->gd, e->surv, e->offs, e->seed, m->hi, m->lo,
+        cpm_sample_apply_kernel<<<W, 256, smem, s>>>(W, e->hd, m->gd, e->surv, rng, e->seed, m->hi, m->lo,
                                                      m->thi, m->tlo, e->logw, e->dt * e->ET,
                                                      engine_one_body_logw(e, 0), nullptr);
         CM(engine_check_launch());

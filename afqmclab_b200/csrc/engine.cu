@@ -200,6 +200,7 @@ int alloc_population(afqmc_engine *e)
     TRY(dalloc(e, &e->number, W));
     TRY(dalloc(e, &e->counter, 1));
     TRY(dalloc(e, &e->offs, W));
+    TRY(dalloc(e, &e->ticket, 2));
     TRY(dalloc(e, &e->weight, W));
     TRY(dalloc(e, &e->tstats, 4));
     long long init[4] = {0, 0, 1LL << 40, 0};
@@ -373,7 +374,7 @@ int taylor_apply(afqmc_engine *e, const zd *M, long long Mstride, const zd *src,
 }
 
 // one-body operator `which` applied to src -> dst for masked walkers
-int one_body(afqmc_engine *e, int which, const zd *src, zd *dst, const int *mask)
+int one_body(afqmc_engine *e, int which, const zd *src, zd *dst, const int *mask, const zd *diag = nullptr)
 {
     if (e->useLog && e->kind == KIND_PL) {
         const zd *Mx = which == 0 ? e->logK : e->expK[which];
@@ -390,7 +391,9 @@ int one_body(afqmc_engine *e, int which, const zd *src, zd *dst, const int *mask
         g.m = L; g.k = L;
         g.parts = 2; g.m1 = L; g.n1 = e->ncol; g.k1 = L;
         g.offA1 = L + (long long)e->n * L; g.offB1 = L; g.offC1 = L;
+        g.offScale1 = L;
     }
+    if (diag) { g.scaleB = diag; g.strideScale = e->n; }
     g.batch = e->W; g.mask = mask;
     return gemm(g, e->stream);
 }
@@ -572,25 +575,24 @@ int project_dtk_dtv(afqmc_engine *e)
     }
     zd hop = one_body_logw(e, 0);
     if (e->kind == KIND_CP) {
-        if (needTheta) {
-            PHASE(AFQMC_PH_FORCE);
-            launch_cp_force(W, e->hd, e->thetaT, e->bl.tStride, e->surv, e->forceCP, s);
-        }
         {
             PHASE(AFQMC_PH_SAMPLE);
-            launch_rng_scan(W, e->surv, e->L, e->counter, e->offs, s);
+            const RngPlace rng = engine_rng_place(e, e->L);
             BPState *bp = (e->bp && e->bp->active) ? e->bp : nullptr;
             // back-propagation: this step's fields and which walkers drew them
             // (twoBodyAuxBackup[i][BPIndex], afqmcConstraintPathProjection.cpp:73)
             int *auxOut = bp ? bp->aux + (size_t)bp->index * W * e->L : nullptr;
-            launch_cp_sample_apply(W, e->hd, e->forceCP, e->surv, e->offs, e->seed, e->wf, e->wfTmp,
+            launch_cp_sample_apply(W, e->hd, e->thetaT, e->bl.tStride, e->surv, rng, e->seed, e->wf, e->wfTmp, e->diagCP,
                                    e->logw, e->dt * e->ET, hop, auxOut, s);
             TRY(check_launch());
             if (bp)
                 CUDA_TRY(cudaMemcpyAsync(bp->valid + (size_t)bp->index * W, e->surv, sizeof(int) * W,
                                          cudaMemcpyDeviceToDevice, s));
         }
-        { PHASE(AFQMC_PH_ONEBODY); TRY(one_body(e, 0, e->wfTmp, e->wf, e->surv)); }
+        // a diagonal sample is a scaling of the product's rows, in place
+        PHASE(AFQMC_PH_ONEBODY);
+        if (e->diagCP) TRY(one_body(e, 0, e->wf, e->wf, e->surv, e->diagCP));
+        else TRY(one_body(e, 0, e->wfTmp, e->wf, e->surv));
     } else {
         if (needTheta) { PHASE(AFQMC_PH_FORCE); TRY(xbar_gemm(e, bl)); }
         {
@@ -951,6 +953,18 @@ template int engine_dalloc<int>(afqmc_engine *, int **, size_t);
 template int engine_dalloc<zd>(afqmc_engine *, zd **, size_t);
 template int engine_dalloc<double>(afqmc_engine *, double **, size_t);
 template int engine_dalloc<unsigned short>(afqmc_engine *, unsigned short **, size_t);
+RngPlace engine_rng_place(afqmc_engine *e, int draws)
+{
+    RngPlace p;
+    if (e->W <= RNG_INLINE_MAX) {
+        p.counter = e->counter;
+        p.ticket = e->ticket;
+    } else {
+        launch_rng_scan(e->W, e->surv, draws, e->counter, e->offs, e->stream);
+        p.offs = e->offs;
+    }
+    return p;
+}
 zd engine_one_body_logw(afqmc_engine *e, int which) { return one_body_logw(e, which); }
 
 // =========================================================== C ABI
@@ -1015,7 +1029,6 @@ int afqmc_cp_create(int L, int N, int W, int decomp, int force_type, double dt, 
     CK(dupload(e, &e->cdiag[0], c00.data(), L)); CK(dupload(e, &e->cdiag[1], c01.data(), L));
     CK(dupload(e, &e->cdiag[2], c10.data(), L)); CK(dupload(e, &e->cdiag[3], c11.data(), L));
     if (const_force) CK(dupload(e, &e->constForceCP, const_force, L));
-    CK(dalloc(e, &e->forceCP, (size_t)W * L));
     CK(dalloc(e, &e->sites, (size_t)W * 4 * L));
     CK(dalloc(e, &e->siteNum, (size_t)4 * L));
     e->hd.L = L; e->hd.N = N; e->hd.n = n; e->hd.decomp = decomp;
@@ -1046,6 +1059,11 @@ int afqmc_cp_create(int L, int N, int W, int decomp, int force_type, double dt, 
     CK(real_operators(e, ops, trials));
     find_spin_blocks(e, phiT, ops);
     e->hd.n0 = e->n0;
+    // density decompositions without transverse fields: the sample is diagonal
+    bool diagonal = precision == AFQMC_FP64 && (decomp == AFQMC_DENSITY_CHARGE || decomp == AFQMC_DENSITY_SPIN) &&
+                    zgemm_scaled_supported(e->spinDiag[0] ? L : n);
+    for (int i = 0; diagonal && i < L; ++i) diagonal = hx[i] == 0.0 && hy[i] == 0.0;
+    if (diagonal) CK(dalloc(e, &e->diagCP, (size_t)W * n));
     cudaError_t ce = cudaStreamSynchronize(e->stream);
     if (ce != cudaSuccess) { free_engine(e); return fail(AFQMC_ERR_CUDA, cudaGetErrorString(ce)); }
 #undef CK

@@ -43,6 +43,7 @@ struct afqmc_engine {
     int *alive = nullptr, *surv = nullptr, *status = nullptr, *done = nullptr, *order = nullptr,
         *table = nullptr, *number = nullptr;
     unsigned long long *counter = nullptr, *offs = nullptr;
+    unsigned int *ticket = nullptr;   // two ints of rng_place
     double *weight = nullptr;
     long long *tstats = nullptr;
     // one-body operators: 0 exp(-dt K), 1 exp(+dt/2 K), 2 exp(-dt/2 K)
@@ -60,6 +61,9 @@ struct afqmc_engine {
     int *realFlag = nullptr;
     int n0 = 0;
     bool spinDiag[3] = {false, false, false};
+    // constrained path: the two-body sample's diagonal (W x 2L), applied by the
+    // one-body product (null: the sample is applied by its own kernel)
+    zd *diagCP = nullptr;
     // propagator rebuild on the GPU: K (n x n), scratch Kp and three Taylor
     // matrices (n x n each), the 1-norm of Kp and sum bg^2
     double *kin = nullptr, *propNorms = nullptr;
@@ -69,7 +73,7 @@ struct afqmc_engine {
     HubbardDev hd{};
     zd *gamma = nullptr, *cdiag[4] = {nullptr, nullptr, nullptr, nullptr};
     double *U = nullptr, *mu = nullptr, *hx = nullptr, *hy = nullptr, *hz = nullptr,
-           *constForceCP = nullptr, *forceCP = nullptr;
+           *constForceCP = nullptr;
     zd *wfDaggerK = nullptr;
     // phaseless
     CholDev cdv{};
@@ -158,6 +162,9 @@ int engine_fail(int code, const std::string &msg);
 int engine_check_launch();
 int engine_gemm(const ZGemmArgs &a, cudaStream_t s);
 template <class T> int engine_dalloc(afqmc_engine *e, T **p, size_t count);
+// The walkers' places in the random stream for a sampling kernel of one CTA per
+// walker (launches the scan where the kernel does not count by itself).
+RngPlace engine_rng_place(afqmc_engine *e, int draws);
 zd engine_one_body_logw(afqmc_engine *e, int which);
 // Local energy of the phaseless engine at the current walkers (logov, Sinv,
 // thetaT, xbar, eloc, den); the exchange form is one of PL_EX_*.

@@ -739,42 +739,6 @@ __global__ void rng_scan_kernel(int W, const int *surv, int draws, unsigned long
     if (tid == 0) *counter = carry;
 }
 
-// ---------------------------------------------------------------------------
-// Hubbard force: HubbardSOCMeasureFixedSDSD::getForce (:73-116) with the
-// Green's function diagonal / off-diagonal of SDSDOperation (:91-141).
-// ---------------------------------------------------------------------------
-__global__ void cp_force_kernel(int W, HubbardDev h, const zd *thetaT, long long tStride,
-                                const int *surv, double *force)
-{
-    const int w = blockIdx.x;
-    if (!surv[w]) return;
-    const int L = h.L, N = h.N, n = h.n;
-    const zd *th = thetaT + (size_t)w * tStride;
-    for (int i = threadIdx.x; i < L; i += blockDim.x) {
-        double f;
-        if (h.constForce) {
-            f = h.constForce[i];
-        } else {
-            zd a = make_double2(0.0, 0.0), b = make_double2(0.0, 0.0);
-            // a trial that keeps the spins apart has its zeros skipped (and only
-            // the other blocks of thetaT are current then)
-            const int ja = h.n0 > 0 ? h.n0 : N, jb = h.n0;
-            const zd *ta = th + (size_t)N * (h.decomp <= 1 ? i : i + L), *tb = th + (size_t)N * (h.decomp <= 1 ? i + L : i);
-            for (int j = 0; j < ja; ++j) zfma(a, zconj(h.phiT[i + (size_t)n * j]), ta[j]);
-            for (int j = jb; j < N; ++j) zfma(b, zconj(h.phiT[i + L + (size_t)n * j]), tb[j]);
-            zd bgv;
-            if (h.decomp == 0) bgv = make_double2(a.x + b.x - 1.0, a.y + b.y);
-            else if (h.decomp == 1) bgv = zsub(a, b);
-            else if (h.decomp == 2) bgv = zadd(a, b);
-            else bgv = zsub(a, b);
-            f = zmul(h.gamma[i], bgv).x;
-            if (f > h.forceCap) f = h.forceCap;
-            if (f < -h.forceCap) f = -h.forceCap;
-        }
-        force[(size_t)w * L + i] = f;
-    }
-}
-
 __device__ __forceinline__ zd zcosh(zd z)
 {
     zd e = zexp(z), ei = zexp(zneg(z));
@@ -845,35 +809,91 @@ __device__ __forceinline__ zd cp_sample_logw(const HubbardDev &h, const int *aux
 }
 
 // ---------------------------------------------------------------------------
-// Hubbard aux-field sampling + two-body sample + its application:
+// Hubbard force (HubbardSOCMeasureFixedSDSD::getForce, :73-116, with the
+// Green's function diagonal / off-diagonal of SDSDOperation, :91-141),
+// aux-field sampling + two-body sample + its application:
 // NiupNidn::sampleAuxFromForce (NiupNidn.cpp:66-84),
 // getTwoBodySampleFromAuxForce (:100-142, setTwoBodySampleMatrix :252-322),
 // NiupNidnSampleSDOperation::applyToRight (NiupNidnSDOperation.cpp:15-41),
 // and the walker log-weight bookkeeping of the driver step
 // (afqmcConstraintPathProjection.cpp:63-72).
+//
+// One CTA per walker, 8 lanes per site for the force, so that the loads of
+// thetaT come in runs of 128 bytes (one thread per site read one entry per
+// line: 35 us for the 8x8 lattice and 1024 walkers in a kernel of its own, and
+// the random stream's scan another 3).  APPLY: the two-body sample is applied,
+// wfTmp = D wf.  Without it the diagonal of D (n per walker) goes to diag, and the
+// one-body product scales its operand's rows by it.  8x8 lattice, 1024 walkers:
+// force, scan and applied sample 86 -> 74 us, the sample alone 33 (and 15 more in
+// the one-body product); 4x4, 100 walkers: 13 -> 7.
 // ---------------------------------------------------------------------------
+template <bool APPLY>
 __global__ void __launch_bounds__(256)
-cp_sample_apply_kernel(int W, HubbardDev h, const double *force, const int *surv,
-                       const unsigned long long *offs, uint64_t seed, const zd *wf, zd *wfTmp,
-                       zd *logw, double dtET, zd hopLogw, int *auxOut)
+cp_sample_apply_kernel(int W, HubbardDev h, const zd *thetaT, long long tStride, const int *surv, RngPlace rng,
+                       uint64_t seed, const zd *wf, zd *wfTmp, zd *diag, zd *logw, double dtET, zd hopLogw,
+                       int *auxOut)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int scratch[33];
     const int w = blockIdx.x;
-    if (!surv[w]) return;
     const int L = h.L, N = h.N, n = h.n;
+    const unsigned long long place = rng_place(rng, W, w, surv, L, scratch);
+    if (!surv[w]) return;
     zd *d00 = (zd *)smem_raw, *d01 = d00 + L, *d10 = d00 + 2 * L, *d11 = d00 + 3 * L;
     int *aux = (int *)(d00 + 4 * L);
     double *fs = (double *)(aux + L + (L & 1));
-    const double *fw = h.constForce ? h.constForce : force + (size_t)w * L;
+    const zd *th = thetaT + (size_t)w * tStride;
+    constexpr int P = 8;
+    const int part = threadIdx.x % P;
+    for (int i0 = 0; i0 < L; i0 += blockDim.x / P) {
+        const int i = i0 + threadIdx.x / P;
+        const bool site = i < L;   // uniform over each lane group of P
+        double f = 0.0;
+        if (h.constForce) {
+            if (site) f = h.constForce[i];
+        } else {
+            // a trial that keeps the spins apart has its zeros skipped (and only
+            // the other blocks of thetaT are current then)
+            zd a = make_double2(0.0, 0.0), b = make_double2(0.0, 0.0);
+            if (site) {
+                const int ja = h.n0 > 0 ? h.n0 : N;
+                const zd *ta = th + (size_t)N * (h.decomp <= 1 ? i : i + L);
+                const zd *tb = th + (size_t)N * (h.decomp <= 1 ? i + L : i);
+                for (int j = part; j < ja; j += P) zfma(a, zconj(h.phiT[i + (size_t)n * j]), ta[j]);
+                for (int j = h.n0 + part; j < N; j += P) zfma(b, zconj(h.phiT[i + L + (size_t)n * j]), tb[j]);
+            }
+            zd g;   // each lane's share of the background, added up over the site's lanes
+            if (h.decomp == 0 || h.decomp == 2) g = zadd(a, b);
+            else g = zsub(a, b);
+#pragma unroll
+            for (int o = 1; o < P; o <<= 1) {
+                g.x += __shfl_xor_sync(0xffffffffu, g.x, o);
+                g.y += __shfl_xor_sync(0xffffffffu, g.y, o);
+            }
+            if (h.decomp == 0) g.x -= 1.0;
+            if (site) {
+                f = zmul(h.gamma[i], g).x;
+                if (f > h.forceCap) f = h.forceCap;
+                if (f < -h.forceCap) f = -h.forceCap;
+            }
+        }
+        if (site && part == 0) fs[i] = f;
+    }
+    __syncthreads();
+    // one lane per site again for the field, its factors and its weight
     for (int i = threadIdx.x; i < L; i += blockDim.x) {
-        double f = fw[i];
+        const double f = fs[i];
         double em = exp(-f), ep = exp(f);
         double prob = em / (em + ep);
-        int x = (rng_uniform(seed, offs[w] + (unsigned long long)i) < prob) ? -1 : 1;
+        int x = (rng_uniform(seed, place + (unsigned long long)i) < prob) ? -1 : 1;
         aux[i] = x;
         if (auxOut) auxOut[(size_t)w * L + i] = x;
         fs[i] = x * f - log(ep + em);   // the site's term of the force's log-probability
         cp_site_matrix(h, i, x, d00[i], d01[i], d10[i], d11[i]);
+        if (!APPLY) {
+            diag[(size_t)w * n + i] = d00[i];
+            diag[(size_t)w * n + i + L] = d11[i];
+        }
     }
     __syncthreads();
     if (threadIdx.x < 32) {
@@ -893,6 +913,7 @@ cp_sample_apply_kernel(int W, HubbardDev h, const double *force, const int *surv
             logw[w] = zadd(hopLogw, t);
         }
     }
+    if (!APPLY) return;
     const zd *src = wf + (size_t)w * n * N;
     zd *dst = wfTmp + (size_t)w * n * N;
     for (int e = threadIdx.x; e < L * N; e += blockDim.x) {
@@ -1812,22 +1833,18 @@ void launch_rng_scan(int W, const int *surv, int draws, unsigned long long *coun
     rng_scan_kernel<<<1, 1024, 0, s>>>(W, surv, draws, counter, offs);
 }
 
-void launch_cp_force(int W, const HubbardDev &h, const zd *thetaT, long long tStride,
-                     const int *surv, double *force, cudaStream_t s)
-{
-    g_launch_count++;
-    cp_force_kernel<<<W, 128, 0, s>>>(W, h, thetaT, tStride, surv, force);
-}
-
-void launch_cp_sample_apply(int W, const HubbardDev &h, const double *force, const int *surv,
-                            const unsigned long long *offs, uint64_t seed, const zd *wf,
-                            zd *wfTmp, zd *logw, double dtET, zd hopLogw, int *auxOut,
-                            cudaStream_t s)
+void launch_cp_sample_apply(int W, const HubbardDev &h, const zd *thetaT, long long tStride, const int *surv,
+                            const RngPlace &rng, uint64_t seed, const zd *wf, zd *wfTmp, zd *diag, zd *logw,
+                            double dtET, zd hopLogw, int *auxOut, cudaStream_t s)
 {
     g_launch_count++;
     size_t smem = (size_t)4 * h.L * sizeof(zd) + (size_t)(h.L + 1) * sizeof(int) + (size_t)h.L * sizeof(double) + 16;
-    cp_sample_apply_kernel<<<W, 256, smem, s>>>(W, h, force, surv, offs, seed, wf, wfTmp, logw,
-                                                 dtET, hopLogw, auxOut);
+    if (diag)
+        cp_sample_apply_kernel<false><<<W, 256, smem, s>>>(W, h, thetaT, tStride, surv, rng, seed, wf, wfTmp, diag, logw,
+                                                           dtET, hopLogw, auxOut);
+    else
+        cp_sample_apply_kernel<true><<<W, 256, smem, s>>>(W, h, thetaT, tStride, surv, rng, seed, wf, wfTmp, diag, logw,
+                                                          dtET, hopLogw, auxOut);
 }
 
 void launch_pl_sample(int W, const CholDev &c, const zd *xbar, const int *surv_in, int *surv,

@@ -37,6 +37,48 @@ void launch_lu_logdet_inverse32(int W, const Blocks &bl, zd *S, zd *Sinv, float 
 
 void launch_rng_scan(int W, const int *surv, int draws, unsigned long long *counter,
                      unsigned long long *offs, cudaStream_t s);
+// The same inside a sampling kernel of one CTA per walker: walker w's place in
+// the random stream is *counter + draws x (survivors before w), counted by its
+// own CTA, and the last CTA to have read *counter advances it.  ticket: two
+// ints, zero between launches.  Saves a launch of 2-3 us on the step's critical
+// path; the counting is W^2 / 2 reads in all, so the scan takes over above
+// RNG_INLINE_MAX walkers (given by offs; ticket is null then).
+constexpr int RNG_INLINE_MAX = 4096;
+struct RngPlace {
+    unsigned long long *counter = nullptr;
+    unsigned int *ticket = nullptr;
+    const unsigned long long *offs = nullptr;
+};
+#ifdef __CUDACC__
+// For every thread of the block; scratch: 33 ints of shared memory.  Reads all
+// of surv, which the kernel must not write.
+__device__ __forceinline__ unsigned long long rng_place(const RngPlace &p, int W, int w, const int *surv, int draws,
+                                                        int *scratch)
+{
+    if (p.ticket == nullptr) return p.offs[w];
+    __shared__ unsigned long long base;
+    const int tid = threadIdx.x, lane = tid & 31;
+    int c = 0;
+    for (int i = tid; i < w; i += blockDim.x) c += surv[i] != 0 ? 1 : 0;
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0) scratch[tid >> 5] = c;
+    if (tid == 0) base = *(volatile unsigned long long *)p.counter;
+    __syncthreads();
+    int before = 0;
+    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) before += scratch[i];
+    if (tid == 0) {
+        volatile unsigned int *v = p.ticket;
+        if (w == W - 1) v[1] = (unsigned)before + (surv[w] != 0 ? 1u : 0u);
+        __threadfence();
+        if (atomicAdd(p.ticket, 1u) == (unsigned)W - 1u) {
+            __threadfence();
+            *p.counter = base + (unsigned long long)v[1] * (unsigned long long)draws;
+            v[0] = 0;
+        }
+    }
+    return base + (unsigned long long)before * (unsigned long long)draws;
+}
+#endif
 
 // Hubbard (NiupNidn) pieces
 struct HubbardDev {
@@ -47,12 +89,11 @@ struct HubbardDev {
     const zd *phiT;
     int n0;   // > 0: columns [0, n0) of phiT live on the spin-up rows, the others on the spin-down rows
 };
-void launch_cp_force(int W, const HubbardDev &h, const zd *thetaT, long long tStride,
-                     const int *surv, double *force, cudaStream_t s);
-void launch_cp_sample_apply(int W, const HubbardDev &h, const double *force, const int *surv,
-                            const unsigned long long *offs, uint64_t seed, const zd *wf,
-                            zd *wfTmp, zd *logw, double dtET, zd hopLogw, int *auxOut,
-                            cudaStream_t s);
+void launch_cp_sample_apply(int W, const HubbardDev &h, const zd *thetaT, long long tStride, const int *surv,
+                            const RngPlace &rng, uint64_t seed, const zd *wf, zd *wfTmp, zd *diag, zd *logw,
+                            double dtET, zd hopLogw, int *auxOut, cudaStream_t s);
+// (diag, W x 2L: the sample's diagonal instead of its application; for samples
+// without entries between the spins)
 
 // Phaseless (CholeskyReal) pieces
 struct CholDev {

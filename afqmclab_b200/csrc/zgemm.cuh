@@ -35,11 +35,19 @@ struct ZGemmArgs {
     // operators that do not mix them
     int parts = 1, m1 = 0, n1 = 0, k1 = 0;
     long long offA1 = 0, offB1 = 0, offC1 = 0;
+    // op(B)'s rows scaled by these factors (k per batch entry, strideScale apart;
+    // the second part's at offScale1): C = alpha op(A) diag(scale) B.  Both
+    // operators N.  One tile then holds all rows of C (m <= 128), and C may be B.
+    const zd *scaleB = nullptr;
+    long long strideScale = 0, offScale1 = 0;
 };
 
 // Launches on `stream`; returns cudaGetLastError() (cudaErrorInvalidValue for an
 // operator pair that no product of the engine has).
 cudaError_t zgemm_batched(const ZGemmArgs &a, cudaStream_t stream);
+
+// Whether scaleB is taken for a product of m rows.
+inline bool zgemm_scaled_supported(int m) { return m <= 128; }
 
 // Autotuner switch (process-wide) and the cached choice for a shape (-1: none).
 void zgemm_set_autotune(int on);

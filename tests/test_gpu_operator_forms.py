@@ -83,3 +83,30 @@ def test_molecule_forms(form, n, nup, ndn):
         m.chol[n - 1, 0, 3] += 0.01
     g, o = pair_pl(m, 4, 78, 1000, 1000)
     check(g, o, 78, 3)
+
+
+@pytest.mark.parametrize("decomp", ["densitySpin", "densityCharge", "hopSpin"])
+@pytest.mark.parametrize("nx,ny,fields", [(4, 8, False), (3, 11, False), (8, 8, True), (5, 13, False), (8, 16, False), (3, 43, False)])
+def test_sample_in_the_one_body_product(decomp, nx, ny, fields):
+    """A diagonal sample scales the one-body product's rows, in place where one
+    tile holds them (32, 64 and 128 sites are the tiles' ends); transverse
+    fields, hopping decompositions and larger lattices apply it on its own."""
+    m = hubbard(decomp, fields, nx=nx, ny=ny, nup=5, ndn=4)
+    g, o = pair_cp(m, 3, 79, 1000, 1000)
+    check(g, o, 79, 5)
+
+
+def test_dead_walkers_and_many_walkers_draw_from_their_own_place():
+    """The place in the random stream counts the survivors before a walker, in
+    the sampling kernel up to 4096 walkers and by the scan above."""
+    m = hubbard("densitySpin", False, nx=2, ny=2, nup=1, ndn=1)
+    for W in (7, 4096, 4097):
+        g, o = pair_cp(m, W, 80, 1000, 1000)
+        wf, lw, al = o.get_walkers()
+        al[::3] = 0
+        o.set_walkers(wf, lw, al)
+        g.set_walkers(wf, lw, al)
+        for _ in range(2):
+            g.step(1)
+            o.step(1)
+            compare_state(g, o, STEP_TOL)
