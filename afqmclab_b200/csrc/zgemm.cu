@@ -273,17 +273,17 @@ cudaError_t launch3(const ZGemmArgs &a, cudaStream_t s)
 }
 
 // The operator pairs and real operands that the engine's products have.
-template <class TL>
+template <class TL, bool ONE_REAL = false>
 cudaError_t launch2(const ZGemmArgs &a, cudaStream_t s)
 {
     const int real = (a.a_real ? 1 : 0) | (a.b_real ? 2 : 0);
 #define ZG_CASE(OA, OB, R) \
     if (a.opA == OA && a.opB == OB && real == R) return launch3<TL, OA, OB, R>(a, s);
-    ZG_CASE(OP_N, OP_N, 0) ZG_CASE(OP_N, OP_N, 1) ZG_CASE(OP_N, OP_N, 2)
-    ZG_CASE(OP_N, OP_T, 0) ZG_CASE(OP_N, OP_T, 1) ZG_CASE(OP_N, OP_T, 3)
-    ZG_CASE(OP_C, OP_N, 0) ZG_CASE(OP_C, OP_N, 2)
-    ZG_CASE(OP_T, OP_N, 0) ZG_CASE(OP_T, OP_N, 1)
-    ZG_CASE(OP_T, OP_T, 0) ZG_CASE(OP_T, OP_C, 0)
+    ZG_CASE(OP_N, OP_N, 1) ZG_CASE(OP_N, OP_N, 2) ZG_CASE(OP_N, OP_T, 1) ZG_CASE(OP_C, OP_N, 2) ZG_CASE(OP_T, OP_N, 1)
+    if constexpr (!ONE_REAL) {
+        ZG_CASE(OP_N, OP_N, 0) ZG_CASE(OP_N, OP_T, 0) ZG_CASE(OP_N, OP_T, 3) ZG_CASE(OP_C, OP_N, 0)
+        ZG_CASE(OP_T, OP_N, 0) ZG_CASE(OP_T, OP_T, 0) ZG_CASE(OP_T, OP_C, 0)
+    }
 #undef ZG_CASE
     return cudaErrorInvalidValue;
 }
@@ -305,20 +305,28 @@ constexpr int NCAND = 3;
 typedef Tile<32, 32, 16, 16, 8, 4, 4> TileS;
 typedef Tile<64, 32, 32, 16, 8, 4, 3> TileM;
 typedef Tile<64, 64, 32, 16, 16, 3, 2> TileL;
+// The largest for one real operand and a long contraction: half the products per
+// stage leave room for 32 columns of it in two stages, half the barriers (4096
+// x 2048 x 4096, real A, 4.24 -> 4.09 ms; 4096 x 640 x 4096, real B, 1.54 -> 1.48; the
+// complex form loses, 4.21 -> 4.56).
+typedef Tile<64, 64, 32, 16, 32, 2, 2> TileLR;
 
 cudaError_t launch_cand(int c, const ZGemmArgs &a, cudaStream_t s)
 {
     switch (c) {
     case 0: return launch2<TileS>(a, s);
     case 1: return launch2<TileM>(a, s);
-    default: return launch2<TileL>(a, s);
+    default:
+        if ((a.a_real != 0) != (a.b_real != 0) && a.k >= 256) return launch2<TileLR, true>(a, s);
+        return launch2<TileL>(a, s);
     }
 }
 
 // Time of the last-finishing SM in units of products: waves of CTAs (148 SMs,
 // MINB CTAs each) times the whole tile, over the tile's measured rate on
 // shapes that fill it (the smaller tiles pay more fragment loads and barriers
-// per product).  A tile counts in full where C covers part of it: the warps
+// per product; half of the largest one's warps lose their branch-free loop where
+// the rows end inside it: 56 x 128 x 56, 1024 walkers, 144 us against 137).  A tile counts in full where C covers part of it: the warps
 // outside C leave their SM quadrant's matrix pipe idle (32 x 32 outputs: 0.076
 // ms in 32 x 32 tiles, 0.140 in 64 x 32, 0.232 in 64 x 64).
 template <class TL>
@@ -350,7 +358,9 @@ cudaError_t launch_scaled(const ZGemmArgs &a, cudaStream_t s)
 
 int default_cand(const ZGemmArgs &a)
 {
-    const double c[NCAND] = {tile_cost<TileS>(a, 0.93), tile_cost<TileM>(a, 0.95), tile_cost<TileL>(a, 1.0)};
+    const bool ragged = a.m < 256 && a.m % 64 != 0;
+    const double c[NCAND] = {tile_cost<TileS>(a, 0.93), tile_cost<TileM>(a, 0.95),
+                             tile_cost<TileL>(a, ragged ? 0.9 : 1.0)};
     int best = 0;
     for (int i = 1; i < NCAND; ++i)
         if (c[i] < c[best]) best = i;
