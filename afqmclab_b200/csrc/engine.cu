@@ -597,9 +597,8 @@ int project_dtk_dtv(afqmc_engine *e)
         if (needTheta) { PHASE(AFQMC_PH_FORCE); TRY(xbar_gemm(e, bl)); }
         {
             PHASE(AFQMC_PH_SAMPLE);
-            launch_rng_scan(W, e->surv, 2 * e->G, e->counter, e->offs, s);
-            launch_pl_sample(W, e->cdv, e->xbar, e->surv, e->surv, e->alive, e->offs, e->seed,
-                             e->aux, e->forcePL, e->logw, e->dt * e->ET, hop, s);
+            launch_pl_sample(W, e->cdv, e->xbar, e->surv, e->alive, engine_rng_place(e, 2 * e->G), e->seed, e->aux,
+                             e->logw, e->dt * e->ET, hop, s);
             TRY(check_launch());
         }
         {
@@ -620,10 +619,10 @@ int project_dtk_dtv(afqmc_engine *e)
         const bool fused = !e->useLog && taylor_f64_supported(e->n, e->ncol);
         {
             PHASE(AFQMC_PH_TAYLOR);
-            TRY(taylor_apply(e, e->M, m_rows(e), e->wf, fused ? e->wf : e->wfTmp, e->surv, true,
+            TRY(taylor_apply(e, e->M, m_rows(e), e->wf, fused ? e->wf : e->wfTmp, e->alive, true,
                              e->cholP != nullptr, fused ? e->expK[0] : nullptr, fused ? e->expKr[0] : nullptr));
         }
-        if (!fused) { PHASE(AFQMC_PH_ONEBODY); TRY(one_body(e, 0, e->wfTmp, e->wf, e->surv)); }
+        if (!fused) { PHASE(AFQMC_PH_ONEBODY); TRY(one_body(e, 0, e->wfTmp, e->wf, e->alive)); }
     }
     return check_launch();
 }
@@ -1140,7 +1139,6 @@ int afqmc_pl_create(int n, int Nup, int Ndn, int G, int W, int force_type, doubl
         CK(gemm(h, e->stream));
     }
     CK(dalloc(e, &e->xbar, (size_t)G * W));
-    CK(dalloc(e, &e->forcePL, (size_t)G * W));
     CK(dalloc(e, &e->aux, (size_t)G * W));
     CK(dalloc(e, &e->ex, (size_t)G * W));
     CK(dalloc(e, &e->bgNum, G));

@@ -79,7 +79,7 @@ struct afqmc_engine {
     CholDev cdv{};
     double *chol = nullptr, *bg = nullptr, *tdev = nullptr;
     double *cholP = nullptr;   // symmetric L_g in panel storage (taylor_panel_size(n) x G)
-    zd *Aall = nullptr, *wfDaggerT = nullptr, *xbar = nullptr, *forcePL = nullptr, *aux = nullptr,
+    zd *Aall = nullptr, *wfDaggerT = nullptr, *xbar = nullptr, *aux = nullptr,
        *M = nullptr, *ex = nullptr, *constForcePL = nullptr;
     long long Ktot = 0;
     // measurement

@@ -166,30 +166,36 @@ __global__ void gather32_kernel(int W, long long ws32, const int *table, float *
 
 // Phaseless force from the tensor-core xbar partials, aux sampling, sample
 // log-weight and second cos projection (same arithmetic as the FP64 form),
-// writing y = sqrt(-dt) x as the bf16 operand of the two-body GEMM.  One warp
-// per walker (four walkers per block): a walker's sums need no block barrier
-// and more walkers are in flight per SM.  Each lane takes its fields two at a
-// time (g and g + 32): both fields' loads and Gaussians are issued before the
-// first field's stores, and the sums still run in field order.
-__global__ void __launch_bounds__(128, 4)
-mixed_sample_warp_kernel(int W, CholDev c, const float *xbarp, int splits, long long splitStride,
-                         int *surv, int *alive, const unsigned long long *offs, uint64_t seed,
-                         __nv_bfloat16 *Y, zd *logw, double dtET, zd hopLogw)
+// writing y = sqrt(-dt) x as the bf16 operand of the two-body GEMM.  One CTA of
+// four warps per walker: a walker's fields are a chain of FP64 log, sqrt and cos
+// per lane, five of them for 640 fields.  One warp per walker (twenty) with the
+// stream's scan before it took 35 us for 2048 walkers and 16 for 512 with 320
+// fields, this takes 34 and 10; ten CTAs per SM bound the registers at 48,
+// without which it took 45 and 9.  Each lane takes its fields two at a time (g
+// and g + 128): both fields' loads and Gaussians are issued before the first
+// field's stores.  Reads all of surv (rng_place), so a walker that the
+// projection kills is marked in alive alone.
+constexpr int MSAMPLE_NT = 128;
+__global__ void __launch_bounds__(MSAMPLE_NT, 10)
+mixed_sample_kernel(int W, CholDev c, const float *xbarp, int splits, long long splitStride, const int *surv,
+                    int *alive, RngPlace rng, uint64_t seed, __nv_bfloat16 *Y, zd *logw, double dtET, zd hopLogw)
 {
-    const int lane = threadIdx.x & 31;
-    const int w = blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (w >= W || !surv[w]) return;
+    __shared__ int scratch[33];
+    __shared__ double part[MSAMPLE_NT / 32][6];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int w = blockIdx.x;
     const int G = c.G;
-    const unsigned long long off = offs[w];
+    const unsigned long long off = rng_place(rng, W, w, surv, 2 * G, scratch);
+    if (!surv[w]) return;
     zd f2 = make_double2(0, 0), xf = make_double2(0, 0), xb = make_double2(0, 0);
-    for (int g0 = lane; g0 < G; g0 += 64) {
-        const int nf = g0 + 32 < G ? 2 : 1;
+    for (int g0 = tid; g0 < G; g0 += 2 * MSAMPLE_NT) {
+        const int nf = g0 + MSAMPLE_NT < G ? 2 : 1;
         double xr[2] = {0.0, 0.0}, xi[2] = {0.0, 0.0}, bgv[2] = {0.0, 0.0}, gs[2] = {0.0, 0.0};
         zd cf[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             if (u < nf) {
-                const int g = g0 + 32 * u;
+                const int g = g0 + MSAMPLE_NT * u;
                 bgv[u] = c.bg[g];
                 if (c.constForce) {
                     cf[u] = c.constForce[g];
@@ -203,11 +209,11 @@ mixed_sample_warp_kernel(int W, CholDev c, const float *xbarp, int splits, long 
         }
 #pragma unroll
         for (int u = 0; u < 2; ++u)
-            if (u < nf) gs[u] = rng_gaussian(seed, off + 2ULL * (g0 + 32 * u));
+            if (u < nf) gs[u] = rng_gaussian(seed, off + 2ULL * (g0 + MSAMPLE_NT * u));
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             if (u < nf) {
-                const int g = g0 + 32 * u;
+                const int g = g0 + MSAMPLE_NT * u;
                 zd f;
                 if (c.constForce) {
                     f = cf[u];
@@ -226,19 +232,28 @@ mixed_sample_warp_kernel(int W, CholDev c, const float *xbarp, int splits, long 
             }
         }
     }
-    f2.x = warp_sum(f2.x); f2.y = warp_sum(f2.y);
-    xf.x = warp_sum(xf.x); xf.y = warp_sum(xf.y);
-    xb.x = warp_sum(xb.x); xb.y = warp_sum(xb.y);
-    if (lane == 0) {
-        double phase = xf.y;
+    double v[6] = {f2.x, f2.y, xf.x, xf.y, xb.x, xb.y};
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        v[q] = warp_sum(v[q]);
+        if (lane == 0) part[tid >> 5][q] = v[q];
+    }
+    __syncthreads();
+    if (tid == 0) {
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            v[q] = part[0][q];
+            for (int t = 1; t < MSAMPLE_NT / 32; ++t) v[q] += part[t][q];
+        }
+        double phase = v[3];
         double cs = cos(phase);
         if (cs <= 0.0) {
-            alive[w] = 0; surv[w] = 0;
+            alive[w] = 0;
         } else {
             zd lw = logw[w];
             lw.x += log(cs);
-            zd smp = zsub(zscale(f2, 0.5), xf);
-            smp = zsub(smp, make_double2(-c.sqrtMinusDtIm * xb.y, c.sqrtMinusDtIm * xb.x));
+            zd smp = zsub(zscale(make_double2(v[0], v[1]), 0.5), make_double2(v[2], v[3]));
+            smp = zsub(smp, make_double2(-c.sqrtMinusDtIm * v[5], c.sqrtMinusDtIm * v[4]));
             zd t = zadd(smp, lw);
             t.x += dtET;
             logw[w] = zadd(hopLogw, t);
@@ -593,7 +608,7 @@ int launch_taylor(afqmc_engine *e, const CUtensorMap &mM, const CUtensorMap &mE,
     const int perSm = TaylorSmem<NC>::bytes(e->n) <= 112 * 1024 ? 2 : 1;
     int grid = std::min(e->W, perSm * sms);
     taylor_onebody_kernel<NC, 128><<<grid, 128, smem, e->stream>>>(
-        mM, mE, e->W, e->n, e->mx->wf32, e->surv, e->order, e->tstats, 30, 1e-10f, 5.9604645e-8f, 4, doOneBody,
+        mM, mE, e->W, e->n, e->mx->wf32, e->alive, e->order, e->tstats, 30, 1e-10f, 5.9604645e-8f, 4, doOneBody,
         e->status, e->mx->err);
     return engine_check_launch();
 }
@@ -1016,7 +1031,7 @@ int launch_taylor_ts(afqmc_engine *e, const CUtensorMap &mM, const CUtensorMap &
     const int grid = std::min(e->W, 2 * sms);
     auto kern = e->n == 128 ? taylor_ts_kernel<NC, 128> : taylor_ts_kernel<NC, 64>;
     kern<<<grid, 128, smem, e->stream>>>(
-        mM, mE, e->W, e->mx->wf32, e->surv, e->order, e->tstats, 30, 1e-10f, 5.9604645e-8f, 4,
+        mM, mE, e->W, e->mx->wf32, e->alive, e->order, e->tstats, 30, 1e-10f, 5.9604645e-8f, 4,
         e->status, e->mx->err);
     return engine_check_launch();
 }
@@ -1355,11 +1370,10 @@ int mixed_project_dtk_dtv(afqmc_engine *e)
     }
     {
         PHASE(AFQMC_PH_SAMPLE);
-        launch_rng_scan(W, e->surv, 2 * e->G, e->counter, e->offs, s);
-        mixed_sample_warp_kernel<<<(W + 3) / 4, 128, 0, s>>>(W, e->cdv, m->xbarp, m->splits,
-                                                            (long long)2 * e->G * W, e->surv, e->alive,
-                                                            e->offs, e->seed, m->Y, e->logw, e->dt * e->ET,
-                                                            engine_one_body_logw(e, 0));
+        const RngPlace rng = engine_rng_place(e, 2 * e->G);
+        mixed_sample_kernel<<<W, MSAMPLE_NT, 0, s>>>(W, e->cdv, m->xbarp, m->splits, (long long)2 * e->G * W, e->surv,
+                                                     e->alive, rng, e->seed, m->Y, e->logw, e->dt * e->ET,
+                                                     engine_one_body_logw(e, 0));
         MTRY(engine_check_launch());
     }
     {

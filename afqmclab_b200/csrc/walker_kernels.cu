@@ -1043,14 +1043,15 @@ __global__ void zconj_kernel(long long count, const zd *src, zd *dst)
 // afqmcPhaselessProjection.cpp:89-118.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-pl_sample_kernel(int W, CholDev c, const zd *xbar, int *surv, int *alive,
-                 const unsigned long long *offs, uint64_t seed, zd *aux, zd *force, zd *logw,
-                 double dtET, zd hopLogw)
+pl_sample_kernel(int W, CholDev c, const zd *xbar, const int *surv, int *alive, RngPlace rng, uint64_t seed,
+                 zd *aux, zd *logw, double dtET, zd hopLogw)
 {
     __shared__ double red[32];
+    __shared__ int scratch[33];
     const int w = blockIdx.x;
-    if (!surv[w]) return;
     const int G = c.G;
+    const unsigned long long place = rng_place(rng, W, w, surv, 2 * G, scratch);
+    if (!surv[w]) return;
     zd f2 = make_double2(0, 0), xf = make_double2(0, 0), xb = make_double2(0, 0);
     for (int g = threadIdx.x; g < G; g += blockDim.x) {
         zd f;
@@ -1063,10 +1064,9 @@ pl_sample_kernel(int W, CholDev c, const zd *xbar, int *surv, int *alive,
             double af = zabs(f);
             if (af > c.forceCap) f = make_double2(f.x * c.forceCap / af, f.y * c.forceCap / af);
         }
-        double gs = rng_gaussian(seed, offs[w] + 2ULL * g);
+        double gs = rng_gaussian(seed, place + 2ULL * g);
         zd x = make_double2(gs + f.x, f.y);
         aux[g + (size_t)G * w] = x;
-        force[g + (size_t)G * w] = f;
         zfma(f2, f, f);
         zfma(xf, x, f);
         zfma(xb, x, make_double2(c.bg[g], 0.0));
@@ -1078,7 +1078,7 @@ pl_sample_kernel(int W, CholDev c, const zd *xbar, int *surv, int *alive,
         double phase = xf.y;
         double cs = cos(phase);
         if (cs <= 0.0) {
-            alive[w] = 0; surv[w] = 0;
+            alive[w] = 0;   // surv is still being counted by other walkers
         } else {
             zd lw = logw[w];
             lw.x += log(cs);
@@ -1847,14 +1847,11 @@ void launch_cp_sample_apply(int W, const HubbardDev &h, const zd *thetaT, long l
                                                           dtET, hopLogw, auxOut);
 }
 
-void launch_pl_sample(int W, const CholDev &c, const zd *xbar, const int *surv_in, int *surv,
-                      int *alive, const unsigned long long *offs, uint64_t seed, zd *aux,
-                      zd *force, zd *logw, double dtET, zd hopLogw, cudaStream_t s)
+void launch_pl_sample(int W, const CholDev &c, const zd *xbar, const int *surv, int *alive, const RngPlace &rng,
+                      uint64_t seed, zd *aux, zd *logw, double dtET, zd hopLogw, cudaStream_t s)
 {
     g_launch_count++;
-    (void)surv_in;
-    pl_sample_kernel<<<W, 256, 0, s>>>(W, c, xbar, surv, alive, offs, seed, aux, force, logw, dtET,
-                                        hopLogw);
+    pl_sample_kernel<<<W, 256, 0, s>>>(W, c, xbar, surv, alive, rng, seed, aux, logw, dtET, hopLogw);
 }
 
 void launch_taylor_accum(int W, long long wsize, const zd *term, zd *wfNew, const int *surv,

@@ -106,9 +106,10 @@ struct CholDev {
     double forceCap, sqrtMinusDtIm;
     const zd *constForce;      // non-null for constForce
 };
-void launch_pl_sample(int W, const CholDev &c, const zd *xbar, const int *surv_in, int *surv,
-                      int *alive, const unsigned long long *offs, uint64_t seed, zd *aux,
-                      zd *force, zd *logw, double dtET, zd hopLogw, cudaStream_t s);
+// A walker that the second cos projection kills leaves alive; surv stays as the
+// overlap left it, so the products after the sample go by alive.
+void launch_pl_sample(int W, const CholDev &c, const zd *xbar, const int *surv, int *alive, const RngPlace &rng,
+                      uint64_t seed, zd *aux, zd *logw, double dtET, zd hopLogw, cudaStream_t s);
 
 // Taylor series bookkeeping: wfNew += term; convergence per walker
 void launch_taylor_accum(int W, long long wsize, const zd *term, zd *wfNew, const int *surv,
