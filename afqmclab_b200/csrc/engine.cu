@@ -184,8 +184,11 @@ int alloc_population(afqmc_engine *e)
     e->wsize = (long long)e->n * e->ncol;
     TRY(dalloc(e, &e->wf, (size_t)W * e->wsize));
     TRY(dalloc(e, &e->wfTmp, (size_t)W * e->wsize));
-    TRY(dalloc(e, &e->term[0], (size_t)W * e->wsize));
-    TRY(dalloc(e, &e->term[1], (size_t)W * e->wsize));
+    if (e->kind == KIND_PL && !taylor_f64_supported(e->n, e->ncol)) {
+        // the series' terms, for shapes beyond the fused Taylor kernel
+        TRY(dalloc(e, &e->term[0], (size_t)W * e->wsize));
+        TRY(dalloc(e, &e->term[1], (size_t)W * e->wsize));
+    }
     TRY(dalloc(e, &e->logw, W));
     TRY(dalloc(e, &e->logov, W));
     TRY(dalloc(e, &e->S, (size_t)W * e->bl.sStride));

@@ -118,6 +118,7 @@ zgemm_kernel(ZGemmArgs a)
     const int b = blockIdx.z / a.parts;
     const bool second = blockIdx.z % a.parts != 0;
     if (a.mask && a.mask[b] == 0) return;
+    if (a.skip && a.skip[b] != 0) return;
     const int m = second ? a.m1 : a.m, n = second ? a.n1 : a.n;
     // a quadratic form's rows get longer downwards: the longest start first
     const int tileM = (a.quad ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * BM, tileN = blockIdx.y * BN;
