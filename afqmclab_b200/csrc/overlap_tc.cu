@@ -15,13 +15,23 @@
 // Ns_b', row 2a = [Re T(:,a) | Im T(:,a)], row 2a+1 = [-Im T(:,a) | Re T(:,a)],
 // so the real and imaginary parts of S(a, c) land in neighbouring TMEM lanes.
 //
-// Persistent CTAs over tiles of BN walker columns (whole walkers), K = 2n in
-// chunks of 32:
+// Persistent CTAs over tiles of wpt whole walkers (at most BN columns), K = 2n
+// in chunks of 32:
 //   warp 0 lane 0 : TMA producer (O_hi, O_lo chunks; raw fp32 walker chunks)
 //   warp 1        : TMEM owner; lane 0 issues the UMMAs (double-buffered TMEM)
-//   warps 2..5    : split each walker chunk in place (hi) and beside it (lo)
-//   warps 6..9    : epilogue (TMEM lane quarter = warp % 4), one complex
+//   warps 2..9    : split each walker chunk in place (hi) and beside it (lo)
+//   warps 10..17  : epilogue (TMEM lane quarter = warp % 4; the two groups of
+//                   four take the 16-column blocks in turn), one complex
 //                   double per lane and column pair after a lane-pair exchange
+//
+// What bounds it: shared-memory traffic (operand loads, the split's read and
+// two writes, and the products' reads of them), then the FP64 stores of S.  A
+// tile reads the whole operator pair again, so it takes the number of walkers
+// that moves the fewest bytes through the busiest CTA (choose_wpt).  With
+// tiles of 128 columns, four epilogue warps and a division per element the
+// epilogue took as long as the products: n = 128, two blocks of 32, 2048
+// walkers 37 us before, 32.6 us now; n = 64, blocks of 16, 512 walkers 8.6 and
+// 7.5 us.
 #include <cudaTypedefs.h>
 
 #include <algorithm>
@@ -39,14 +49,15 @@ extern std::atomic<long long> g_launch_count;
 
 namespace {
 
-constexpr int BM = 128, BK = 32, BN = 128, STAGES = 3, NT = 320;
+constexpr int BM = 128, BK = 32, BN = 256, MAX_STAGES = 4, NSPLIT = 256, NEPI = 256,
+              NT = 64 + NSPLIT + NEPI;
 constexpr int A_BYTES = BM * BK * 4;
-constexpr int B_BYTES = BN * BK * 4;
-constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;
-constexpr size_t SMEM = 1024 + (size_t)STAGES * STAGE_BYTES + 256;
+constexpr size_t SMEM_CAP = 227 * 1024;
 
 struct OvArgs {
     int n, W, kbA, bnw, wpt, tiles, rows;
+    int stages;          // of 2 A_BYTES + 2 ncols BK floats
+    int tcols;           // TMEM columns of one accumulator buffer
     int nb, Ns[2], rowBase[2];
     long long sOff[2];
     uint32_t idesc;
@@ -61,32 +72,32 @@ ov_split_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_constant__
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *base = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const int ncols = p.wpt * p.bnw;
+    const int STAGES = p.stages, B_BYTES = ncols * BK * 4, STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;
     uint64_t *full = (uint64_t *)(base + STAGES * STAGE_BYTES);
-    uint64_t *split = full + STAGES;
-    uint64_t *empty = split + STAGES;
-    uint64_t *tfull = empty + STAGES;   // 2
+    uint64_t *split = full + MAX_STAGES;
+    uint64_t *empty = split + MAX_STAGES;
+    uint64_t *tfull = empty + MAX_STAGES;   // 2
     uint64_t *tempty = tfull + 2;       // 2
     uint32_t *tmemSlot = (uint32_t *)(tempty + 2);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int KT = 2 * p.kbA;
-    const int ncols = p.wpt * p.bnw;
-    const uint32_t bBytes = (uint32_t)(ncols * BK * 4);
     const int myTiles = (p.tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&full[s], 1);
-            mbar_init(&split[s], 128);
+            mbar_init(&split[s], NSPLIT);
             mbar_init(&empty[s], 1);
         }
-        for (int b = 0; b < 2; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], 128); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], NEPI); }
         fence_mbar_init();
         tma_prefetch_desc(&tAh);
         tma_prefetch_desc(&tAl);
         tma_prefetch_desc(&tB);
     }
-    if (warp == 1) { tmem_alloc(tmemSlot, 2 * BN); tmem_relinquish(); }
+    if (warp == 1) { tmem_alloc(tmemSlot, 2 * p.tcols); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -122,14 +133,14 @@ ov_split_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_constant__
                 const int buf = ti & 1;
                 if (ti >= 2) ok = mbar_wait(&tempty[buf], ((ti >> 1) - 1) & 1);
                 if (!ok) break;
-                const uint32_t d = tmem + (uint32_t)(buf * BN);
+                const uint32_t d = tmem + (uint32_t)(buf * p.tcols);
                 for (int kt = 0; kt < KT && ok; ++kt, ++it) {
                     const int s = it % STAGES;
                     ok = mbar_wait(&split[s], (it / STAGES) & 1);
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t st = smem_u32(base + s * STAGE_BYTES);
-                    const uint32_t ah = st, al = st + A_BYTES, bh = st + 2 * A_BYTES, bl = bh + B_BYTES;
+                    const uint32_t ah = st, al = st + A_BYTES, bh = st + 2 * A_BYTES, bl = bh + (uint32_t)B_BYTES;
 #pragma unroll
                     for (int k8 = 0; k8 < BK / 8; ++k8) {
                         const uint32_t acc0 = (kt > 0 || k8 > 0) ? 1u : 0u;
@@ -143,10 +154,10 @@ ov_split_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_constant__
             }
         }
         __syncwarp();
-    } else if (warp < 6) {
+    } else if (warp < 2 + NSPLIT / 32) {
         // split the raw walker chunk: hi in place, lo in the slot beside it
         const int t = threadIdx.x - 64;
-        const int n4 = (int)(bBytes / 16);
+        const int n4 = B_BYTES / 16;
         const int items = myTiles * KT;
         for (int it = 0; it < items && ok; ++it) {
             const int s = it % STAGES;
@@ -154,7 +165,8 @@ ov_split_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_constant__
             if (!ok) break;
             float4 *bh = (float4 *)(base + s * STAGE_BYTES + 2 * A_BYTES);
             float4 *bl = (float4 *)(base + s * STAGE_BYTES + 2 * A_BYTES + B_BYTES);
-            for (int i = t; i < n4; i += 128) {
+#pragma unroll 2
+            for (int i = t; i < n4; i += NSPLIT) {
                 const float4 x = bh[i];
                 float4 h, l;
                 h.x = tf32_round(x.x); l.x = x.x - h.x;
@@ -176,28 +188,30 @@ ov_split_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_constant__
         const int Ns = b ? p.Ns[1] : p.Ns[0];
         const long long sOff = b ? p.sOff[1] : p.sOff[0];
         const bool rowOK = row < p.rows;
-        const int odd = lane & 1;
+        const int odd = lane & 1, grp = (warp - 2 - NSPLIT / 32) >> 2;
         for (int ti = 0; ti < myTiles && ok; ++ti) {
             const int buf = ti & 1;
             ok = mbar_wait(&tfull[buf], (ti >> 1) & 1);
             if (!ok) break;
             tc_fence_after();
             const int t = (int)blockIdx.x + ti * (int)gridDim.x;
-            const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN);
+            const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * p.tcols);
 #pragma unroll 1
-            for (int c0 = 0; c0 < ncols; c0 += 32) {
-                float v[32];
-                tmem_ld32(trow + (uint32_t)c0, v);
+            for (int c0 = 16 * grp; c0 < ncols; c0 += 32) {
+                // bnw is a multiple of 16: these columns belong to one walker
+                const int wj = c0 / p.bnw, c = c0 - wj * p.bnw + odd;
+                const int w = t * p.wpt + wj;
+                float v[16];
+                tmem_ld16(trow + (uint32_t)c0, v);
+                double2 *out = p.S + (size_t)w * p.sStride + sOff + a + (size_t)Ns * c;
+                const bool rowW = rowOK && a < Ns && w < p.W;
 #pragma unroll
-                for (int j = 0; j < 32; j += 2) {
+                for (int j = 0; j < 16; j += 2) {
                     // even lane: Re S(a, col j) and Re S(a, col j+1); odd lane: the Im parts
                     const float send = odd ? v[j] : v[j + 1];
                     const float recv = __shfl_xor_sync(0xffffffffu, send, 1);
-                    const int col = c0 + j + odd;
-                    const int wj = col / p.bnw, c = col - wj * p.bnw;
-                    const int w = t * p.wpt + wj;
-                    if (rowOK && a < Ns && c < Ns && w < p.W)
-                        p.S[(size_t)w * p.sStride + sOff + a + (size_t)Ns * c] =
+                    if (rowW && c + j < Ns)
+                        out[(size_t)(Ns * j)] =
                             odd ? make_double2((double)recv, (double)v[j + 1]) : make_double2((double)v[j], (double)recv);
                 }
             }
@@ -209,7 +223,7 @@ ov_split_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_constant__
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 1) tmem_dealloc(tmem, 2 * BN);
+    if (warp == 1) tmem_dealloc(tmem, 2 * p.tcols);
 }
 
 // ---------------------------------------------------------------------------
@@ -433,6 +447,21 @@ int map_f32(CUtensorMap *map, const float *ptr, int rank, const cuuint64_t *dims
     return r == CUDA_SUCCESS ? 0 : (int)r + 10000;
 }
 
+// Walkers per tile: the count (at most BN columns) that moves the fewest bytes
+// through the busiest CTA, each tile being 2 operator chunks and wpt walker
+// chunks per K step.  Few walkers spread over the SMs one by one.
+int choose_wpt(int W, int bnw, int sms)
+{
+    int best = 1;
+    long long bestCost = -1;
+    for (int wpt = 1; wpt * bnw <= BN && wpt <= W; ++wpt) {
+        const long long tiles = (W + wpt - 1) / wpt, waves = (tiles + sms - 1) / sms;
+        const long long cost = waves * (2LL * BM + (long long)wpt * bnw);
+        if (bestCost < 0 || cost < bestCost) { best = wpt; bestCost = cost; }
+    }
+    return best;
+}
+
 float tf32_host(float x)
 {
     uint32_t u;
@@ -492,7 +521,7 @@ int overlap_tc_launch(cudaStream_t s, int n, int ncol, int nb, const int *Ns, in
     if (!overlap_tc_supported(n, nb, Ns)) return (int)cudaErrorInvalidValue;
     static std::atomic<unsigned long long> attr{0};
     if (first_on_device(attr)) {
-        cudaFuncSetAttribute(ov_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+        cudaFuncSetAttribute(ov_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_CAP);
     }
     OvArgs a{};
     a.n = n; a.W = W; a.nb = nb;
@@ -518,15 +547,18 @@ int overlap_tc_launch(cudaStream_t s, int n, int ncol, int nb, const int *Ns, in
     if (r) return r;
     a.kbA = (n + BK - 1) / BK;
     a.bnw = bnw;
-    a.wpt = std::max(1, BN / bnw);
-    a.tiles = (W + a.wpt - 1) / a.wpt;
-    a.idesc = idesc_tf32(BM, a.wpt * bnw);
-    a.S = S; a.sStride = sStride; a.err = err;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    a.wpt = choose_wpt(W, bnw, sms);
+    a.tiles = (W + a.wpt - 1) / a.wpt;
+    a.idesc = idesc_tf32(BM, a.wpt * bnw);
+    a.S = S; a.sStride = sStride; a.err = err;
+    const size_t stage = 2 * (size_t)A_BYTES + 2 * (size_t)a.wpt * bnw * BK * 4;
+    a.stages = std::min(MAX_STAGES, (int)((SMEM_CAP - 1024 - 256) / stage));
+    a.tcols = a.wpt * bnw <= 128 ? 128 : 256;
     g_launch_count++;
-    ov_split_kernel<<<std::min(a.tiles, sms), NT, SMEM, s>>>(ah, al, b, a);
+    ov_split_kernel<<<std::min(a.tiles, sms), NT, 1024 + a.stages * stage + 256, s>>>(ah, al, b, a);
     return (int)cudaGetLastError();
 }
 

@@ -20,9 +20,17 @@
 //   warp 0 lane 0 : producer (TMA walker chunks, bulk copy of the inverses)
 //   warp 1        : TMEM owner, UMMA issuer
 //   warps 2..9    : rewrite of P (K-major, hi/lo) and build of X (hi/lo)
-//   warps 10..13  : epilogue (double-buffered TMEM): TMEM lane = output
-//                   column, so each thread writes its column over the sites
-//                   with 16-byte stores
+//   warps 10..17  : epilogue (double-buffered TMEM): TMEM lane = output
+//                   column; two groups of four warps take one half of the
+//                   sites each.  The re and im lanes of a column exchange
+//                   8-site pieces so that each pair writes whole 32-byte
+//                   sectors, not 16 bytes of each.  Both together: n = 128,
+//                   two blocks of 32, 2048 walkers 55.5 -> 50.0 us, n = 64,
+//                   blocks of 16, 512 walkers 12.7 -> 11.4 us.
+// What is left is shared-memory bandwidth: per walker 64 KB of split operands
+// written twice and read by 24 products (about 3700 of 6500 cycles), and the
+// hand-over between converters and products; 16 converter warps instead of 8
+// spill (55.5 us).
 #include <cudaTypedefs.h>
 
 #include <algorithm>
@@ -39,7 +47,8 @@ extern std::atomic<long long> g_launch_count;
 namespace {
 
 constexpr int NCONV = 256;                 // converter threads (warps 2..9)
-constexpr int NT = 64 + NCONV + 128;       // + producer, MMA warps and 4 epilogue warps
+constexpr int NEPI = 256;                  // epilogue threads (warps 10..17)
+constexpr int NT = 64 + NCONV + NEPI;      // + producer and MMA warps
 constexpr int MAX_RS = 4, MAX_XS = 2, MAX_OS = 2;
 constexpr size_t SMEM_CAP = 227 * 1024;
 
@@ -120,7 +129,7 @@ theta_tc_kernel(const __grid_constant__ CUtensorMap tA, ThArgs p)
         for (int s = 0; s < p.RS; ++s) { mbar_init(&rawFull[s], 1); mbar_init(&rawEmpty[s], NCONV); }
         for (int s = 0; s < p.XS; ++s) { mbar_init(&xFull[s], 1); mbar_init(&xEmpty[s], NCONV); }
         for (int s = 0; s < p.OS; ++s) { mbar_init(&opFull[s], NCONV); mbar_init(&opEmpty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], 128); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], NEPI); }
         fence_mbar_init();
         tma_prefetch_desc(&tA);
     }
@@ -228,9 +237,16 @@ theta_tc_kernel(const __grid_constant__ CUtensorMap tA, ThArgs p)
                 float xr[4] = {0.f, 0.f, 0.f, 0.f}, xi[4] = {0.f, 0.f, 0.f, 0.f};
                 if (on && a < Ns) {
                     const float *Xr = xsrc + so + (size_t)Ns * a, *Xi = Xr + (size_t)Ns * Ns;
+                    if (((Ns | (int)so) & 3) == 0) {   // every column of the block starts on 16 bytes
+                        if (4 * g < Ns) {
+                            *(float4 *)xr = *(const float4 *)(Xr + 4 * g);
+                            *(float4 *)xi = *(const float4 *)(Xi + 4 * g);
+                        }
+                    } else {
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (4 * g + j < Ns) { xr[j] = Xr[4 * g + j]; xi[j] = Xi[4 * g + j]; }
+                        for (int j = 0; j < 4; ++j)
+                            if (4 * g + j < Ns) { xr[j] = Xr[4 * g + j]; xi[j] = Xi[4 * g + j]; }
+                    }
                 }
                 float vre[4], vim[4];
 #pragma unroll
@@ -257,6 +273,7 @@ theta_tc_kernel(const __grid_constant__ CUtensorMap tA, ThArgs p)
         const int Ns = b == 0 ? p.Ns[0] : (b == 1 ? p.Ns[1] : 0);
         const bool valid = b < p.nb && a < Ns;
         const long long tOff = b ? p.tOff[1] : p.tOff[0];
+        const int half = (warp - 2 - NCONV / 32) >> 2;
         for (int lw = 0; lw < nw && ok; ++lw) {
             const int buf = lw & 1;
             ok = mbar_wait_sleep(&tfull[buf], (lw >> 1) & 1);
@@ -264,20 +281,28 @@ theta_tc_kernel(const __grid_constant__ CUtensorMap tA, ThArgs p)
             tc_fence_after();
             const int w = (int)blockIdx.x + lw * (int)gridDim.x;
             const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * 128);
-            __nv_bfloat16 *th = p.Theta + (size_t)w * p.thetaStride + tOff + (size_t)im * p.plane + (size_t)n * a;
+            // the pair stores pieces 2k and 2k + 1 of both planes: the re lane the even ones
+            __nv_bfloat16 *th = p.Theta + (size_t)w * p.thetaStride + tOff + (size_t)n * a + 8 * im;
             double2 *tz = p.thetaZ ? (double2 *)(p.thetaZ + (size_t)w * p.zStride + tOff + (size_t)n * a) : nullptr;
-            for (int c0 = 0; c0 < n; c0 += 32) {
+            for (int c0 = half * (n >> 1); c0 < (half + 1) * (n >> 1); c0 += 32) {
                 float v[32];
                 tmem_ld32(trow + (uint32_t)c0, v);
-                if (valid) {
 #pragma unroll
-                    for (int j = 0; j < 32; j += 8) {
-                        uint4 pk;
-                        pk.x = pack_bf16x2(v[j], v[j + 1]);
-                        pk.y = pack_bf16x2(v[j + 2], v[j + 3]);
-                        pk.z = pack_bf16x2(v[j + 4], v[j + 5]);
-                        pk.w = pack_bf16x2(v[j + 6], v[j + 7]);
-                        *(uint4 *)(th + c0 + j) = pk;
+                for (int j = 0; j < 32; j += 16) {
+                    uint32_t mine[4], other[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const uint32_t e = pack_bf16x2(v[j + 2 * k], v[j + 2 * k + 1]);
+                        const uint32_t o = pack_bf16x2(v[j + 8 + 2 * k], v[j + 9 + 2 * k]);
+                        mine[k] = im ? o : e;
+                        other[k] = __shfl_xor_sync(0xffffffffu, im ? e : o, 1);
+                    }
+                    if (valid) {
+                        // re lane: own even piece, the im lane's even piece; im lane: the odd ones
+                        const uint4 m4 = make_uint4(mine[0], mine[1], mine[2], mine[3]);
+                        const uint4 o4 = make_uint4(other[0], other[1], other[2], other[3]);
+                        *(uint4 *)(th + c0 + j) = im ? o4 : m4;
+                        *(uint4 *)(th + p.plane + c0 + j) = im ? m4 : o4;
                     }
                 }
                 if (tz) {
