@@ -19,9 +19,10 @@
 // Y = R X (complex x real, K x G), each followed by a dot.  V, M and R are
 // symmetric: M is computed as its lower triangle, and Z and Y, which only the
 // dots read, take the off-diagonal blocks of V and R once and doubled
-// (ZGemmArgs::quad), half the products of the full ones.  n = 128, 32
-// electrons, 640 vectors, 2048 walkers: 10.7 -> 8.3 ms; n = 256, 64 electrons, 1280
-// vectors, 512 walkers: 80.2 -> 52.3 ms.
+// (ZGemmArgs::quad), half the products of the full ones; small outputs are sums of
+// pieces of the contraction (zgemm_pieces).  n = 128, 32
+// electrons, 640 vectors, 2048 walkers: 10.7 -> 7.9 ms; n = 256, 64 electrons, 1280
+// vectors, 512 walkers: 80.2 -> 46.1 ms.
 #include <algorithm>
 #include <atomic>
 #include <string>
@@ -55,10 +56,10 @@ __global__ void vf64_kernel(long long K, int Ns, const zd *C, double *V)
     }
 }
 
-// exTot[w] (+)= mult sum_q u_w(q) Z(q, w) for alive walkers
+// exTot[w] (+)= mult sum_q u_w(q) Z(q, w) for alive walkers, Z the sum of S pieces
 __global__ void __launch_bounds__(256)
 ex_walker_dot_kernel(long long K, const zd *U, long long ldu, const zd *Z, const int *alive, int mult,
-                     int accumulate, zd *exTot)
+                     int accumulate, zd *exTot, int S, long long strideS)
 {
     __shared__ double red[32];
     const int w = blockIdx.x;
@@ -66,7 +67,11 @@ ex_walker_dot_kernel(long long K, const zd *U, long long ldu, const zd *Z, const
     const zd *u = U + (size_t)w * ldu;
     const zd *z = Z + (size_t)w * K;
     zd s = make_double2(0.0, 0.0);
-    for (long long q = threadIdx.x; q < K; q += blockDim.x) zfma(s, u[q], z[q]);
+    for (long long q = threadIdx.x; q < K; q += blockDim.x) {
+        zd v = z[q];
+        for (int p = 1; p < S; ++p) v = zadd(v, z[q + p * strideS]);
+        zfma(s, u[q], v);
+    }
     s = block_zsum(s, red);
     if (threadIdx.x == 0) {
         s = zscale(s, (double)mult);
@@ -101,9 +106,9 @@ __global__ void ex_exchange_kernel(long long K, int Ns, const zd *M, zd *R, int 
     }
 }
 
-// exNum[g] += mult sum_q x_g(q) Y(q, g)
+// exNum[g] += mult sum_q x_g(q) Y(q, g), Y the sum of S pieces
 __global__ void __launch_bounds__(256)
-ex_vector_dot_kernel(long long K, const double *X, const zd *Y, int mult, zd *exNum)
+ex_vector_dot_kernel(long long K, const double *X, const zd *Y, int mult, zd *exNum, int S, long long strideS)
 {
     __shared__ double red[32];
     const int g = blockIdx.x;
@@ -111,8 +116,10 @@ ex_vector_dot_kernel(long long K, const double *X, const zd *Y, int mult, zd *ex
     const zd *y = Y + (size_t)g * K;
     zd s = make_double2(0.0, 0.0);
     for (long long q = threadIdx.x; q < K; q += blockDim.x) {
-        s.x = fma(x[q], y[q].x, s.x);
-        s.y = fma(x[q], y[q].y, s.y);
+        zd v = y[q];
+        for (int p = 1; p < S; ++p) v = zadd(v, y[q + p * strideS]);
+        s.x = fma(x[q], v.x, s.x);
+        s.y = fma(x[q], v.y, s.y);
     }
     s = block_zsum(s, red);
     if (threadIdx.x == 0) exNum[g] = zadd(exNum[g], zscale(s, (double)mult));
@@ -128,6 +135,33 @@ __global__ void ex_force_sum_kernel(long long count, int S, const zd *P, zd alph
         v = zmul(alpha, v);
         xbar[e] = accumulate ? zadd(xbar[e], v) : v;
     }
+}
+
+// The block's products, K = Ns n: Z = V U and Y = R X as quadratic forms, the
+// force X^T U.
+ZGemmArgs z_product(const afqmc_engine *e, long long K)
+{
+    ZGemmArgs z;
+    z.m = (int)K; z.n = e->W; z.k = (int)K; z.a_real = 1; z.quad = 1;
+    z.lda = K; z.ldb = e->bl.tStride; z.ldc = K;
+    return z;
+}
+
+ZGemmArgs y_product(const afqmc_engine *e, long long K)
+{
+    ZGemmArgs y;
+    y.m = (int)K; y.n = e->G; y.k = (int)K; y.b_real = 1; y.quad = 1;
+    y.lda = K; y.ldb = K; y.ldc = K;
+    return y;
+}
+
+ZGemmArgs force_product(const afqmc_engine *e, long long K)
+{
+    ZGemmArgs g;
+    g.m = e->G; g.n = e->W; g.k = (int)K;
+    g.opA = OP_T; g.opB = OP_N; g.a_real = ST_R64;
+    g.lda = K; g.ldb = e->bl.tStride; g.ldc = e->G;
+    return g;
 }
 
 int gemm_check(const ZGemmArgs &a, cudaStream_t s)
@@ -164,18 +198,23 @@ int exf64_build(afqmc_engine *e, int b, ExF64 &x)
 int exf64_alloc(afqmc_engine *e, long long Kmax, ExF64Scratch &s)
 {
     int r;
-    if ((r = engine_dalloc(e, &s.Z, (size_t)Kmax * e->W))) return r;
+    // outputs of few tiles are partial products over K (zgemm_pieces): the blocks'
+    // widest split sizes each buffer
+    size_t zCount = (size_t)Kmax * e->W, yCount = (size_t)Kmax * e->G, xCount = 0;
+    for (int b = 0; b < e->bl.nblk; ++b) {
+        const long long K = (long long)e->bl.Ns[b] * e->n;
+        if (K == 0) continue;
+        zCount = std::max(zCount, (size_t)K * e->W * zgemm_pieces(z_product(e, K)));
+        yCount = std::max(yCount, (size_t)K * e->G * zgemm_pieces(y_product(e, K)));
+        const int S = zgemm_pieces(force_product(e, K));
+        if (S > 1) xCount = std::max(xCount, (size_t)S * e->G * e->W);
+    }
+    if ((r = engine_dalloc(e, &s.Z, zCount))) return r;
     if ((r = engine_dalloc(e, &s.M, (size_t)Kmax * Kmax))) return r;
     if ((r = engine_dalloc(e, &s.R, (size_t)Kmax * Kmax))) return r;
-    if ((r = engine_dalloc(e, &s.Y, (size_t)Kmax * e->G))) return r;
+    if ((r = engine_dalloc(e, &s.Y, yCount))) return r;
+    if (xCount > 0 && (r = engine_dalloc(e, &s.xp, xCount))) return r;
     if ((r = engine_dalloc(e, &s.exTot, (size_t)e->W))) return r;
-    // the force's output (G x W) may be too few 64 x 64 tiles for the SMs:
-    // about four CTA slots' worth of work in partial products over K
-    const long long tiles = (long long)((e->G + 63) / 64) * ((e->W + 63) / 64);
-    int S = 1;
-    while (S < 8 && tiles * S < 592) S *= 2;
-    s.xsplit = S;
-    if (S > 1 && (r = engine_dalloc(e, &s.xp, (size_t)S * e->G * e->W))) return r;
     return AFQMC_OK;
 }
 
@@ -188,22 +227,18 @@ int exf64_force(afqmc_engine *e, const Blocks &bl)
     for (int b = 0; b < bl.nblk; ++b) {
         if (bl.Ns[b] == 0) continue;
         const ExF64 x = exf64_block(e, b);
-        int S = s.xsplit;
-        while (S > 1 && x.K % S) S /= 2;
-        ZGemmArgs g;
-        g.m = G; g.n = W; g.k = (int)(x.K / S);
-        g.opA = OP_T; g.opB = OP_N; g.a_real = ST_R64;
-        g.A = x.X; g.lda = x.K; g.strideA = x.K / S;
-        g.B = e->thetaT + e->bl.tOff[b]; g.ldb = e->bl.tStride; g.strideB = x.K / S;
+        ZGemmArgs g = force_product(e, x.K);
+        const int S = zgemm_split(g, zgemm_pieces(g), (long long)G * W);
+        g.A = x.X;
+        g.B = e->thetaT + e->bl.tOff[b];
         const zd mult = make_double2((double)bl.mult, 0.0);
         if (S == 1) {
-            g.C = e->xbar; g.ldc = G;
+            g.C = e->xbar;
             g.alpha = mult;
             g.beta = first ? make_double2(0.0, 0.0) : make_double2(1.0, 0.0);
             if ((r = gemm_check(g, e->stream))) return r;
         } else {
-            g.C = s.xp; g.ldc = G; g.strideC = (long long)G * W;
-            g.batch = S;
+            g.C = s.xp;
             if ((r = gemm_check(g, e->stream))) return r;
             g_launch_count++;
             ex_force_sum_kernel<<<296, 256, 0, e->stream>>>((long long)G * W, S, s.xp, mult, first ? 0 : 1,
@@ -232,13 +267,13 @@ int exf64_walker_totals(afqmc_engine *e, const ExF64 &x, bool accumulate, int mu
     cudaStream_t st = e->stream;
     int r;
     // Z = V U
-    ZGemmArgs z;
-    z.m = (int)K; z.n = W; z.k = (int)K; z.a_real = 1;
-    z.A = x.V; z.lda = K; z.B = U; z.ldb = ldu; z.C = s.Z; z.ldc = K;
-    z.quad = wantZ ? 0 : 1;
+    ZGemmArgs z = z_product(e, K);
+    if (wantZ) z.quad = 0;
+    const int S = wantZ ? 1 : zgemm_split(z, zgemm_pieces(z), K * W);
+    z.A = x.V; z.B = U; z.C = s.Z;
     if ((r = gemm_check(z, st))) return r;
     g_launch_count++;
-    ex_walker_dot_kernel<<<W, 256, 0, st>>>(K, U, ldu, s.Z, e->alive, mult, accumulate ? 1 : 0, s.exTot);
+    ex_walker_dot_kernel<<<W, 256, 0, st>>>(K, U, ldu, s.Z, e->alive, mult, accumulate ? 1 : 0, s.exTot, S, K * W);
     return engine_check_launch();
 }
 
@@ -278,12 +313,11 @@ int exf64_run(afqmc_engine *e, const ExF64 &x, bool accumulate, int mult)
     g_launch_count++;
     ex_exchange_kernel<<<1184, 256, 0, st>>>(K, x.Ns, s.M, s.R, 1);
     // Y = R X, exNum_g += x_g^T Y_g
-    ZGemmArgs y;
-    y.m = (int)K; y.n = G; y.k = (int)K; y.b_real = 1;
-    y.A = s.R; y.lda = K; y.B = x.X; y.ldb = K; y.C = s.Y; y.ldc = K;
-    y.quad = 1;
+    ZGemmArgs y = y_product(e, K);
+    const int S = zgemm_split(y, zgemm_pieces(y), K * G);
+    y.A = s.R; y.B = x.X; y.C = s.Y;
     if ((r = gemm_check(y, st))) return r;
     g_launch_count++;
-    ex_vector_dot_kernel<<<G, 256, 0, st>>>(K, x.X, s.Y, mult, e->exNum);
+    ex_vector_dot_kernel<<<G, 256, 0, st>>>(K, x.X, s.Y, mult, e->exNum, S, K * G);
     return engine_check_launch();
 }

@@ -14,14 +14,13 @@ struct ExF64 {
 };
 
 // The FP64 form's closed-shell and GEMM-exchange state: per-block operands,
-// shared scratch (Z: K x W, M and R: K x K, Y: K x G) and the per-walker
+// shared scratch (Z: K x W and Y: K x G, one per piece of their
+// contraction; M and R: K x K) and the per-walker
 // exchange totals; `restricted` when both spin blocks carry the same trial
 // bit for bit (bl1 lists block 0 with multiplicity 2).
 struct ExF64Scratch {
     zd *Z = nullptr, *M = nullptr, *R = nullptr, *Y = nullptr, *exTot = nullptr;
-    // the force's K split: xsplit partial products (G x W each) in xp
-    zd *xp = nullptr;
-    int xsplit = 1;
+    zd *xp = nullptr;   // the force's partial products (G x W each)
     ExF64 blk[2];
     bool gemm = false, restricted = false;
     Blocks bl1{};

@@ -124,7 +124,12 @@ zgemm_kernel(ZGemmArgs a)
     const int tileM = (a.quad ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * BM, tileN = blockIdx.y * BN;
     if (tileM >= m || tileN >= n) return;
     if (a.lower && tileM + BM <= tileN) return;
-    const int k = a.quad ? min(a.k, tileM + BM) : second ? a.k1 : a.k;
+    int k = second ? a.k1 : a.k;
+    const int kBegin = a.ksum ? b * a.k : 0;   // this piece's place in the contraction
+    if (a.quad || a.ksum) {
+        const int kAll = a.ksum ? a.ksum : a.k;
+        k = max(0, min(a.k, (a.quad ? min(kAll, tileM + BM) : kAll) - kBegin));
+    }
 
     extern __shared__ __align__(16) unsigned char smem[];
     const unsigned smem0 = (unsigned)__cvta_generic_to_shared(smem);
@@ -146,7 +151,9 @@ zgemm_kernel(ZGemmArgs a)
         for (int j = 0; j < NI; ++j) cr[i][j][0] = cr[i][j][1] = ci[i][j][0] = ci[i][j][1] = 0.0;
 
     const int KT = (k + BK - 1) / BK;
-    const int ktDiag = a.quad && tileM > 0 ? tileM / BK : -1;   // first stage of the diagonal block
+    // first stage of the diagonal block (KT: it lies in a later piece)
+    const int left = a.quad ? tileM - kBegin : 0;
+    const int ktDiag = left <= 0 ? -1 : left >= k ? KT : left / BK;
     static_assert(BM % BK == 0, "a diagonal block starts a stage");
 #pragma unroll
     for (int s = 0; s < ST - 1; ++s) {
@@ -203,6 +210,14 @@ zgemm_kernel(ZGemmArgs a)
             }
         }
     };
+    auto twice = [&] {
+#pragma unroll
+        for (int i = 0; i < MI; ++i)
+#pragma unroll
+            for (int j = 0; j < NI; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) { cr[i][j][h] *= 2.0; ci[i][j][h] *= 2.0; }
+    };
     const bool full = mb >= MI && nb >= NI;
     int slot = 0, fill = ST - 1;
     for (int kt = 0; kt < KT; ++kt) {
@@ -220,14 +235,7 @@ zgemm_kernel(ZGemmArgs a)
             lb.load(smem0 + fill * (unsigned)SH::STAGE + (unsigned)LA::BYTES, kt + ST - 1);
         }
         cp_async_commit();
-        if (kt == ktDiag) {
-#pragma unroll
-            for (int i = 0; i < MI; ++i)
-#pragma unroll
-                for (int j = 0; j < NI; ++j)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) { cr[i][j][h] *= 2.0; ci[i][j][h] *= 2.0; }
-        }
+        if (kt == ktDiag) twice();
         const typename LA::T *As = (const typename LA::T *)(smem + slot * SH::STAGE);
         const typename LB::T *Bs = (const typename LB::T *)(smem + slot * SH::STAGE + LA::BYTES);
         if (full) products(std::true_type{}, As, Bs);
@@ -235,6 +243,7 @@ zgemm_kernel(ZGemmArgs a)
         slot = slot + 1 == ST ? 0 : slot + 1;
         fill = fill + 1 == ST ? 0 : fill + 1;
     }
+    if (ktDiag == KT) twice();
 
     zd *Cb = a.C + (size_t)b * a.strideC + (second ? a.offC1 : 0);
     const bool beta0 = (a.beta.x == 0.0 && a.beta.y == 0.0);
@@ -323,7 +332,7 @@ cudaError_t launch_cand(int c, const ZGemmArgs &a, cudaStream_t s)
     }
 }
 
-// Time of the last-finishing SM in units of products: waves of CTAs (148 SMs,
+// Time of the last-finishing SM in products: waves of CTAs (148 SMs,
 // MINB CTAs each) times the whole tile, over the tile's measured rate on
 // shapes that fill it (the smaller tiles pay more fragment loads and barriers
 // per product; half of the largest one's warps lose their branch-free loop where
@@ -333,13 +342,20 @@ cudaError_t launch_cand(int c, const ZGemmArgs &a, cudaStream_t s)
 template <class TL>
 double tile_cost(const ZGemmArgs &a, double rate)
 {
+    // a quadratic form's pieces end where the row block ends: their total length
+    // over the slots, and half the longest for the last ones to finish
+    if (a.quad) {
+        const double t = (double)((a.m + TL::BM - 1) / TL::BM) * ((a.n + TL::BN - 1) / TL::BN) / (148.0 * TL::MINB);
+        const double all = a.ksum ? a.ksum : a.k, piece = a.k;
+        return std::max(piece, 0.5 * t * all + 0.5 * piece) * TL::MINB * TL::BM * TL::BN / rate;
+    }
     double tiles = (double)((a.m + TL::BM - 1) / TL::BM) * ((a.n + TL::BN - 1) / TL::BN);
     if (a.parts > 1) tiles += (double)((a.m1 + TL::BM - 1) / TL::BM) * ((a.n1 + TL::BN - 1) / TL::BN);
-    tiles *= a.batch * (a.lower || a.quad ? 0.5 : 1.0);
+    tiles *= a.batch * (a.lower ? 0.5 : 1.0);
     double waves = tiles / (148.0 * TL::MINB);
     // beyond a few waves the ragged last one overlaps the stragglers
     waves = waves < 4.0 ? (double)(long long)(waves + 0.999999) : waves + 0.5;
-    return waves * TL::MINB * TL::BM * TL::BN / rate;
+    return waves * a.k * TL::MINB * TL::BM * TL::BN / rate;
 }
 
 // C = A diag(scale) B in one tile per column block, so that C may be B: 32 x 32 up
@@ -357,7 +373,7 @@ cudaError_t launch_scaled(const ZGemmArgs &a, cudaStream_t s)
     return cudaErrorInvalidValue;
 }
 
-int default_cand(const ZGemmArgs &a)
+double cand_cost(const ZGemmArgs &a, int *cand)
 {
     const bool ragged = a.m < 256 && a.m % 64 != 0;
     const double c[NCAND] = {tile_cost<TileS>(a, 0.93), tile_cost<TileM>(a, 0.95),
@@ -365,19 +381,55 @@ int default_cand(const ZGemmArgs &a)
     int best = 0;
     for (int i = 1; i < NCAND; ++i)
         if (c[i] < c[best]) best = i;
-    return best;
+    if (cand) *cand = best;
+    return c[best];
 }
 
 std::mutex g_tune_mu;
-typedef std::tuple<int, int, int, int, int, int, int, int, int> TuneKey;
+typedef std::tuple<int, int, int, int, int, int, int, int, int, int> TuneKey;
 TuneKey tune_key(const ZGemmArgs &a)
 {
-    return TuneKey(a.m, a.n, a.k, a.opA, a.opB, a.a_real, a.b_real, a.batch, a.lower + 2 * a.quad + 4 * a.parts);
+    return TuneKey(a.m, a.n, a.k, a.opA, a.opB, a.a_real, a.b_real, a.batch, a.lower + 2 * a.quad + 4 * a.parts, a.ksum);
 }
 std::map<TuneKey, int> g_tuned;
 std::atomic<int> g_autotune{0};
 
 }  // namespace
+
+// A piece more costs its output written and read once more (as much as 40 elements of
+// the contraction) and the stages in flight at its start (32); the sum is a
+// launch.  The pieces take at most 256 MB.  In one piece and in those chosen: force
+// 277 x 300 x 1890 72 us (two equal pieces) and 42 (six; the best of a sweep over
+// pieces and tiles is 37); forms 1890 x 300 164 and 113 (five; 109), 1024 x 512 74
+// and 58 (four; 55), 4096 x 640 911 and 748 (four; 725), 16384 x 512 9.69 ms and
+// 8.54 (two; 8.43), 16384 x 1280 20.6 ms in one, within 0.3% of the best.
+int zgemm_pieces(const ZGemmArgs &a)
+{
+    int best = 1;
+    double bestCost = 0.0;
+    for (int p = 1; p <= 8 && (p == 1 || (double)a.m * a.n * p <= (1 << 24)); ++p) {
+        ZGemmArgs s = a;
+        if (zgemm_split(s, p, 0) != p) continue;
+        double cost = cand_cost(s, nullptr) * (s.k + 32.0) / s.k;
+        if (p > 1) cost += (double)a.m * a.n / 148.0 * 40.0 * p + (a.quad ? 0.0 : 2e5);
+        if (p == 1 || cost < bestCost) { best = p; bestCost = cost; }
+    }
+    return best;
+}
+
+int zgemm_split(ZGemmArgs &a, int pieces, long long strideC)
+{
+    if (pieces <= 1) return 1;
+    const int all = a.k;
+    a.k = (all + pieces - 1) / pieces;
+    if (a.quad) a.k = (a.k + 63) / 64 * 64;
+    a.ksum = all;
+    a.batch = (all + a.k - 1) / a.k;
+    a.strideA = a.opA == OP_N ? a.lda * a.k : a.k;
+    a.strideB = a.opB == OP_N ? a.k : a.ldb * a.k;
+    a.strideC = strideC;
+    return a.batch;
+}
 
 void zgemm_set_autotune(int on) { g_autotune = on; }
 
@@ -429,6 +481,6 @@ cudaError_t zgemm_batched(const ZGemmArgs &a, cudaStream_t stream)
         std::lock_guard<std::mutex> lock(g_tune_mu);
         g_tuned[key] = choice;
     }
-    if (choice < 0) choice = default_cand(a);
+    if (choice < 0) cand_cost(a, &choice);
     return launch_cand(choice, a, stream);
 }

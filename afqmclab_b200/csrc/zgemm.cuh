@@ -30,6 +30,10 @@ struct ZGemmArgs {
     // and the blocks left of it twice, half the products.  Only A's entries
     // with row >= column and its 64 x 64 diagonal blocks are read.
     int quad = 0;
+    // > 0: the batch entries are pieces of one contraction over ksum elements:
+    // entry b takes the k from b k on (those that are left at the end; none: C_b =
+    // 0), and strideA, strideB step by k of them.  With quad k is a multiple of 64.
+    int ksum = 0;
     // A second product in the same launch and batch (parts = 2), of its own
     // sizes and at these element offsets from A, B and C: the two spins of
     // operators that do not mix them
@@ -45,6 +49,12 @@ struct ZGemmArgs {
 // Launches on `stream`; returns cudaGetLastError() (cudaErrorInvalidValue for an
 // operator pair that no product of the engine has).
 cudaError_t zgemm_batched(const ZGemmArgs &a, cudaStream_t stream);
+
+// Pieces (1 to 8) of the contraction of `a` (batch 1) for which the product and
+// the sum of the pieces take the least time: small outputs leave SMs idle.
+int zgemm_pieces(const ZGemmArgs &a);
+// `a` as that many pieces whose outputs are strideC apart; returns their number.
+int zgemm_split(ZGemmArgs &a, int pieces, long long strideC);
 
 // Whether scaleB is taken for a product of m rows.
 inline bool zgemm_scaled_supported(int m) { return m <= 128; }
