@@ -6,9 +6,9 @@
 // A CTA holds 16 columns of one walker and all n rows: the current term in
 // shared memory (the right operand of the next order), the running sum in
 // the registers that also define the accumulator layout (a warp owns 16 rows
-// by 16 columns).  M is streamed through four cp.async stages of 8 columns,
-// once per order; the walkers in flight (148 SMs times n^2 16 bytes per walker,
-// 39 MB at n = 128) stay in L2, so memory sees M once.  The CTAs of one
+// by 16 columns).  M is streamed through three or four cp.async stages of 8
+// columns, once per order; the walkers in flight (148 SMs times n^2 16 bytes per
+// walker, 39 MB at n = 128) stay in L2, so memory sees M once.  The CTAs of one
 // walker form a cluster: the stopping test is the walker's largest term, so
 // each order from `checkFrom` on ends with one exchange of maxima over
 // distributed shared memory.
@@ -41,7 +41,6 @@ namespace {
 
 constexpr int TF_COLS = 16;      // columns of phi per CTA
 constexpr int TF_BK = 8;         // columns of M per stage
-constexpr int TF_STAGES = 4;
 constexpr int TF_MAXN = 256;     // 16 rows per warp, 16 warps
 constexpr int TF_MAXCL = 8;      // CTAs per walker (portable cluster size)
 
@@ -51,9 +50,9 @@ __host__ __device__ constexpr int tf_rows(int n) { return (n + 15) / 16 * 16; }
 __host__ __device__ constexpr int tf_lda(int n) { return tf_rows(n) + 2; }
 __host__ __device__ constexpr int tf_ldt(int n) { return tf_rows(n) + 4; }
 __host__ __device__ constexpr size_t tf_stage(int n) { return (size_t)TF_BK * tf_lda(n) * sizeof(zd); }
-__host__ __device__ constexpr size_t tf_smem(int n)
+__host__ __device__ constexpr size_t tf_smem(int n, int stages)
 {
-    return TF_STAGES * tf_stage(n) + (size_t)TF_COLS * tf_ldt(n) * sizeof(zd);
+    return stages * tf_stage(n) + (size_t)TF_COLS * tf_ldt(n) * sizeof(zd);
 }
 
 struct TfAcc {
@@ -68,7 +67,7 @@ struct TfAcc {
 // triangle packed by columns; a tile's rows above the diagonal block come from
 // the mirrored entries, 8 neighbouring threads taking one row's 8 columns (128
 // contiguous bytes).
-template <bool REAL, bool PACKED>
+template <bool REAL, bool PACKED, int STAGES>
 struct TfStream {
     const void *base;
     int n, npad, KT, it;
@@ -82,12 +81,12 @@ struct TfStream {
         r = threadIdx.x % npad;
         k0 = threadIdx.x / npad;   // 0 or 1: the CTA has 2 npad threads
 #pragma unroll
-        for (int s = 0; s < TF_STAGES - 1; ++s) fill(s);
+        for (int s = 0; s < STAGES - 1; ++s) fill(s);
     }
     __device__ __forceinline__ void fill(int at)
     {
         constexpr int E = REAL ? 8 : 16;
-        const int kt = at % KT, slot = at % TF_STAGES;
+        const int kt = at % KT, slot = at % STAGES;
         const int ld = REAL ? npad + 4 : npad + 2;
         const unsigned dst = st0 + (unsigned)(slot * stage);
         const int c0 = kt * TF_BK;
@@ -138,10 +137,10 @@ struct TfStream {
                                            int nb, TfAcc &c)
     {
         for (int kt = 0; kt < KT; ++kt, ++it) {
-            cp_async_wait<TF_STAGES - 2>();
+            cp_async_wait<STAGES - 2>();
             __syncthreads();
-            fill(it + TF_STAGES - 1);
-            const unsigned char *sp = smem + (it % TF_STAGES) * stage;
+            fill(it + STAGES - 1);
+            const unsigned char *sp = smem + (it % STAGES) * stage;
 #pragma unroll
             for (int k4 = 0; k4 < TF_BK; k4 += 4) {
                 double ar[2], ai[2], an[2];
@@ -173,8 +172,8 @@ struct TfStream {
     }
 };
 
-template <bool PACKED>
-__global__ void __launch_bounds__(2 * TF_MAXN, 1)
+template <bool PACKED, int MAXT, int MINB, int STAGES>
+__global__ void __launch_bounds__(MAXT, MINB)
 taylor_f64_kernel(TaylorF64 a)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -185,12 +184,12 @@ taylor_f64_kernel(TaylorF64 a)
     const int col0 = rank * TF_COLS, ncols = min(TF_COLS, N - col0), nb = (ncols + 7) / 8;
     const int ldt = tf_ldt(n);
     const size_t stage = tf_stage(n);
-    zd *T = (zd *)(smem + TF_STAGES * stage);
+    zd *T = (zd *)(smem + STAGES * stage);
     const unsigned st0 = (unsigned)__cvta_generic_to_shared(smem);
     const int tid = threadIdx.x, NT = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const int wr = warp * 16, fr = lane >> 2, fk = lane & 3;
 
-    TfStream<false, PACKED> ms;
+    TfStream<false, PACKED, STAGES> ms;
     ms.start(a.M + (size_t)w * a.Mstride, n, st0, stage);
     const zd *src = a.src + ((size_t)w * N + col0) * n;
     for (int e = tid; e < TF_COLS * tf_rows(n); e += NT) {
@@ -264,11 +263,11 @@ taylor_f64_kernel(TaylorF64 a)
                     T[(size_t)(8 * j + 2 * fk + h) * ldt + wr + 8 * i + fr] =
                         make_double2(sum.r[i][j][h], sum.i[i][j][h]);
         if (a.postR) {
-            TfStream<true, false> ps;
+            TfStream<true, false, STAGES> ps;
             ps.start(a.postR, n, st0, stage);
             ps.product(smem, T, ldt, wr, fr, fk, nb, sum);
         } else {
-            TfStream<false, false> ps;
+            TfStream<false, false, STAGES> ps;
             ps.start(a.postZ, n, st0, stage);
             ps.product(smem, T, ldt, wr, fr, fk, nb, sum);
         }
@@ -292,20 +291,21 @@ taylor_f64_kernel(TaylorF64 a)
 
 bool taylor_f64_supported(int n, int N) { return n <= TF_MAXN && N <= TF_COLS * TF_MAXCL; }
 
-template <bool PACKED>
+template <bool PACKED, int MAXT, int MINB, int STAGES>
 static cudaError_t launch(const TaylorF64 &a, cudaStream_t s)
 {
+    const auto kernel = taylor_f64_kernel<PACKED, MAXT, MINB, STAGES>;
     static std::atomic<unsigned long long> attr{0};
     cudaError_t r = each_device_once(attr, [] {
-        return cudaFuncSetAttribute(taylor_f64_kernel<PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)tf_smem(TF_MAXN));
+        return cudaFuncSetAttribute(taylor_f64_kernel<PACKED, MAXT, MINB, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)tf_smem(MAXT / 2, STAGES));
     });
     if (r != cudaSuccess) return r;
     const int cs = (a.N + TF_COLS - 1) / TF_COLS;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)cs * (unsigned)a.W);
     cfg.blockDim = dim3((unsigned)(2 * tf_rows(a.n)));
-    cfg.dynamicSmemBytes = tf_smem(a.n);
+    cfg.dynamicSmemBytes = tf_smem(a.n, STAGES);
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -314,12 +314,21 @@ static cudaError_t launch(const TaylorF64 &a, cudaStream_t s)
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    r = cudaLaunchKernelEx(&cfg, taylor_f64_kernel<PACKED>, a);
+    r = cudaLaunchKernelEx(&cfg, kernel, a);
     return r != cudaSuccess ? r : cudaGetLastError();
 }
 
+// 128 registers a thread, four stages.  192 threads (n = 81..96) take 96
+// registers so that three CTAs are resident instead of two, 288 (n = 129..144) two
+// instead of one: n = 90, N = 21, 300 walkers 303 -> 277 us; n = 64 and 128, whose
+// number of CTAs stays the same, 98 us either way and 2.47 against 2.49 ms.  Above
+// that one CTA per SM has three stages: n = 256 6.00 -> 5.81 ms (n = 64 and 128 with
+// three: 98 us and 2.51 ms).
 cudaError_t taylor_f64(const TaylorF64 &a, cudaStream_t s)
 {
     g_launch_count++;
-    return a.packed ? launch<true>(a, s) : launch<false>(a, s);
+    const int nt = 2 * tf_rows(a.n);
+    if (nt == 192 || nt == 288) return a.packed ? launch<true, 288, 2, 4>(a, s) : launch<false, 288, 2, 4>(a, s);
+    if (nt <= 256) return a.packed ? launch<true, 256, 2, 4>(a, s) : launch<false, 256, 2, 4>(a, s);
+    return a.packed ? launch<true, 512, 1, 3>(a, s) : launch<false, 512, 1, 3>(a, s);
 }
