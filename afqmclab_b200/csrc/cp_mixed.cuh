@@ -22,6 +22,7 @@ int cp_mixed_modify_gm(afqmc_engine *e);
 int cp_mixed_pop_control(afqmc_engine *e);
 int cp_mixed_pop_weights(afqmc_engine *e);
 int cp_mixed_sync_to_fp64(afqmc_engine *e);
+int cp_mixed_pack_walkers(afqmc_engine *e, int count, const int *idx, zd *buf);
 int cp_mixed_sync_from_fp64(afqmc_engine *e);
 int cp_mixed_status(afqmc_engine *e);
 // the measurement's half step and overlap on the tensor cores (S in e->S,

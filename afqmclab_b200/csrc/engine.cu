@@ -2233,6 +2233,11 @@ int walker_xfer(afqmc_engine *e, int count, const int *idx, zd *buf, bool unpack
         if (unpack && seen[idx[k]]++) return fail(AFQMC_ERR_ARG, "a slot appears twice in the unpack list");
     }
     CUDA_TRY(cudaMemcpyAsync(e->table, idx, sizeof(int) * count, cudaMemcpyHostToDevice, e->stream));
+    if (e->precision == AFQMC_MIXED && !unpack) {
+        TRY(mixed_pack_walkers(e, count, e->table, buf));
+        CUDA_TRY(cudaStreamSynchronize(e->stream));
+        return AFQMC_OK;
+    }
     if (e->precision == AFQMC_MIXED) TRY(mixed_sync_to_fp64(e));
     launch_walker_xfer(count, e->wsize, e->table, e->wf, e->logw, buf, unpack, e->stream);
     TRY(check_launch());

@@ -152,6 +152,21 @@ __global__ void f32p_to_wf_kernel(int W, long long wsize, const float *w32, zd *
                                                  w32[(size_t)w * 2 * wsize + wsize + e]);
 }
 
+// Transfer record k = walker idx[k] in FP64 and its log-weight: bound by memory, 8
+// bytes read and 16 written per element, of the packed walkers only (by way of
+// the FP64 population: 16 + 8 for all walkers and 16 + 16 for the packed ones;
+// 2048 walkers of 128 x 32 85 us that way, 39 here)
+__global__ void pack_f32p_kernel(int count, long long wsize, const int *idx, const float *w32, const zd *logw, zd *buf)
+{
+    const int w = idx[blockIdx.x];
+    zd *rec = buf + (size_t)blockIdx.x * (wsize + 1);
+    const float *re = w32 + (size_t)w * 2 * wsize, *im = re + wsize;
+#pragma unroll 4
+    for (long long e = threadIdx.x; e < wsize; e += blockDim.x)
+        rec[e] = make_double2((double)re[e], (double)im[e]);
+    if (threadIdx.x == 0) rec[wsize] = logw[w];
+}
+
 // populationControl<T> in-place copies of fp32 walkers (populationControl.h:110-117)
 __global__ void gather32_kernel(int W, long long ws32, const int *table, float *w32, zd *logw)
 {
@@ -1322,6 +1337,13 @@ int mixed_sync_from_fp64(afqmc_engine *e)
 {
     if (e->kind == KIND_CP) return cp_mixed_sync_from_fp64(e);
     wf_to_f32p_kernel<<<e->W, 256, 0, e->stream>>>(e->W, e->wsize, e->wf, e->mx->wf32, nullptr);
+    return engine_check_launch();
+}
+
+int mixed_pack_walkers(afqmc_engine *e, int count, const int *idx, zd *buf)
+{
+    if (e->kind == KIND_CP) return cp_mixed_pack_walkers(e, count, idx, buf);
+    pack_f32p_kernel<<<count, 256, 0, e->stream>>>(count, e->wsize, idx, e->mx->wf32, e->logw, buf);
     return engine_check_launch();
 }
 

@@ -12,6 +12,9 @@ int mixed_add_measurement(afqmc_engine *e);
 int mixed_update_operators(afqmc_engine *e);
 // keep the FP64 walker copy and the reduced-precision working copy in step
 int mixed_sync_to_fp64(afqmc_engine *e);
+// Transfer records (walker matrix in FP64, then its log-weight) of the `count`
+// walkers idx, straight from the mixed form's planes.
+int mixed_pack_walkers(afqmc_engine *e, int count, const int *idx, zd *buf);
 int mixed_sync_from_fp64(afqmc_engine *e);
 // The phaseless mixed form can take a population (FP64, reference layout) into
 // its fp32 walkers directly from another device buffer; the FP64 copy is
