@@ -292,7 +292,7 @@ int theta_gemm(afqmc_engine *e, const zd *wf, const int *mask, const Blocks &bl)
 // one-body 0.266 -> 0.090 (its traffic alone is 0.036).
 //
 // The blocks of thetaT that the Hubbard force reads when the trial keeps the
-// spins apart (cp_force_kernel): same-spin ones for the density
+// spins apart (cp_sample_apply_kernel): same-spin ones for the density
 // decompositions, opposite-spin ones for the hopping decompositions.
 int theta_force_gemm(afqmc_engine *e, const zd *wf, const int *mask)
 {

@@ -1863,8 +1863,8 @@ void launch_taylor_accum(int W, long long wsize, const zd *term, zd *wfNew, cons
                                            acc, isLast, status);
 }
 
-// Gram-Schmidt with the columns in registers (mgs_col_kernel) where
-// ncol * TPC lanes fit one CTA of 512; false where the shape does not fit.
+// Gram-Schmidt by panels (mgs_block.cu) where its shared memory holds the walker,
+// else column by column.
 void launch_mgs(int W, int n, int ncol, int nup, int ndn, int isSD2is, zd *wf, zd *logw,
                 const int *alive, int *status, cudaStream_t s)
 {

@@ -164,11 +164,15 @@ class ClockSampler:
 
 
 # ------------------------------------------------------- algorithmic counts
-def phase_flops(c, m, taylor_avg):
+def phase_flops(c, m, taylor_avg, precision):
     """Algorithmic real FLOPs of one launch of each timed phase (complex MAC = 8,
     real x complex MAC = 4), for the phaseless workload."""
     n, nup, ndn, G, W = m.n, m.nup, m.ndn, m.G, c["W"]
-    K = (nup + ndn) * n
+    # equal spin blocks are computed once
+    once = nup == ndn and np.array_equal(m.phiTUp, m.phiTDn)
+    blocks = [nup] if once else [ns for ns in (nup, ndn) if ns]
+    K = sum(blocks) * n
+    pairs = sum(ns * ns for ns in blocks)
     # A_g = phiT^H L_g is real for a real trial (the Cholesky vectors are
     # real): the exchange product D = A_g theta is then real x complex
     real_a = not (np.any(np.asarray(m.phiTUp).imag) or np.any(np.asarray(m.phiTDn).imag))
@@ -177,16 +181,21 @@ def phase_flops(c, m, taylor_avg):
         "mbuild": 4.0 * n * n * G * W,
         "force": fa * G * K * W,
         "taylor": 8.0 * n * n * max(nup, ndn) * W * taylor_avg,
-        "exchange": fa * (nup * nup + ndn * ndn) * n * G * W + 8.0 * (nup * nup + ndn * ndn) * G * W,
-        "overlap": 8.0 * (nup * nup + ndn * ndn) * n * W,
+        "exchange": fa * pairs * n * G * W + 8.0 * pairs * G * W,
+        "overlap": 8.0 * pairs * n * W,
         "onebody": 8.0 * n * n * max(nup, ndn) * W,
     }
+    if precision != "mixed" and n <= 256:
+        # the series kernel ends with the one-body product; symmetric vectors
+        # give the two-body matrix as its lower triangle, in panels of 8 columns
+        f["taylor"] += f.pop("onebody")
+        f["mbuild"] *= (n + 8.0) / (2.0 * n)
     # with real A the exchange runs as three GEMMs per spin block of
-    # Kb = Ns n: Z = V U^T (2 Kb^2 2W), [M_re; M_im] = [Ar; Ai] Bt^T
-    # (2 2Kb Kb 2W) and Y = Rt X^T (2 2Kb G Kb); the flops counted are those
-    # executed, fewer than the blockwise tr(DD) count above
-    if real_a and n % 32 == 0 and W % 4 == 0 and all((ns * n) % 256 == 0 for ns in (nup, ndn) if ns):
-        f["exchange"] = sum((ns * n) ** 2 * (12.0 * W + 4.0 * G) for ns in (nup, ndn) if ns)
+    # Kb = Ns n, each half of a full one by symmetry: Z = V U^T (Kb^2 2W),
+    # [M_re; M_im] = [Ar; Ai] Bt^T (2Kb Kb 2W) and Y = Rt X^T (2Kb G Kb); the flops
+    # counted are those executed, fewer than the blockwise tr(DD) count above
+    if real_a and n % 32 == 0 and W % 4 == 0 and all((ns * n) % 256 == 0 for ns in blocks):
+        f["exchange"] = sum((ns * n) ** 2 * (6.0 * W + 2.0 * G) for ns in blocks)
     return f
 
 
@@ -213,10 +222,12 @@ def cp_phase_model(m, W, precision):
             "sample": ("bytes", W * 2 * walker),
             "onebody": ("bytes", W * 2 * walker),
         }
+    # real trial and one-body operator, spins apart: half the multiply-adds of
+    # half the entries; theta (complex) the blocks that the force reads
     return {
-        "overlap": ("flops", 8.0 * N * N * n * W),
-        "theta": ("flops", 8.0 * N * N * n * W),
-        "onebody": ("flops", 8.0 * n * n * N * W),
+        "overlap": ("flops", 2.0 * N * N * n * W),
+        "theta": ("flops", 4.0 * N * N * n * W),
+        "onebody": ("flops", 2.0 * n * n * N * W),
     }
 
 
@@ -747,7 +758,7 @@ def main():
     tavg = total / calls if calls else 0.0
     roof = None
     if c["kind"] == "pl":
-        fl = phase_flops(c, m, tavg)
+        fl = phase_flops(c, m, tavg, precision)
         cand = {k: v for k, v in prof.items() if k in fl and v[1] > 0}
         top = max(cand, key=lambda k: cand[k][0])
         t_launch = prof[top][0] / prof[top][1] / 1e3
@@ -814,7 +825,7 @@ def main():
         side = {"value": W * k64 * world / (ms64 / 1e3), "ms_per_step": ms64 / k64, "steps": k64,
                 "speedup_mixed_over_fp64": (ms64 / k64) / (ms / args.steps),
                 "algorithm": "same as the mixed form: closed-shell single spin block, exchange as "
-                             "GEMMs (FP64 CUDA-core GEMMs)"}
+                             "GEMMs (FP64 matrix-instruction GEMMs)"}
         # per-phase times of the FP64 form (direct launches, after the timed steps)
         f64.profile(True)
         run_steps(f64, k64, 2 + k64, args.measure_skip)
