@@ -3,10 +3,11 @@
 // 159-195), FP64, one kernel for the whole series and, where asked, the
 // one-body product that follows it.
 //
-// A CTA holds 16 columns of one walker and all n rows: the current term in
+// A CTA holds 16 columns (24 where that is all the walker has) of one walker
+// and all n rows: the current term in
 // shared memory (the right operand of the next order), the running sum in
 // the registers that also define the accumulator layout (a warp owns 16 rows
-// by 16 columns).  M is streamed through three or four cp.async stages of 8
+// and all columns).  M is streamed through three or four cp.async stages of 8
 // columns, once per order; the walkers in flight (148 SMs times n^2 16 bytes per
 // walker, 39 MB at n = 128) stay in L2, so memory sees M once.  The CTAs of one
 // walker form a cluster: the stopping test is the walker's largest term, so
@@ -39,7 +40,7 @@ extern std::atomic<long long> g_launch_count;
 
 namespace {
 
-constexpr int TF_COLS = 16;      // columns of phi per CTA
+constexpr int TF_COLS = 16;      // columns of phi per CTA (8 NJ, NJ = 2; 24 for a walker of 17..24)
 constexpr int TF_BK = 8;         // columns of M per stage
 constexpr int TF_MAXN = 256;     // 16 rows per warp, 16 warps
 constexpr int TF_MAXCL = 8;      // CTAs per walker (portable cluster size)
@@ -50,13 +51,14 @@ __host__ __device__ constexpr int tf_rows(int n) { return (n + 15) / 16 * 16; }
 __host__ __device__ constexpr int tf_lda(int n) { return tf_rows(n) + 2; }
 __host__ __device__ constexpr int tf_ldt(int n) { return tf_rows(n) + 4; }
 __host__ __device__ constexpr size_t tf_stage(int n) { return (size_t)TF_BK * tf_lda(n) * sizeof(zd); }
-__host__ __device__ constexpr size_t tf_smem(int n, int stages)
+__host__ __device__ constexpr size_t tf_smem(int n, int stages, int cols)
 {
-    return stages * tf_stage(n) + (size_t)TF_COLS * tf_ldt(n) * sizeof(zd);
+    return stages * tf_stage(n) + (size_t)cols * tf_ldt(n) * sizeof(zd);
 }
 
+template <int NJ>
 struct TfAcc {
-    double r[2][2][2], i[2][2][2];   // 8-row block, 8-column block, column parity
+    double r[2][NJ][2], i[2][NJ][2];   // 8-row block, 8-column block, column parity
 };
 
 // One n x n matrix times the term in shared memory, accumulated into c.  The
@@ -67,7 +69,7 @@ struct TfAcc {
 // triangle packed by columns; a tile's rows above the diagonal block come from
 // the mirrored entries, 8 neighbouring threads taking one row's 8 columns (128
 // contiguous bytes).
-template <bool REAL, bool PACKED, int STAGES>
+template <bool REAL, bool PACKED, int STAGES, int NJ>
 struct TfStream {
     const void *base;
     int n, npad, KT, it;
@@ -122,19 +124,19 @@ struct TfStream {
         cp_async_commit();
     }
     __device__ __forceinline__ void product(const unsigned char *smem, const zd *T, int ldt, int wr, int fr, int fk,
-                                            int nb, TfAcc &c)
+                                            int nb, TfAcc<NJ> &c)
     {
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int j = 0; j < 2; ++j) c.r[i][j][0] = c.r[i][j][1] = c.i[i][j][0] = c.i[i][j][1] = 0.0;
-        // both 8-column blocks (no branch between the products), or the first alone
-        if (nb == 2) stages<true>(smem, T, ldt, wr, fr, fk, nb, c);
+            for (int j = 0; j < NJ; ++j) c.r[i][j][0] = c.r[i][j][1] = c.i[i][j][0] = c.i[i][j][1] = 0.0;
+        // all 8-column blocks (no branch between the products), or the first ones
+        if (nb == NJ) stages<true>(smem, T, ldt, wr, fr, fk, nb, c);
         else stages<false>(smem, T, ldt, wr, fr, fk, nb, c);
     }
     template <bool FULL>
     __device__ __forceinline__ void stages(const unsigned char *smem, const zd *T, int ldt, int wr, int fr, int fk,
-                                           int nb, TfAcc &c)
+                                           int nb, TfAcc<NJ> &c)
     {
         for (int kt = 0; kt < KT; ++kt, ++it) {
             cp_async_wait<STAGES - 2>();
@@ -154,7 +156,7 @@ struct TfStream {
                     }
                 }
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
+                for (int j = 0; j < NJ; ++j) {
                     if (!FULL && j >= nb) continue;
                     const zd b = T[(size_t)(8 * j + fr) * ldt + kt * TF_BK + k4 + fk];
 #pragma unroll
@@ -172,16 +174,17 @@ struct TfStream {
     }
 };
 
-template <bool PACKED, int MAXT, int MINB, int STAGES>
+template <bool PACKED, int MAXT, int MINB, int STAGES, int NJ>
 __global__ void __launch_bounds__(MAXT, MINB)
 taylor_f64_kernel(TaylorF64 a)
 {
+    constexpr int COLS = 8 * NJ;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ double wmax[16], cmax[2][TF_MAXCL];
     const int n = a.n, N = a.N;
-    const int cs = (N + TF_COLS - 1) / TF_COLS, w = blockIdx.x / cs, rank = blockIdx.x % cs;
+    const int cs = (N + COLS - 1) / COLS, w = blockIdx.x / cs, rank = blockIdx.x % cs;
     if (a.mask && !a.mask[w]) return;   // the whole cluster
-    const int col0 = rank * TF_COLS, ncols = min(TF_COLS, N - col0), nb = (ncols + 7) / 8;
+    const int col0 = rank * COLS, ncols = min(COLS, N - col0), nb = (ncols + 7) / 8;
     const int ldt = tf_ldt(n);
     const size_t stage = tf_stage(n);
     zd *T = (zd *)(smem + STAGES * stage);
@@ -189,19 +192,19 @@ taylor_f64_kernel(TaylorF64 a)
     const int tid = threadIdx.x, NT = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const int wr = warp * 16, fr = lane >> 2, fk = lane & 3;
 
-    TfStream<false, PACKED, STAGES> ms;
+    TfStream<false, PACKED, STAGES, NJ> ms;
     ms.start(a.M + (size_t)w * a.Mstride, n, st0, stage);
     const zd *src = a.src + ((size_t)w * N + col0) * n;
-    for (int e = tid; e < TF_COLS * tf_rows(n); e += NT) {
+    for (int e = tid; e < COLS * tf_rows(n); e += NT) {
         const int r = e % tf_rows(n), c = e / tf_rows(n);
         T[(size_t)c * ldt + r] = (r < n && c < ncols) ? src[(size_t)c * n + r] : make_double2(0.0, 0.0);
     }
     __syncthreads();
-    TfAcc sum, c;
+    TfAcc<NJ> sum, c;
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+        for (int j = 0; j < NJ; ++j)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const zd v = T[(size_t)(8 * j + 2 * fk + h) * ldt + wr + 8 * i + fr];
@@ -218,7 +221,7 @@ taylor_f64_kernel(TaylorF64 a)
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
+            for (int j = 0; j < NJ; ++j)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const double x = c.r[i][j][h] * inv, y = c.i[i][j][h] * inv;
@@ -257,24 +260,24 @@ taylor_f64_kernel(TaylorF64 a)
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
+            for (int j = 0; j < NJ; ++j)
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
                     T[(size_t)(8 * j + 2 * fk + h) * ldt + wr + 8 * i + fr] =
                         make_double2(sum.r[i][j][h], sum.i[i][j][h]);
         if (a.postR) {
-            TfStream<true, false, STAGES> ps;
+            TfStream<true, false, STAGES, NJ> ps;
             ps.start(a.postR, n, st0, stage);
             ps.product(smem, T, ldt, wr, fr, fk, nb, sum);
         } else {
-            TfStream<false, false, STAGES> ps;
+            TfStream<false, false, STAGES, NJ> ps;
             ps.start(a.postZ, n, st0, stage);
             ps.product(smem, T, ldt, wr, fr, fk, nb, sum);
         }
     }
     zd *dst = a.dst + ((size_t)w * N + col0) * n;
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
+    for (int j = 0; j < NJ; ++j)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int cc = 8 * j + 2 * fk + h;
@@ -291,21 +294,21 @@ taylor_f64_kernel(TaylorF64 a)
 
 bool taylor_f64_supported(int n, int N) { return n <= TF_MAXN && N <= TF_COLS * TF_MAXCL; }
 
-template <bool PACKED, int MAXT, int MINB, int STAGES>
+template <bool PACKED, int MAXT, int MINB, int STAGES, int NJ = 2>
 static cudaError_t launch(const TaylorF64 &a, cudaStream_t s)
 {
-    const auto kernel = taylor_f64_kernel<PACKED, MAXT, MINB, STAGES>;
+    const auto kernel = taylor_f64_kernel<PACKED, MAXT, MINB, STAGES, NJ>;
     static std::atomic<unsigned long long> attr{0};
     cudaError_t r = each_device_once(attr, [] {
-        return cudaFuncSetAttribute(taylor_f64_kernel<PACKED, MAXT, MINB, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)tf_smem(MAXT / 2, STAGES));
+        return cudaFuncSetAttribute(taylor_f64_kernel<PACKED, MAXT, MINB, STAGES, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)tf_smem(MAXT / 2, STAGES, 8 * NJ));
     });
     if (r != cudaSuccess) return r;
-    const int cs = (a.N + TF_COLS - 1) / TF_COLS;
+    const int cs = (a.N + 8 * NJ - 1) / (8 * NJ);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)cs * (unsigned)a.W);
     cfg.blockDim = dim3((unsigned)(2 * tf_rows(a.n)));
-    cfg.dynamicSmemBytes = tf_smem(a.n, STAGES);
+    cfg.dynamicSmemBytes = tf_smem(a.n, STAGES, 8 * NJ);
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -318,7 +321,15 @@ static cudaError_t launch(const TaylorF64 &a, cudaStream_t s)
     return r != cudaSuccess ? r : cudaGetLastError();
 }
 
-// 128 registers a thread, four stages.  192 threads (n = 81..96) take 96
+// A walker of 17 to 24 columns, n <= 96: one CTA of 24 columns (168 registers)
+// instead of a cluster of 16 and 8, which streams M twice and meets at each order
+// (n, N, walkers: 96, 20, 2048 1297 -> 963 us; 64, 24, 2048 579 -> 420; 90, 21, 300
+// 277 -> 253; 32, 20, 1000 117 -> 102; 48, 24, 100 57 -> 51).  Small matrices of
+// no more walkers than SMs stay on two SMs each (40, 18, 64: 40 us against 45; 32, 20,
+// 148: 38 and 40), and wider walkers on 16 columns a CTA: 24 gain where waves are
+// full (96, 48, 1000 1036 -> 978) and lose where they are not (90, 45, 300 355 -> 368).
+//
+// Otherwise 128 registers a thread, four stages.  192 threads (n = 81..96) take 96
 // registers so that three CTAs are resident instead of two, 288 (n = 129..144) two
 // instead of one: n = 90, N = 21, 300 walkers 303 -> 277 us; n = 64 and 128, whose
 // number of CTAs stays the same, 98 us either way and 2.47 against 2.49 ms.  Above
@@ -328,6 +339,8 @@ cudaError_t taylor_f64(const TaylorF64 &a, cudaStream_t s)
 {
     g_launch_count++;
     const int nt = 2 * tf_rows(a.n);
+    if (nt <= 192 && a.N > 16 && a.N <= 24 && (a.n > 40 || a.W > 148))
+        return a.packed ? launch<true, 192, 2, 4, 3>(a, s) : launch<false, 192, 2, 4, 3>(a, s);
     if (nt == 192 || nt == 288) return a.packed ? launch<true, 288, 2, 4>(a, s) : launch<false, 288, 2, 4>(a, s);
     if (nt <= 256) return a.packed ? launch<true, 256, 2, 4>(a, s) : launch<false, 256, 2, 4>(a, s);
     return a.packed ? launch<true, 512, 1, 3>(a, s) : launch<false, 512, 1, 3>(a, s);
