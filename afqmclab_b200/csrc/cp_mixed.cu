@@ -755,10 +755,10 @@ int cp_mixed_create(afqmc_engine *e)
     if (!cp_mixed_supported(e->L, e->ncol, &why)) return engine_fail(AFQMC_ERR_UNSUPPORTED, why);
     const int n = e->n, N = e->ncol, W = e->W;
     std::vector<zd> E((size_t)n * n), T((size_t)n * N), H((size_t)n * n);
-    if (cudaMemcpy(E.data(), e->expK[0], sizeof(zd) * E.size(), cudaMemcpyDeviceToHost) != cudaSuccess ||
-        cudaMemcpy(H.data(), e->expK[1], sizeof(zd) * H.size(), cudaMemcpyDeviceToHost) != cudaSuccess ||
-        cudaMemcpy(T.data(), e->phiT[0], sizeof(zd) * T.size(), cudaMemcpyDeviceToHost) != cudaSuccess)
-        return engine_fail(AFQMC_ERR_CUDA, "reading operators for the mixed form");
+#define CM(x) do { int r_ = (x); if (r_ != AFQMC_OK) return r_; } while (0)
+    CM(engine_read(e, E.data(), e->expK[0], sizeof(zd) * E.size()));
+    CM(engine_read(e, H.data(), e->expK[1], sizeof(zd) * H.size()));
+    CM(engine_read(e, T.data(), e->phiT[0], sizeof(zd) * T.size()));
     for (const zd &v : E)
         if (v.y != 0.0) return engine_fail(AFQMC_ERR_UNSUPPORTED, "mixed constrained-path form needs a real exp(-dt K)");
     CpMixedState *m = new CpMixedState();
@@ -768,7 +768,6 @@ int cp_mixed_create(afqmc_engine *e)
     m->bnw = (N + 15) / 16 * 16;
     m->wptO = std::max(1, BN / m->bnw);
     m->wptG = std::max(1, BN / (2 * N));
-#define CM(x) do { int r_ = (x); if (r_ != AFQMC_OK) return r_; } while (0)
     CM(engine_dalloc(e, &m->hi, (size_t)W * m->ws));
     CM(engine_dalloc(e, &m->lo, (size_t)W * m->ws));
     CM(engine_dalloc(e, &m->thi, (size_t)W * m->ws));
@@ -814,19 +813,14 @@ int cp_mixed_create(afqmc_engine *e)
                 split_host(H[i + (size_t)n * k].x - (i == k ? 1.0 : 0.0), hh[(size_t)i * n + k], hl[(size_t)i * n + k]);
         CM(engine_dalloc(e, &m->Hhi, (size_t)n * n));
         CM(engine_dalloc(e, &m->Hlo, (size_t)n * n));
-        if (cudaMemcpy(m->Hhi, hh.data(), 4 * hh.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(m->Hlo, hl.data(), 4 * hl.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-            return engine_fail(AFQMC_ERR_CUDA, "uploading the mixed-form half-step operator");
+        CM(engine_write(e, m->Hhi, hh.data(), 4 * hh.size()));
+        CM(engine_write(e, m->Hlo, hl.data(), 4 * hl.size()));
     }
-    if (cudaMemcpy(m->Ehi, eh.data(), 4 * eh.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(m->Elo, el.data(), 4 * el.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(m->Ohi, oh.data(), 4 * oh.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(m->Olo, ol.data(), 4 * ol.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(m->Ag, ag.data(), 4 * ag.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-        return engine_fail(AFQMC_ERR_CUDA, "uploading mixed-form operators");
-    if (cudaMemset(m->Bg, 0, sizeof(float) * (size_t)W * 2 * N * m->K2) != cudaSuccess ||
-        cudaMemset(m->err, 0, sizeof(int)) != cudaSuccess)
-        return engine_fail(AFQMC_ERR_CUDA, "clearing mixed-form buffers");
+    CM(engine_write(e, m->Ehi, eh.data(), 4 * eh.size()));
+    CM(engine_write(e, m->Elo, el.data(), 4 * el.size()));
+    CM(engine_write(e, m->Ohi, oh.data(), 4 * oh.size()));
+    CM(engine_write(e, m->Olo, ol.data(), 4 * ol.size()));
+    CM(engine_write(e, m->Ag, ag.data(), 4 * ag.size()));
     return AFQMC_OK;
 }
 
@@ -879,7 +873,7 @@ int cp_mixed_measure_prep(afqmc_engine *e, bool *done)
 int cp_mixed_status(afqmc_engine *e)
 {
     int h = 0;
-    cudaMemcpy(&h, e->cpm->err, sizeof(int), cudaMemcpyDeviceToHost);
+    if (engine_read(e, &h, e->cpm->err, sizeof(int)) != AFQMC_OK) return 32;
     return h ? 32 : 0;
 }
 

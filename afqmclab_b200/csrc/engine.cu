@@ -140,6 +140,9 @@ struct BPState {
 
 namespace {
 
+// Zeroed device memory.  Everything that sets an engine's memory up runs on
+// the engine's stream: it does not wait for the legacy default stream, so a
+// fill or a copy issued there could land after the kernel that follows it here.
 template <class T>
 int dalloc(afqmc_engine *e, T **p, size_t count)
 {
@@ -148,8 +151,11 @@ int dalloc(afqmc_engine *e, T **p, size_t count)
     cudaError_t r = cudaMalloc(&q, count * sizeof(T));
     if (r != cudaSuccess)
         return fail(AFQMC_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(r));
-    r = cudaMemset(q, 0, count * sizeof(T));
-    if (r != cudaSuccess) return fail(AFQMC_ERR_CUDA, cudaGetErrorString(r));
+    r = cudaMemsetAsync(q, 0, count * sizeof(T), e->stream);
+    if (r != cudaSuccess) {
+        cudaFree(q);
+        return fail(AFQMC_ERR_CUDA, cudaGetErrorString(r));
+    }
     e->allocs.push_back(q);
     *p = (T *)q;
     return AFQMC_OK;
@@ -159,7 +165,7 @@ template <class T>
 int dupload(afqmc_engine *e, T **p, const void *host, size_t count)
 {
     TRY(dalloc(e, p, count));
-    if (host) CUDA_TRY(cudaMemcpy(*p, host, count * sizeof(T), cudaMemcpyHostToDevice));
+    if (host) CUDA_TRY(cudaMemcpyAsync(*p, host, count * sizeof(T), cudaMemcpyHostToDevice, e->stream));
     return AFQMC_OK;
 }
 
@@ -181,6 +187,8 @@ int gemm(const ZGemmArgs &a, cudaStream_t s)
 int alloc_population(afqmc_engine *e)
 {
     const int W = e->W;
+    CUDA_TRY(cudaStreamCreateWithFlags(&e->own, cudaStreamNonBlocking));
+    e->stream = e->own;
     e->wsize = (long long)e->n * e->ncol;
     TRY(dalloc(e, &e->wf, (size_t)W * e->wsize));
     TRY(dalloc(e, &e->wfTmp, (size_t)W * e->wsize));
@@ -207,13 +215,11 @@ int alloc_population(afqmc_engine *e)
     TRY(dalloc(e, &e->weight, W));
     TRY(dalloc(e, &e->tstats, 4));
     long long init[4] = {0, 0, 1LL << 40, 0};
-    CUDA_TRY(cudaMemcpy(e->tstats, init, sizeof(init), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpyAsync(e->tstats, init, sizeof(init), cudaMemcpyHostToDevice, e->stream));
     TRY(dalloc(e, &e->acc, 8));
     TRY(dalloc(e, &e->eloc, W));
     TRY(dalloc(e, &e->den, W));
     TRY(dalloc(e, &e->parts, (size_t)3 * W));
-    CUDA_TRY(cudaStreamCreateWithFlags(&e->own, cudaStreamNonBlocking));
-    e->stream = e->own;
     return AFQMC_OK;
 }
 
@@ -926,8 +932,8 @@ int fp64_exchange_setup(afqmc_engine *e)
     if (e->bl.nblk == 2 && e->nup == e->ndn && e->nup > 0) {
         const size_t cnt = (size_t)e->n * e->nup;
         std::vector<zd> t0(cnt), t1(cnt);
-        CUDA_TRY(cudaMemcpy(t0.data(), e->phiT[0], sizeof(zd) * cnt, cudaMemcpyDeviceToHost));
-        CUDA_TRY(cudaMemcpy(t1.data(), e->phiT[1], sizeof(zd) * cnt, cudaMemcpyDeviceToHost));
+        TRY(engine_read(e, t0.data(), e->phiT[0], sizeof(zd) * cnt));
+        TRY(engine_read(e, t1.data(), e->phiT[1], sizeof(zd) * cnt));
         if (std::memcmp(t0.data(), t1.data(), sizeof(zd) * cnt) == 0) {
             x.restricted = true;
             x.bl1 = e->bl;
@@ -949,6 +955,18 @@ int fp64_exchange_setup(afqmc_engine *e)
 int engine_fail(int code, const std::string &msg) { return fail(code, msg); }
 int engine_check_launch() { return check_launch(); }
 int engine_gemm(const ZGemmArgs &a, cudaStream_t s) { return gemm(a, s); }
+int engine_read(afqmc_engine *e, void *host, const void *dev, size_t bytes)
+{
+    CUDA_TRY(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, e->stream));
+    CUDA_TRY(cudaStreamSynchronize(e->stream));
+    return AFQMC_OK;
+}
+int engine_write(afqmc_engine *e, void *dev, const void *host, size_t bytes)
+{
+    CUDA_TRY(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, e->stream));
+    CUDA_TRY(cudaStreamSynchronize(e->stream));
+    return AFQMC_OK;
+}
 template <class T> int engine_dalloc(afqmc_engine *e, T **p, size_t count) { return dalloc(e, p, count); }
 template int engine_dalloc<float>(afqmc_engine *, float **, size_t);
 template int engine_dalloc<int>(afqmc_engine *, int **, size_t);
@@ -1202,6 +1220,13 @@ int afqmc_set_walkers(afqmc_engine *e, const double *wf, const double *logw, con
 
 namespace {
 
+// The copy stream takes the staging slots after they are cleared (dalloc).
+int upload_slots_cleared(afqmc_engine *e)
+{
+    for (int k = 0; k < 2; ++k) CUDA_TRY(cudaEventRecord(e->upFree[k], e->stream));
+    return AFQMC_OK;
+}
+
 // the copy stream, its events and the log-weight / alive staging slots,
 // made by the first asynchronous upload
 int upload_init(afqmc_engine *e)
@@ -1211,11 +1236,10 @@ int upload_init(afqmc_engine *e)
     for (int k = 0; k < 2; ++k) {
         CUDA_TRY(cudaEventCreateWithFlags(&e->upReady[k], cudaEventDisableTiming));
         CUDA_TRY(cudaEventCreateWithFlags(&e->upFree[k], cudaEventDisableTiming));
-        CUDA_TRY(cudaEventRecord(e->upFree[k], e->stream));
         TRY(dalloc(e, &e->stgLw[k], (size_t)e->W));
         TRY(dalloc(e, &e->stgAl[k], (size_t)e->W));
     }
-    return AFQMC_OK;
+    return upload_slots_cleared(e);
 }
 
 }  // namespace
@@ -1224,8 +1248,10 @@ int afqmc_set_walkers_async(afqmc_engine *e, const double *wf, const double *log
 {
     if (!e || !wf || !logw || !alive) return fail(AFQMC_ERR_ARG, "null argument");
     TRY(upload_init(e));
-    if (!e->stgWf[0])
+    if (!e->stgWf[0]) {
         for (int k = 0; k < 2; ++k) TRY(dalloc(e, &e->stgWf[k], (size_t)e->wsize * e->W));
+        TRY(upload_slots_cleared(e));
+    }
     const int k = e->upNext;
     e->upNext ^= 1;
     // the slot's previous contents must have been installed first
@@ -1256,8 +1282,10 @@ int afqmc_set_walkers_f32_async(afqmc_engine *e, const float *wf32, const double
         return fail(AFQMC_ERR_UNSUPPORTED, "fp32 walker upload is for the phaseless mixed form");
     TRY(upload_init(e));
     const size_t count = (size_t)2 * e->wsize * e->W;   // [re | im] planes per walker
-    if (!e->stgWf32[0])
+    if (!e->stgWf32[0]) {
         for (int k = 0; k < 2; ++k) TRY(dalloc(e, &e->stgWf32[k], count));
+        TRY(upload_slots_cleared(e));
+    }
     const int k = e->upNext;
     e->upNext ^= 1;
     CUDA_TRY(cudaStreamWaitEvent(e->upStream, e->upFree[k], 0));

@@ -161,6 +161,9 @@ inline void prof_resolve(afqmc_engine *e)
 int engine_fail(int code, const std::string &msg);
 int engine_check_launch();
 int engine_gemm(const ZGemmArgs &a, cudaStream_t s);
+// Blocking copies in the engine's stream order.
+int engine_read(afqmc_engine *e, void *host, const void *dev, size_t bytes);
+int engine_write(afqmc_engine *e, void *dev, const void *host, size_t bytes);
 template <class T> int engine_dalloc(afqmc_engine *e, T **p, size_t count);
 // The walkers' places in the random stream for a sampling kernel of one CTA per
 // walker (launches the scan where the kernel does not count by itself).

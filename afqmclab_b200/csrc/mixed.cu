@@ -1228,10 +1228,8 @@ int mixed_create(afqmc_engine *e)
             // spin-restricted when both blocks carry the same trial bit for bit
             if (e->bl.nblk == 2 && e->nup == e->ndn && e->nup > 0) {
                 std::vector<zd> t0((size_t)n * e->nup), t1((size_t)n * e->ndn);
-                MTRY(cuda_check(cudaMemcpy(t0.data(), e->phiT[0], sizeof(zd) * t0.size(), cudaMemcpyDeviceToHost),
-                                "copy"));
-                MTRY(cuda_check(cudaMemcpy(t1.data(), e->phiT[1], sizeof(zd) * t1.size(), cudaMemcpyDeviceToHost),
-                                "copy"));
+                MTRY(engine_read(e, t0.data(), e->phiT[0], sizeof(zd) * t0.size()));
+                MTRY(engine_read(e, t1.data(), e->phiT[1], sizeof(zd) * t1.size()));
                 if (std::memcmp(t0.data(), t1.data(), sizeof(zd) * t0.size()) == 0) {
                     m->restricted = true;
                     m->bl1 = e->bl;
@@ -1261,14 +1259,14 @@ int mixed_create(afqmc_engine *e)
     // exp(+dt/2 K) of the measurement's half step on the tensor cores
     {
         std::vector<zd> E1((size_t)n * n);
-        MTRY(cuda_check(cudaMemcpy(E1.data(), e->expK[1], sizeof(zd) * E1.size(), cudaMemcpyDeviceToHost), "copy"));
+        MTRY(engine_read(e, E1.data(), e->expK[1], sizeof(zd) * E1.size()));
         std::vector<float> eh, el;
         if (tf32_split_operator(E1.data(), n, eh, el))
             return engine_fail(AFQMC_ERR_UNSUPPORTED, "mixed precision one-body needs a real exp(dt/2 K)");
         MTRY(engine_dalloc(e, &m->E1h, eh.size()));
         MTRY(engine_dalloc(e, &m->E1l, el.size()));
-        MTRY(cuda_check(cudaMemcpy(m->E1h, eh.data(), 4 * eh.size(), cudaMemcpyHostToDevice), "upload"));
-        MTRY(cuda_check(cudaMemcpy(m->E1l, el.data(), 4 * el.size(), cudaMemcpyHostToDevice), "upload"));
+        MTRY(engine_write(e, m->E1h, eh.data(), 4 * eh.size()));
+        MTRY(engine_write(e, m->E1l, el.data(), 4 * el.size()));
         MTRY(engine_dalloc(e, &m->sh, (size_t)W * m->ws32));
         MTRY(engine_dalloc(e, &m->sl, (size_t)W * m->ws32));
     }
@@ -1287,8 +1285,7 @@ int mixed_create(afqmc_engine *e)
             if (bl.Ns[b] == 0) continue;
             Ns[nb] = bl.Ns[b];
             T[nb].resize((size_t)n * Ns[nb]);
-            MTRY(cuda_check(cudaMemcpy(T[nb].data(), e->phiT[b], sizeof(zd) * T[nb].size(), cudaMemcpyDeviceToHost),
-                            "copy"));
+            MTRY(engine_read(e, T[nb].data(), e->phiT[b], sizeof(zd) * T[nb].size()));
             Tp[nb] = T[nb].data();
             ++nb;
         }
@@ -1304,8 +1301,8 @@ int mixed_create(afqmc_engine *e)
             overlap_tc_build(nbo, Tp + o, n, Ns + o, oh, ol);
             MTRY(engine_dalloc(e, &m->Ohi[o], oh.size()));
             MTRY(engine_dalloc(e, &m->Olo[o], ol.size()));
-            MTRY(cuda_check(cudaMemcpy(m->Ohi[o], oh.data(), 4 * oh.size(), cudaMemcpyHostToDevice), "upload"));
-            MTRY(cuda_check(cudaMemcpy(m->Olo[o], ol.data(), 4 * ol.size(), cudaMemcpyHostToDevice), "upload"));
+            MTRY(engine_write(e, m->Ohi[o], oh.data(), 4 * oh.size()));
+            MTRY(engine_write(e, m->Olo[o], ol.data(), 4 * ol.size()));
         }
     }
     m->ready = true;
@@ -1367,7 +1364,7 @@ int mixed_status(afqmc_engine *e)
 {
     if (e->kind == KIND_CP) return cp_mixed_status(e);
     int h = 0;
-    cudaMemcpy(&h, e->mx->err, sizeof(int), cudaMemcpyDeviceToHost);
+    if (engine_read(e, &h, e->mx->err, sizeof(int)) != AFQMC_OK) return 32;
     return h ? 32 : 0;
 }
 
