@@ -174,6 +174,9 @@ struct TfStream {
     }
 };
 
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory"); }
+
 template <bool PACKED, int MAXT, int MINB, int STAGES, int NJ>
 __global__ void __launch_bounds__(MAXT, MINB)
 taylor_f64_kernel(TaylorF64 a)
@@ -184,6 +187,10 @@ taylor_f64_kernel(TaylorF64 a)
     const int n = a.n, N = a.N;
     const int cs = (N + COLS - 1) / COLS, w = blockIdx.x / cs, rank = blockIdx.x % cs;
     if (a.mask && !a.mask[w]) return;   // the whole cluster
+    // the peers' shared memory may be written to once all of them have started:
+    // said here, waited for before the first store, which is orders away
+    if (cs > 1) cluster_arrive();
+    const int kFirst = max(1, a.checkFrom);
     const int col0 = rank * COLS, ncols = min(COLS, N - col0), nb = (ncols + 7) / 8;
     const int ldt = tf_ldt(n);
     const size_t stage = tf_stage(n);
@@ -241,6 +248,7 @@ taylor_f64_kernel(TaylorF64 a)
         for (int q = 0; q < NT / 32; ++q) all = fmax(all, wmax[q]);
         if (cs > 1) {
             cg::cluster_group cl = cg::this_cluster();
+            if (k == kFirst) cluster_wait();
             if (tid < cs) cl.map_shared_rank(&cmax[k & 1][0], tid)[rank] = all;
             cl.sync();
             for (int q = 0; q < cs; ++q) all = fmax(all, cmax[k & 1][q]);
