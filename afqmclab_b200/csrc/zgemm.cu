@@ -115,13 +115,16 @@ zgemm_kernel(ZGemmArgs a)
     typedef GemmShape<TL, OPA, OPB, REAL> SH;
     typedef typename SH::LA LA;
     typedef typename SH::LB LB;
-    const int b = blockIdx.z / a.parts;
-    const bool second = blockIdx.z % a.parts != 0;
+    // the second part's tiles follow the first one's in x: z, the batch, is limited
+    // to 65535
+    const int b = blockIdx.z, tilesM = a.parts > 1 ? gridDim.x >> 1 : gridDim.x;
+    const bool second = blockIdx.x >= tilesM;
+    const int bx = second ? blockIdx.x - tilesM : blockIdx.x;
     if (a.mask && a.mask[b] == 0) return;
     if (a.skip && a.skip[b] != 0) return;
     const int m = second ? a.m1 : a.m, n = second ? a.n1 : a.n;
     // a quadratic form's rows get longer downwards: the longest start first
-    const int tileM = (a.quad ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * BM, tileN = blockIdx.y * BN;
+    const int tileM = (a.quad ? tilesM - 1 - bx : bx) * BM, tileN = blockIdx.y * BN;
     if (tileM >= m || tileN >= n) return;
     if (a.lower && tileM + BM <= tileN) return;
     int k = second ? a.k1 : a.k;
@@ -271,7 +274,7 @@ cudaError_t launch3(const ZGemmArgs &a, cudaStream_t s)
 {
     typedef GemmShape<TL, OPA, OPB, REAL> SH;
     const int m = a.parts > 1 ? std::max(a.m, a.m1) : a.m, n = a.parts > 1 ? std::max(a.n, a.n1) : a.n;
-    dim3 grid((m + TL::BM - 1) / TL::BM, (n + TL::BN - 1) / TL::BN, a.batch * a.parts);
+    dim3 grid((m + TL::BM - 1) / TL::BM * a.parts, (n + TL::BN - 1) / TL::BN, a.batch);
     static std::atomic<unsigned long long> attr{0};
     const cudaError_t r = each_device_once(attr, [] {
         return cudaFuncSetAttribute(zgemm_kernel<TL, OPA, OPB, REAL, SCALE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
