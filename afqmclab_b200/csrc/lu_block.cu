@@ -6,9 +6,8 @@
 // row i, a CTA up to 8 block columns (64 columns; blocks of 65 to 128 columns
 // are split over a cluster of two CTAs).  Panel p is block column p.  Its
 // eight elimination steps run on the panel alone, one row per lane, with
-// zgetf2's pivot rule (first position of the largest |re| + |im|, to 15 bits;
-// rows stay where they are and carry their position in the interchanged
-// matrix).  The
+// zgetf2's pivot rule (first position of the largest |re| + |im|; rows stay
+// where they are and carry their position in the interchanged matrix).  The
 // panel's own in-place result G then updates every other block column at once:
 // with B the eight pivot rows before the update,
 //     A <- A with the pivot rows zeroed + G B        (rank 8, matrix products)
@@ -23,11 +22,13 @@
 // the kernel; the products themselves take a third of that.  Hence one warp
 // reduction per search (lb_rank) and the hardware's reciprocal start (lb_rcp);
 // with the compute warps as panel warps the registers spilled and a step took
-// 1200.
+// 1200.  Rows that tie in the rank are told apart by all 64 bits: at once where one
+// warp holds the rows, else by one more pass over the panel (lb_again); the test
+// costs nothing up to 64 columns and 3 to 4 % on 80 and 120.
 //
 // Against the element-wise kernels it replaces (us per launch, one B200): 14
 // columns, 100 matrices 35 -> 17; 16 columns, 512 matrices 31 -> 17; 56, 1024: 203
-// -> 181; 64, 512: 131 -> 109; 80, 1024: 1459 -> 796; 120, 1024: 2867 -> 1413.
+// -> 183; 64, 512: 131 -> 109; 80, 1024: 1459 -> 822; 120, 1024: 2867 -> 1464.
 #include <cooperative_groups.h>
 
 #include <atomic>
@@ -63,6 +64,126 @@ struct LbShared {
 
 __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+// Whether any of the barrier's threads votes for it.
+__device__ __forceinline__ bool bar_any(int id, int threads, bool vote)
+{
+    int r;
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.s32 p, %3, 0;\nbar.red.or.pred q, %1, %2, p;\nselp.s32 %0, 1, 0, q;\n}\n"
+                 : "=r"(r)
+                 : "r"(id), "r"(threads), "r"((int)vote)
+                 : "memory");
+    return r != 0;
+}
+
+// The steps of panel p on the panel warps' rows a (row prow at position pos; the
+// step that takes it as pivot in myslot).  The row rotates by one register per
+// step, so that the current column is always a[0] and the step is one loop body
+// with static register indices.  One warp (NCB = 4) chooses by rank and by all bits in the same
+// step.  Several choose by rank; tied: a row ties with a chosen one, and the
+// panel has to be done again by all bits (EXACT).
+template <bool EXACT, int C, int NCB>
+__device__ __forceinline__ void lb_steps(LbShared<C, NCB> &sh, LbShared<C, NCB> *peer, int p, int Ns, int pw, int prow,
+                                         zd (&a)[8], int &pos, int &myslot, bool &tied)
+{
+    const int pwarp = prow >> 5, lane = prow & 31, steps = min(8, Ns - 8 * p);
+#pragma unroll 1
+    for (int c = 0; c < steps; ++c) {
+        const int k = 8 * p + c;
+        const unsigned u = lb_rank(a[0], pos, prow < Ns && pos >= k);
+        unsigned best = __reduce_max_sync(0xffffffffu, u);
+        if constexpr (EXACT) {
+            best = lb_exact(a[0], u, best);
+        } else if constexpr (NCB == 4) {
+            if (__any_sync(0xffffffffu, lb_rival(u, best))) best = lb_exact(a[0], u, best);
+        }
+        double d;
+        const zd qr = lb_rcp(a[0], d);
+        zd *cw = sh.crow[c & 1][pwarp];
+        if (u == best && u != 0) {
+            cw[0] = (d > 1e-280 && d < 1e280) ? qr : lb_rcp_any(a[0]);
+#pragma unroll
+            for (int j = 1; j < 8; ++j) cw[j] = a[j];
+            cw[8] = a[0];
+        }
+        const zd *pr = sh.crow[c & 1][0];
+        if (pw > 1) {
+            if (lane == 0) ((unsigned *)&sh.rank[c & 1])[pwarp] = best;
+            bar_sync(1, 32 * pw);
+            const int4 v = sh.rank[c & 1];
+            const unsigned t[4] = {(unsigned)v.x, (unsigned)v.y, pw > 2 ? (unsigned)v.z : 0u,
+                                   pw > 3 ? (unsigned)v.w : 0u};
+            int bw = 0;
+            best = t[0];
+#pragma unroll
+            for (int q = 1; q < 2 * C; ++q)
+                if (t[q] > best) { best = t[q]; bw = q; }
+            if constexpr (EXACT) {   // the warps' candidates by all bits, then the lower position
+                const unsigned top = best;
+                unsigned long long v = lb_bits(sh.crow[c & 1][bw][8]);
+#pragma unroll
+                for (int q = 0; q < 2 * C; ++q) {
+                    if (!lb_tied(t[q], top)) continue;
+                    const unsigned long long vq = lb_bits(sh.crow[c & 1][q][8]);
+                    if (vq > v || (vq == v && t[q] > best)) { v = vq; best = t[q]; bw = q; }
+                }
+            }
+            pr = sh.crow[c & 1][bw];
+        } else {
+            __syncwarp();
+        }
+        if constexpr (!EXACT && NCB == 8) tied = tied || lb_rival(u, best);
+        const int key = 127 - (int)(best & 127u);   // the pivot's position
+        const zd q = pr[0];
+        if (pwarp == 0 && lane == 0) {
+            const zd a0 = pr[8];
+            sh.piv[k] = a0;
+            sh.pv[k] = key;
+        }
+        const bool isP = pos == key;
+        if (pos == k) pos = key;
+        if (isP) {
+            pos = k;
+            myslot = c;
+            sh.rowOf[k] = prow;
+            if constexpr (C > 1) peer->rowOf[k] = prow;
+        }
+        // the pivot row becomes q times itself, the others lose f times it
+        const zd f = isP ? zneg(q) : zmul(a[0], q);
+#pragma unroll
+        for (int j = 1; j < 8; ++j) {
+            const zd pj = pr[j];
+            const zd base = isP ? make_double2(0.0, 0.0) : a[j];
+            a[j - 1].x = fma(-f.x, pj.x, fma(f.y, pj.y, base.x));
+            a[j - 1].y = fma(-f.x, pj.y, fma(-f.y, pj.x, base.y));
+        }
+        a[7] = zneg(f);
+    }
+}
+
+struct LbRow {
+    zd a[8];
+    int pos, slot;
+};
+
+// Panel p once more from its columns, the pivots chosen by all bits: about one
+// panel in 700 of random 56 x 56 matrices, and matrices with equal entries.  Out
+// of line: inside the loop above it cost 8 % without ever running.
+template <int C, int NCB>
+__device__ __noinline__ LbRow lb_again(LbShared<C, NCB> &sh, LbShared<C, NCB> *peer, int p, int Ns, int pw, int prow, int pos)
+{
+    LbRow row;
+    row.pos = pos;
+    row.slot = -1;
+    bool tied;
+    zd a[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) a[c] = prow < Ns ? sh.G[p & 1][c][prow] : make_double2(0.0, 0.0);
+    lb_steps<true>(sh, peer, p, Ns, pw, prow, a, row.pos, row.slot, tied);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) row.a[c] = a[c];
+    return row;
+}
 
 // NBK: spin blocks per walker.
 template <int NBK, int C, int LB_NCB>
@@ -102,9 +223,7 @@ lu_block_kernel(int nbw, Blocks bl, const zd *S, zd *Sinv, float *Sinv32, long l
 
         int pos = prow;                          // position of this lane's panel row
 
-        // The steps of panel p on the columns in G[p & 1].  The row rotates by one
-        // register per step, so that the current column is always a[0] and the
-        // step is one loop body with static register indices.
+        // the steps of panel p on the columns in G[p & 1], in place
         auto factor = [&](int p) {
             zd (*G)[LDG] = sh.G[p & 1];
             zd a[8];
@@ -112,66 +231,15 @@ lu_block_kernel(int nbw, Blocks bl, const zd *S, zd *Sinv, float *Sinv32, long l
 #pragma unroll
             for (int c = 0; c < 8; ++c) a[c] = prow < Ns ? G[c][prow] : make_double2(0.0, 0.0);
             int myslot = -1;
-            const int steps = min(8, Ns - 8 * p);
-#pragma unroll 1
-            for (int c = 0; c < steps; ++c) {
-                const int k = 8 * p + c;
-                const unsigned u = lb_rank(a[0], pos, prow < Ns && pos >= k);
-                unsigned best = __reduce_max_sync(0xffffffffu, u);
-                double d;
-                const zd qr = lb_rcp(a[0], d);
-                zd *cw = sh.crow[c & 1][pwarp];
-                if (u == best && u != 0) {
-                    cw[0] = (d > 1e-280 && d < 1e280) ? qr : lb_rcp_any(a[0]);
+            const int steps = min(8, Ns - 8 * p), pos0 = pos;
+            bool tied = false;
+            lb_steps<false>(sh, peer, p, Ns, pw, prow, a, pos, myslot, tied);
+            if (LB_NCB == 8 && bar_any(1, 32 * pw, tied)) {
+                LbRow row = lb_again(sh, peer, p, Ns, pw, prow, pos0);
 #pragma unroll
-                    for (int j = 1; j < 8; ++j) cw[j] = a[j];
-                    cw[8] = a[0];
-                }
-                const zd *pr = sh.crow[c & 1][0];
-                if (pw > 1) {
-                    if (lane == 0) ((unsigned *)&sh.rank[c & 1])[pwarp] = best;
-                    bar_sync(1, 32 * pw);
-                    const int4 v = sh.rank[c & 1];
-                    const unsigned t[4] = {(unsigned)v.x, (unsigned)v.y, pw > 2 ? (unsigned)v.z : 0u,
-                                           pw > 3 ? (unsigned)v.w : 0u};
-                    int bw = 0;
-                    best = t[0];
-#pragma unroll
-                    for (int q = 1; q < 2 * C; ++q)
-                        if (t[q] > best) { best = t[q]; bw = q; }
-                    pr = sh.crow[c & 1][bw];
-                } else {
-                    __syncwarp();
-                }
-                const int key = 127 - (int)(best & 127u);   // the pivot's position
-                const zd q = pr[0];
-                if (pwarp == 0 && lane == 0) {
-                    const zd a0 = pr[8];
-                    sh.piv[k] = a0;
-                    sh.pv[k] = key;
-                    if (zeq0(a0)) {
-                        sh.sing = 1;
-                        if constexpr (C > 1) peer->sing = 1;
-                    }
-                }
-                const bool isP = pos == key;
-                if (pos == k) pos = key;
-                if (isP) {
-                    pos = k;
-                    myslot = c;
-                    sh.rowOf[k] = prow;
-                    if constexpr (C > 1) peer->rowOf[k] = prow;
-                }
-                // the pivot row becomes q times itself, the others lose f times it
-                const zd f = isP ? zneg(q) : zmul(a[0], q);
-#pragma unroll
-                for (int j = 1; j < 8; ++j) {
-                    const zd pj = pr[j];
-                    const zd base = isP ? make_double2(0.0, 0.0) : a[j];
-                    a[j - 1].x = fma(-f.x, pj.x, fma(f.y, pj.y, base.x));
-                    a[j - 1].y = fma(-f.x, pj.y, fma(-f.y, pj.x, base.y));
-                }
-                a[7] = zneg(f);
+                for (int c = 0; c < 8; ++c) a[c] = row.a[c];
+                pos = row.pos;
+                myslot = row.slot;
             }
             if (prow < Ns) {
 #pragma unroll
@@ -224,9 +292,11 @@ lu_block_kernel(int nbw, Blocks bl, const zd *S, zd *Sinv, float *Sinv32, long l
                 // update runs
                 double ln = 0.0;
                 zd ph = make_double2(1.0, 0.0);
+                bool zero = false;
                 const int k1 = min(Ns, 8 * (jb0 + ncb));
                 for (int k = 8 * jb0 + lane; k < k1; k += 32) {
                     const zd d = sh.piv[k];
+                    zero = zero || zeq0(d);
                     const double ad = zabs(d);
                     ln += log(ad);
                     zd t = make_double2(d.x / ad, d.y / ad);
@@ -242,6 +312,10 @@ lu_block_kernel(int nbw, Blocks bl, const zd *S, zd *Sinv, float *Sinv32, long l
                     ph = zmul(ph, t);
                 }
                 if (lane == 0) { sh.ln = ln; sh.ph = ph; }
+                if (zero) {
+                    sh.sing = 1;
+                    if constexpr (C > 1) peer->sing = 1;
+                }
             }
             sync_all();
             if (inv)

@@ -6,13 +6,39 @@
 
 // A 32-bit rank for the pivot search, one warp reduction wide: the leading 25
 // bits of |re| + |im| (11 of exponent, 14 of mantissa; NaN ranks as infinity),
-// then the lower position.  The chosen pivot is within 2^-14 of zgetf2's, which
-// changes neither the bound on the growth nor any result beyond rounding.
-// Ineligible rows rank 0.
+// then the lower position.  Ineligible rows rank 0.  Where a row ties with the
+// chosen one in the leading bits (lb_rival), which the kernels test beside other
+// work, the choice is made again by all 64 bits (lb_exact).
 __device__ __forceinline__ unsigned lb_rank(zd a, int pos, bool eligible)
 {
     const unsigned hi = min((unsigned)__double2hiint(zcabs1(a)) & 0x7fffffffu, 0x7ff00000u);   // a NaN as infinity
     return eligible ? (((hi >> 6) + 1u) << 7) | (unsigned)(127 - pos) : 0u;
+}
+
+__device__ __forceinline__ bool lb_tied(unsigned u, unsigned v) { return (u >> 7) == (v >> 7); }
+// Whether a row of rank u ties with the chosen one of rank `best` (and is not it).
+__device__ __forceinline__ bool lb_rival(unsigned u, unsigned best) { return (u ^ best) - 1u < 127u; }
+
+// The bits of |re| + |im|, monotonic in the value; NaN as infinity.
+__device__ __forceinline__ unsigned long long lb_bits(zd a)
+{
+    const unsigned long long v = (unsigned long long)__double_as_longlong(zcabs1(a));
+    return min(v, 0x7ff0000000000000ull);
+}
+
+// The rank of the warp's pivot among the ties with `best` by zgetf2's rule: the
+// first position of the largest |re| + |im|.  u: this lane's lb_rank of a.
+__device__ __forceinline__ unsigned lb_exact(zd a, unsigned u, unsigned best)
+{
+    const unsigned long long v = lb_bits(a);
+    bool in = lb_tied(u, best);
+    const unsigned hi = in ? (unsigned)(v >> 32) : 0u;
+    const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
+    in = in && hi == mhi;
+    const unsigned lo = in ? (unsigned)v : 0u;
+    const unsigned mlo = __reduce_max_sync(0xffffffffu, lo);
+    in = in && lo == mlo;
+    return __reduce_max_sync(0xffffffffu, in ? u : 0u);
 }
 
 // 1 / b: conj(b) / |b|^2 with the reciprocal of d = |b|^2 from the hardware's

@@ -444,7 +444,7 @@ gj_cta_kernel(int W, Blocks bl, const zd *S, zd *Sinv, const int *active, const 
 // column loop is not unrolled; instead every row rotates by one slot per
 // step, so the current column is always register slot 0 and every register
 // index is static.
-//   - pivot: zgetf2's choice, first position >= k of maximal |re|+|im| in the
+//   - pivot: zgetf2's choice (lb_rank, lb_exact), first position >= k of maximal |re|+|im| in the
 //     column; rows are not moved, each lane keeps the position its row has in
 //     the interchanged matrix (ties go to the lower position, as in izamax);
 //   - the chosen row is published in shared memory (a broadcast source);
@@ -545,7 +545,8 @@ gj_regw_kernel(int W, Blocks bl, const zd *S, zd *Sinv, float *Sinv32, long long
         if (ch == 0) {
             colS[0][r] = a[0];
             const unsigned u = lb_rank(a[0], pos, r < Ns);
-            const unsigned best = __reduce_max_sync(0xffffffffu, u);
+            unsigned best = __reduce_max_sync(0xffffffffu, u);
+            if (__any_sync(0xffffffffu, lb_rival(u, best))) best = lb_exact(a[0], u, best);
             if (u != 0 && u == best) {
                 cand[0] = {pos, r, a[0], lb_rcp_any(a[0])};
 #pragma unroll
@@ -582,8 +583,8 @@ gj_regw_kernel(int W, Blocks bl, const zd *S, zd *Sinv, float *Sinv32, long long
                 // one straight-line block the compiler can interleave)
                 colS[pb][r] = a[0];
                 const unsigned u = lb_rank(a[0], pos, r < Ns && pos > k);
-                const unsigned best = __reduce_max_sync(0xffffffffu, u);
-                const bool win = u != 0 && u == best;
+                unsigned best = __reduce_max_sync(0xffffffffu, u);
+                const bool tied = __any_sync(0xffffffffu, lb_rival(u, best));
                 double d;
                 const zd qr = lb_rcp(a[0], d);
 #pragma unroll
@@ -592,7 +593,8 @@ gj_regw_kernel(int W, Blocks bl, const zd *S, zd *Sinv, float *Sinv32, long long
                     a[s - 1].x = fma(-f.x, pv.x, fma(f.y, pv.y, a[s].x));
                     a[s - 1].y = fma(-f.x, pv.y, fma(-f.y, pv.x, a[s].y));
                 }
-                if (win) {
+                if (tied) best = lb_exact(a[0], u, best);
+                if (u != 0 && u == best) {
                     GR64Cand &c = cand[pb];
                     c.key = pos; c.row = r; c.a0 = a[0];
                     c.q = (d > 1e-280 && d < 1e280) ? qr : lb_rcp_any(a[0]);
