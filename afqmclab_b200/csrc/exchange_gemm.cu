@@ -16,12 +16,16 @@
 //   Z = V U^T (K x 2W), ex_w = sum_q u_w(q) Z_w(q)           (energy)
 //   M_re, M_im = [den u]^T-weighted outer products over walkers (K x K)
 //   Y_g = [R_re | R_im]^T x_g (2K per vector), exNum_g = sum_q x_g(q) Y_g(q)
-// Both are quadratic forms of symmetric matrices, so the 256-blocks right of
-// the diagonal are left out of all three products and the ones left of it count
-// twice (doubled in the stored V and R, exact in bf16): for K = 4096, W = 2048,
-// G = 640 about 0.12 T multiply-adds per spin instead of 0.23 T for the full
-// products and 0.34 T for the blockwise form.  Exchange phase of n = 128, 32
-// electrons: 0.483 -> 0.309 ms.
+// V is symmetric to the bit, so the 256-blocks right of its diagonal are left
+// out of Z and the ones left of it count twice (doubled in the stored V, exact in
+// bf16): for K = 4096, W = 2048, G = 640 about 0.19 T multiply-adds per spin
+// instead of 0.23 T for the full products and 0.34 T for the blockwise form.  The
+// fp32 sums are half as long and their error falls (mean of ex_w 1.6e-5 ->
+// 1.1e-5 at n = 128, 32 electrons); exchange phase there 0.483 -> 0.436 ms.
+// R is not symmetric: den u is rounded to bf16 on one side of M only, and both
+// sides of the diagonal enter.  One side doubled took 0.309 ms, but made the sums
+// per vector depend on the electrons' order by 1e-4 .. 6e-4 (1e-5 with both) and
+// their error 1 to 12 % larger.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -309,9 +313,6 @@ int exchange_gemm_run(afqmc_engine *e, const ExGemmBlock &blk, const __nv_bfloat
         a.B = s.Bt; a.ldb = W2;
         a.C = s.Rt; a.outType = TC_OUT_BF16; a.err = err;
         a.permN = n; a.permK = K;
-        // whole orbital runs per 256-block: half of M, and of Y's products
-        const int half = 256 % n == 0 ? 1 : 0;
-        a.half = half;
         int r = tc_gemm_bf16(a, st);
         if (r) return engine_fail(AFQMC_ERR_CUDA, "exchange M gemm: " + std::to_string(r));
         TcGemmArgs y;
@@ -319,7 +320,6 @@ int exchange_gemm_run(afqmc_engine *e, const ExGemmBlock &blk, const __nv_bfloat
         y.A = s.Rt; y.lda = K;
         y.B = A2r; y.ldb = K;
         y.C = s.Y; y.ldc = 2 * K; y.outType = TC_OUT_F32; y.err = err;
-        y.quad = half;
         r = tc_gemm_bf16(y, st);
         if (r) return engine_fail(AFQMC_ERR_CUDA, "exchange Y gemm: " + std::to_string(r));
         g_launch_count++;

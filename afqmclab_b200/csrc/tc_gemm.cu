@@ -153,24 +153,14 @@ constexpr int TT_BN = 128, TT_BM = 256, TT_STAGES = 4, TT_THREADS = 320;
 constexpr int TT_A_BYTES = TT_BM * TC_BK * 2, TT_B_BYTES = TT_BN * TC_BK * 2;
 constexpr size_t TT_SMEM = 1024 + (size_t)TT_STAGES * (TT_A_BYTES + TT_B_BYTES) + 256;
 
-// Tile orders: TT_ALL every tile of every split; TT_QUAD the row blocks of a
-// quadratic form (TcGemmArgs::quad), the longest contractions first and every
-// second round of CTAs reversed, so that each CTA's sum is about the same;
-// TT_HALF the tiles up to the diagonal block (TcGemmArgs::half).
-enum { TT_ALL = 0, TT_QUAD = 1, TT_HALF = 2 };
-
-__host__ __device__ inline long long tt_tiles(int order, int M, int N, int K, int splits)
-{
-    const long long MT = (M + TT_BM - 1) / TT_BM, NTn = (N + TT_BN - 1) / TT_BN;
-    if (order == TT_HALF) return M / N * ((long long)(N / TT_BM) * (N / TT_BM + 1));
-    return MT * NTn * splits;
-}
-
+// quad (TcGemmArgs::quad): the row blocks with the longest contractions come
+// first and every second round of CTAs is reversed, so that each CTA's sum is
+// about the same.
 template <int OUT>
 __global__ void __launch_bounds__(TT_THREADS, 1)
 tc_gemm_t_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M,
                  int N, int K, int kSplit, int splits, void *C, long long ldc, long long splitStride,
-                 float alpha, int *err, int permN, long long permK, int order)
+                 float alpha, int *err, int permN, long long permK, int quad)
 {
     constexpr uint32_t IDESC = idesc_bf16(TT_BN, TT_BM);
     extern __shared__ uint8_t smem_raw[];
@@ -185,29 +175,18 @@ tc_gemm_t_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int MT = (M + TT_BM - 1) / TT_BM, NTn = (N + TT_BN - 1) / TT_BN;
-    const int tiles = (int)tt_tiles(order, M, N, K, splits);
+    const int tiles = MT * NTn * splits;
     // this CTA's tile of round i (tiles or more: none)
     auto tile_of = [&](int i) {
-        const int b = order == TT_QUAD && (i & 1) ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
+        const int b = quad && (i & 1) ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
         return i * (int)gridDim.x + b;
     };
     auto tile_kt = [&](int t, int &m0, int &n0, int &k0) {
-        if (order == TT_QUAD) {
-            const int planes = M / K, per = planes * NTn, r = t % per;
-            const int i0 = K - TT_BM * (1 + t / per);
-            m0 = (r / NTn) * K + i0;
-            n0 = (r % NTn) * TT_BN;
+        if (quad) {
+            m0 = K - TT_BM * (1 + t / NTn);
+            n0 = (t % NTn) * TT_BN;
             k0 = 0;
-            return (i0 + TT_BM) / TC_BK;
-        }
-        if (order == TT_HALF) {
-            const int nb = N / TT_BM, per = nb * (nb + 1), r = t % per;
-            int i = 0;
-            while ((i + 1) * (i + 2) <= r) ++i;
-            m0 = (t / per) * N + i * TT_BM;
-            n0 = (r - i * (i + 1)) * TT_BN;
-            k0 = 0;
-            return (K + TC_BK - 1) / TC_BK;
+            return (m0 + TT_BM) / TC_BK;
         }
         const int z = t / (MT * NTn), r = t - z * (MT * NTn);
         m0 = (r % MT) * TT_BM;
@@ -293,9 +272,7 @@ tc_gemm_t_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             if (!ok) break;
             tc_fence_after();
             const int n = n0 + q * 32 + lane;
-            const size_t colOff = (size_t)(order == TT_ALL ? t / (MT * NTn) : 0) * splitStride + (size_t)n * ldc;
-            // a half product's blocks left of the diagonal count twice
-            const float al = order == TT_HALF && (m0 % N) / TT_BM > n0 / TT_BM ? 2.0f * alpha : alpha;
+            const size_t colOff = (size_t)(t / (MT * NTn)) * splitStride + (size_t)n * ldc;
             const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * TT_BM);
 #pragma unroll 1
             for (int c0 = half * 128; c0 < half * 128 + 128; c0 += 32) {
@@ -322,16 +299,16 @@ tc_gemm_t_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                         for (int j = 0; j < 32; j += 8) {
                             if (mb + j + 8 <= M) {
                                 uint4 pk;
-                                __nv_bfloat162 h0 = __floats2bfloat162_rn(al * v[j], al * v[j + 1]);
-                                __nv_bfloat162 h1 = __floats2bfloat162_rn(al * v[j + 2], al * v[j + 3]);
-                                __nv_bfloat162 h2 = __floats2bfloat162_rn(al * v[j + 4], al * v[j + 5]);
-                                __nv_bfloat162 h3 = __floats2bfloat162_rn(al * v[j + 6], al * v[j + 7]);
+                                __nv_bfloat162 h0 = __floats2bfloat162_rn(alpha * v[j], alpha * v[j + 1]);
+                                __nv_bfloat162 h1 = __floats2bfloat162_rn(alpha * v[j + 2], alpha * v[j + 3]);
+                                __nv_bfloat162 h2 = __floats2bfloat162_rn(alpha * v[j + 4], alpha * v[j + 5]);
+                                __nv_bfloat162 h3 = __floats2bfloat162_rn(alpha * v[j + 6], alpha * v[j + 7]);
                                 pk.x = *(uint32_t *)&h0; pk.y = *(uint32_t *)&h1;
                                 pk.z = *(uint32_t *)&h2; pk.w = *(uint32_t *)&h3;
                                 *(uint4 *)(dst + j) = pk;
                             } else {
                                 for (int u = 0; u < 8; ++u)
-                                    if (mb + j + u < M) dst[j + u] = __float2bfloat16_rn(al * v[j + u]);
+                                    if (mb + j + u < M) dst[j + u] = __float2bfloat16_rn(alpha * v[j + u]);
                             }
                         }
                     } else {
@@ -340,10 +317,10 @@ tc_gemm_t_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                         for (int j = 0; j < 32; j += 4) {
                             if (mb + j + 4 <= M) {
                                 *(float4 *)(dst + j) =
-                                    make_float4(al * v[j], al * v[j + 1], al * v[j + 2], al * v[j + 3]);
+                                    make_float4(alpha * v[j], alpha * v[j + 1], alpha * v[j + 2], alpha * v[j + 3]);
                             } else {
                                 for (int u = 0; u < 4; ++u)
-                                    if (mb + j + u < M) dst[j + u] = al * v[j + u];
+                                    if (mb + j + u < M) dst[j + u] = alpha * v[j + u];
                             }
                         }
                     }
@@ -411,14 +388,13 @@ int launch_t(const TcGemmArgs &a, cudaStream_t s)
     const int splits = a.splits > 1 ? a.splits : 1;
     int kSplit = a.K;
     if (splits > 1) kSplit = ((a.K + splits - 1) / splits + TC_BK - 1) / TC_BK * TC_BK;
-    const int order = a.half ? TT_HALF : a.quad ? TT_QUAD : TT_ALL;
-    const long long tiles = tt_tiles(order, a.M, a.N, a.K, splits);
+    const long long tiles = (long long)((a.M + TT_BM - 1) / TT_BM) * ((a.N + TT_BN - 1) / TT_BN) * splits;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int grid = (int)std::min<long long>(tiles, sms);
     tc_gemm_t_kernel<OUT><<<grid, TT_THREADS, TT_SMEM, s>>>(ma, mb, a.M, a.N, a.K, kSplit, splits, a.C, a.ldc,
-                                                            a.splitStride, a.alpha, a.err, a.permN, a.permK, order);
+                                                            a.splitStride, a.alpha, a.err, a.permN, a.permK, a.quad);
     return (int)cudaGetLastError();
 }
 
@@ -448,14 +424,13 @@ int tc_gemm_bf16(const TcGemmArgs &a, cudaStream_t s)
         // exchanged bf16 store of the persistent form: M = 2 permK, N = permK,
         // 32-row runs inside one orbital run, 16-byte aligned destinations
         if (a.outType != TC_OUT_BF16 || a.splits > 1 || a.permN % 32 != 0 || a.permK % TT_BM != 0 ||
-            a.permK % a.permN != 0 || a.M != 2 * a.permK || a.N != a.permK || ((uintptr_t)a.C % 16) != 0 ||
-            (a.half && TT_BM % a.permN != 0))
+            a.permK % a.permN != 0 || a.M != 2 * a.permK || a.N != a.permK || ((uintptr_t)a.C % 16) != 0)
             return (int)cudaErrorInvalidValue;
         return launch_t<TC_OUT_BF16>(a, s);
     }
     if (a.quad) {
         // fp32 column stores of the persistent form; whole 256-blocks
-        if (a.outType != TC_OUT_F32 || a.splits > 1 || a.K % TT_BM != 0 || a.M % a.K != 0 || ((uintptr_t)a.C % 16) != 0 ||
+        if (a.outType != TC_OUT_F32 || a.splits > 1 || a.K % TT_BM != 0 || a.M != a.K || ((uintptr_t)a.C % 16) != 0 ||
             a.ldc % 4 != 0)
             return (int)cudaErrorInvalidValue;
         return launch_t<TC_OUT_F32>(a, s);

@@ -22,15 +22,11 @@ struct TcGemmArgs {
     // M = 2 permK, N = permK, element (p permK + i + n b, j + n a) goes to
     // C[(p permK + j + n b) permK + i + n a] (ldc unused)
     int permN = 0; long long permK = 0;
-    // Quadratic forms x^T R x of a symmetric R (persistent form only), in blocks
-    // of 256: the blocks right of the diagonal are left out and the blocks left
-    // of it count twice, half the products.
-    // quad: A holds M / K planes of such an R (K x K, K a multiple of 256, the
-    //   doubling done in its stored values) and a row block takes the columns
-    //   up to its diagonal block;
-    // half: with the exchanged store, where permN divides 256: the blocks right
-    //   of the diagonal are not computed and the ones left of it are stored doubled
-    int quad = 0, half = 0;
+    // Quadratic form x^T A x of a symmetric A (M = K, a multiple of 256; persistent
+    // form only), in blocks of 256: a row block takes the columns up to its
+    // diagonal block, half the products; the blocks left of the diagonal count
+    // twice by A's stored values.
+    int quad = 0;
 };
 
 // Returns 0 on success, a cudaError_t / CUresult value otherwise.

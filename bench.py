@@ -191,11 +191,13 @@ def phase_flops(c, m, taylor_avg, precision):
         f["taylor"] += f.pop("onebody")
         f["mbuild"] *= (n + 8.0) / (2.0 * n)
     # with real A the exchange runs as three GEMMs per spin block of
-    # Kb = Ns n, each half of a full one by symmetry: Z = V U^T (Kb^2 2W),
-    # [M_re; M_im] = [Ar; Ai] Bt^T (2Kb Kb 2W) and Y = Rt X^T (2Kb G Kb); the flops
-    # counted are those executed, fewer than the blockwise tr(DD) count above
+    # Kb = Ns n: Z = V U^T (Kb^2 2W), [M_re; M_im] = [Ar; Ai] Bt^T (2Kb Kb 2W) and
+    # Y = Rt X^T (2Kb G Kb).  By symmetry half of each is executed in FP64, half of Z
+    # in the mixed form; the flops counted are those executed, fewer than the
+    # blockwise tr(DD) count above
     if real_a and n % 32 == 0 and W % 4 == 0 and all((ns * n) % 256 == 0 for ns in blocks):
-        f["exchange"] = sum((ns * n) ** 2 * (6.0 * W + 2.0 * G) for ns in blocks)
+        per = 10.0 * W + 4.0 * G if precision == "mixed" else 6.0 * W + 2.0 * G
+        f["exchange"] = sum((ns * n) ** 2 * per for ns in blocks)
     return f
 
 
