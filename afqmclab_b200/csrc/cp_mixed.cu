@@ -904,6 +904,13 @@ int cp_mixed_project_dtk_dtv(afqmc_engine *e)
         const int L = e->L;
         const size_t smem = sizeof(float2) * 4 * L + sizeof(int) * (L + (L & 1)) + sizeof(double) * L + sizeof(zd) * L;
         g_launch_count++;
+        // all 48 KB of the launch for the lattice (818 sites), beside the kernel's own
+        // shared variables
+        static std::atomic<unsigned long long> attr{0};
+        const cudaError_t ar = each_device_once(attr, [] {
+            return cudaFuncSetAttribute(cpm_sample_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024);
+        });
+        if (ar != cudaSuccess) return engine_fail(AFQMC_ERR_CUDA, cudaGetErrorString(ar));
         cpm_sample_apply_kernel<<<W, 256, smem, s>>>(W, e->hd, m->gd, e->surv, rng, e->seed, m->hi, m->lo,
                                                      m->thi, m->tlo, e->logw, e->dt * e->ET,
                                                      engine_one_body_logw(e, 0), nullptr);

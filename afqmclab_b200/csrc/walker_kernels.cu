@@ -1841,6 +1841,14 @@ void launch_cp_sample_apply(int W, const HubbardDev &h, const zd *thetaT, long l
 {
     g_launch_count++;
     size_t smem = (size_t)4 * h.L * sizeof(zd) + (size_t)(h.L + 1) * sizeof(int) + (size_t)h.L * sizeof(double) + 16;
+    // all 48 KB of the launch for the lattice (646 sites), beside the kernel's own
+    // shared variables
+    static std::atomic<unsigned long long> attr{0};
+    const cudaError_t r = each_device_once(attr, [] {
+        const cudaError_t a = cudaFuncSetAttribute(cp_sample_apply_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024);
+        return a != cudaSuccess ? a : cudaFuncSetAttribute(cp_sample_apply_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024);
+    });
+    if (r != cudaSuccess) return;   // the launch check reports it
     if (diag)
         cp_sample_apply_kernel<false><<<W, 256, smem, s>>>(W, h, thetaT, tStride, surv, rng, seed, wf, wfTmp, diag, logw,
                                                            dtET, hopLogw, auxOut);
