@@ -1172,6 +1172,28 @@ __global__ void any_imag_kernel(long long count, const zd *A, int *flag)
     if (__syncthreads_or(any) && threadIdx.x == 0) atomicOr(flag, 1);
 }
 
+namespace {
+
+// exp(+dt/2 K) of the measurement's half step on the tensor cores, from its FP64
+// form
+int load_half_step(afqmc_engine *e)
+{
+    MixedState *m = e->mx;
+    std::vector<zd> E1((size_t)e->n * e->n);
+    MTRY(engine_read(e, E1.data(), e->expK[1], sizeof(zd) * E1.size()));
+    std::vector<float> eh, el;
+    if (tf32_split_operator(E1.data(), e->n, eh, el))
+        return engine_fail(AFQMC_ERR_UNSUPPORTED, "mixed precision one-body needs a real exp(dt/2 K)");
+    if (!m->E1h) {
+        MTRY(engine_dalloc(e, &m->E1h, eh.size()));
+        MTRY(engine_dalloc(e, &m->E1l, el.size()));
+    }
+    MTRY(engine_write(e, m->E1h, eh.data(), 4 * eh.size()));
+    return engine_write(e, m->E1l, el.data(), 4 * el.size());
+}
+
+}  // namespace
+
 int mixed_create(afqmc_engine *e)
 {
     if (e->kind == KIND_CP) return cp_mixed_create(e);
@@ -1256,20 +1278,9 @@ int mixed_create(afqmc_engine *e)
     MTRY(cuda_check(cudaStreamSynchronize(e->stream), "sync"));
     for (const zd &v : h)
         if (v.y != 0.0) return engine_fail(AFQMC_ERR_UNSUPPORTED, "mixed precision one-body needs a real exp(-dt K)");
-    // exp(+dt/2 K) of the measurement's half step on the tensor cores
-    {
-        std::vector<zd> E1((size_t)n * n);
-        MTRY(engine_read(e, E1.data(), e->expK[1], sizeof(zd) * E1.size()));
-        std::vector<float> eh, el;
-        if (tf32_split_operator(E1.data(), n, eh, el))
-            return engine_fail(AFQMC_ERR_UNSUPPORTED, "mixed precision one-body needs a real exp(dt/2 K)");
-        MTRY(engine_dalloc(e, &m->E1h, eh.size()));
-        MTRY(engine_dalloc(e, &m->E1l, el.size()));
-        MTRY(engine_write(e, m->E1h, eh.data(), 4 * eh.size()));
-        MTRY(engine_write(e, m->E1l, el.data(), 4 * el.size()));
-        MTRY(engine_dalloc(e, &m->sh, (size_t)W * m->ws32));
-        MTRY(engine_dalloc(e, &m->sl, (size_t)W * m->ws32));
-    }
+    MTRY(load_half_step(e));
+    MTRY(engine_dalloc(e, &m->sh, (size_t)W * m->ws32));
+    MTRY(engine_dalloc(e, &m->sl, (size_t)W * m->ws32));
     // S^{-1} of the theta product, fp32 planes written by the LU
     MTRY(engine_dalloc(e, &m->Sinv32, (size_t)W * sinv32_stride(e->bl)));
     for (int b = 0; b < e->bl.nblk; ++b)
@@ -1320,7 +1331,8 @@ int mixed_update_operators(afqmc_engine *e)
 {
     if (e->kind == KIND_CP) return AFQMC_OK;
     build_et_kernel<<<64, 256, 0, e->stream>>>(e->n, e->expK[0], e->mx->Et);
-    return engine_check_launch();
+    MTRY(engine_check_launch());
+    return load_half_step(e);
 }
 
 int mixed_sync_to_fp64(afqmc_engine *e)
