@@ -16,8 +16,6 @@ namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int LU_SMEM_MAX_NS = 64;
-
 // ---------------------------------------------------------------------------
 // LU with partial pivoting + log-determinant (+ inverse) of every overlap
 // block of a walker; one CTA per walker.
@@ -29,20 +27,18 @@ constexpr int LU_SMEM_MAX_NS = 64;
 // The first cos projection of the driver step
 // (afqmcConstraintPathProjection.cpp:45-48, afqmcPhaselessProjection.cpp:85-88)
 // and the population-control weights (afqmcConstraintPathProjection.cpp:108-122)
-// are fused into the epilogue.
+// are fused into the epilogue.  One block of more than 128 columns, or two with one
+// above 120: the matrix is factored where it lies, in device memory.
 // ---------------------------------------------------------------------------
-template <bool SMEM>
 __global__ void __launch_bounds__(256)
 lu_kernel(int W, Blocks bl, zd *S, zd *Sinv, const int *active, const zd *logw, zd logwAdd,
           zd logwT, zd *logov, int *alive, int *surv, zd *logwOut, double *weight, int *status,
-          int mode, int wantInverse, int maxNs)
+          int mode, int wantInverse)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int w = blockIdx.x;
     const int tid = threadIdx.x, nt = blockDim.x;
-    zd *sA = (zd *)smem_raw;
-    zd *sX = sA + (SMEM ? maxNs * maxNs : 0);
-    int *piv = (int *)(sX + (SMEM ? maxNs * maxNs : 0));
+    int *piv = (int *)smem_raw;
     __shared__ int sFlag, sBlk;   // singular anywhere / in the current block
 
     const bool act = (active == nullptr) || active[w] != 0;
@@ -59,12 +55,8 @@ lu_kernel(int W, Blocks bl, zd *S, zd *Sinv, const int *active, const zd *logw, 
     for (int b = 0; b < bl.nblk; ++b) {
         const int Ns = bl.Ns[b];
         if (Ns == 0) continue;
-        zd *Sg = S + (size_t)w * bl.sStride + bl.sOff[b];
-        zd *Xg = Sinv ? Sinv + (size_t)w * bl.sStride + bl.sOff[b] : nullptr;
-        zd *A = SMEM ? sA : Sg;
-        zd *X = SMEM ? sX : Xg;
-        if (SMEM)
-            for (int e = tid; e < Ns * Ns; e += nt) A[e] = Sg[e];
+        zd *A = S + (size_t)w * bl.sStride + bl.sOff[b];
+        zd *X = Sinv ? Sinv + (size_t)w * bl.sStride + bl.sOff[b] : nullptr;
         if (tid == 0) sBlk = 0;
         __syncthreads();
         for (int j = 0; j < Ns; ++j) {
@@ -132,7 +124,7 @@ lu_kernel(int W, Blocks bl, zd *S, zd *Sinv, const int *active, const zd *logw, 
             }
         }
         // inverse: X = A^{-1} column by column (P, unit-L forward, U backward)
-        if (wantInverse && Xg) {
+        if (wantInverse && X) {
             for (int c = tid; c < Ns; c += nt) {
                 zd *x = X + (size_t)c * Ns;
                 for (int i = 0; i < Ns; ++i) x[i] = make_double2(i == c ? 1.0 : 0.0, 0.0);
@@ -159,9 +151,6 @@ lu_kernel(int W, Blocks bl, zd *S, zd *Sinv, const int *active, const zd *logw, 
                     x[i] = zdiv(s, A[i + (size_t)i * Ns]);
                 }
             }
-            __syncthreads();
-            if (SMEM)
-                for (int e = tid; e < Ns * Ns; e += nt) Xg[e] = X[e];
         }
         __syncthreads();
     }
@@ -199,7 +188,8 @@ lu_kernel(int W, Blocks bl, zd *S, zd *Sinv, const int *active, const zd *logw, 
 }
 
 // ---------------------------------------------------------------------------
-// Same contract as lu_kernel for blocks of 33..GJ_CTA_MAX_NS columns, one CTA
+// Same contract as lu_kernel for two blocks of which one has more than 64 and none
+// more than GJ_CTA_MAX_NS columns (lu_block.cu takes the smaller ones), one CTA
 // per walker, the block resident in shared memory (column-major, as in S).
 // Warp w owns the columns c = w (mod warps); lane l holds rows l, l+32, ...
 // With the inverse requested: Gauss-Jordan elimination in place (zgetf2 pivot
@@ -438,7 +428,8 @@ gj_cta_kernel(int W, Blocks bl, const zd *S, zd *Sinv, const int *active, const 
 
 // ---------------------------------------------------------------------------
 // Gauss-Jordan with the matrix in registers (gj_regw_kernel below), same
-// contract as lu_kernel for one or two blocks of 17..32 columns: each
+// contract as lu_kernel for one or two blocks of up to 32 columns, used for 25
+// to 32 and more than 888 matrices (lu_regw_faster): each
 // row lives in registers (padded with zeros to the window; only Ns steps
 // run, after which the last Ns window slots hold the inverse columns).  The
 // column loop is not unrolled; instead every row rotates by one slot per
@@ -1779,7 +1770,7 @@ void launch_lu_logdet_inverse32(int W, const Blocks &bl, zd *S, zd *Sinv, float 
                  weight, status, mode, wantInverse, s);
         return;
     }
-    if (maxNs > 16 && maxNs <= 32) {
+    if (maxNs <= 32) {
         g_launch_count++;
         launch_regw(W, bl, S, Sinv32 ? nullptr : Sinv, Sinv32, s32, active, logw, logwAdd, logwT, logov, alive, surv,
                     logwOut, weight, status, mode, wantInverse ? 1 : 0, s);
@@ -1811,21 +1802,9 @@ static void launch_lu_fp64(int W, const Blocks &bl, zd *S, zd *Sinv, const int *
                                                     logwOut, weight, status, mode, wantInverse ? 1 : 0, maxNs);
         return;
     }
-    if (maxNs <= LU_SMEM_MAX_NS) {
-        size_t smem = (size_t)2 * maxNs * maxNs * sizeof(zd) + (size_t)(maxNs + 4) * sizeof(int);
-        static std::atomic<unsigned long long> attr{0};
-        if (first_on_device(attr)) {
-            cudaFuncSetAttribute(lu_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-        }
-        lu_kernel<true><<<W, 256, smem, s>>>(W, bl, S, Sinv, active, logw, logwAdd, logwT, logov,
-                                              alive, surv, logwOut, weight, status, mode,
-                                              wantInverse ? 1 : 0, maxNs);
-    } else {
-        size_t smem = (size_t)(maxNs + 4) * sizeof(int);
-        lu_kernel<false><<<W, 256, smem, s>>>(W, bl, S, Sinv, active, logw, logwAdd, logwT, logov,
-                                               alive, surv, logwOut, weight, status, mode,
-                                               wantInverse ? 1 : 0, maxNs);
-    }
+    const size_t smem = (size_t)maxNs * sizeof(int);
+    lu_kernel<<<W, 256, smem, s>>>(W, bl, S, Sinv, active, logw, logwAdd, logwT, logov, alive, surv, logwOut, weight,
+                                   status, mode, wantInverse ? 1 : 0);
 }
 
 void launch_rng_scan(int W, const int *surv, int draws, unsigned long long *counter,
