@@ -16,6 +16,14 @@ namespace cg = cooperative_groups;
 
 namespace {
 
+// |re| + |im| of a pivot candidate; a NaN as infinity, so that a column of NaN still
+// has a pivot row
+__device__ __forceinline__ double pivot_size(zd a)
+{
+    const double v = zcabs1(a);
+    return v == v ? v : INFINITY;
+}
+
 // ---------------------------------------------------------------------------
 // LU with partial pivoting + log-determinant (+ inverse) of every overlap
 // block of a walker; one CTA per walker.
@@ -63,7 +71,7 @@ lu_kernel(int W, Blocks bl, zd *S, zd *Sinv, const int *active, const zd *logw, 
             if (tid < 32) {
                 double best = -1.0; int bi = Ns;
                 for (int i = j + tid; i < Ns; i += 32) {
-                    double v = zcabs1(A[i + (size_t)j * Ns]);
+                    const double v = pivot_size(A[i + (size_t)j * Ns]);
                     if (v > best) { best = v; bi = i; }
                 }
                 for (int o = 16; o > 0; o >>= 1) {
@@ -228,7 +236,7 @@ __device__ __forceinline__ void gj_cta_pivot(const zd *A, int Ns, int j, int lan
     for (int r = 0; r < RPL; ++r) {
         const int i = lane + 32 * r;
         if (i >= j && i < Ns) {
-            const double v = zcabs1(A[i + (size_t)Ns * j]);
+            const double v = pivot_size(A[i + (size_t)Ns * j]);
             if (v > best) { best = v; bi = i; }
         }
     }
