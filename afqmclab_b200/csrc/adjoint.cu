@@ -247,7 +247,11 @@ struct DevBufs {
             if (s.p) cudaFree(s.p);
             s = {nullptr, 0};
             cudaError_t c = cudaMalloc(&s.p, bytes);
-            if (c != cudaSuccess) { s.p = nullptr; return c; }
+            if (c != cudaSuccess) {
+                cudaGetLastError();   // reported here: the next launch check must not see it
+                s.p = nullptr;
+                return c;
+            }
             s.bytes = bytes;
         }
         ++next;
@@ -259,6 +263,7 @@ struct DevBufs {
         *out = nullptr;
         cudaError_t c = cudaMalloc((void **)out, sizeof(T) * std::max<size_t>(count, 1));
         if (c == cudaSuccess) p.push_back((void *)*out);
+        else cudaGetLastError();
         return c;
     }
 };

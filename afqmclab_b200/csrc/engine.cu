@@ -149,8 +149,10 @@ int dalloc(afqmc_engine *e, T **p, size_t count)
     if (count == 0) count = 1;
     void *q = nullptr;
     cudaError_t r = cudaMalloc(&q, count * sizeof(T));
-    if (r != cudaSuccess)
+    if (r != cudaSuccess) {
+        cudaGetLastError();   // reported here: the next launch check must not see it
         return fail(AFQMC_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(r));
+    }
     r = cudaMemsetAsync(q, 0, count * sizeof(T), e->stream);
     if (r != cudaSuccess) {
         cudaFree(q);

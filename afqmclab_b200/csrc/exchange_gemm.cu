@@ -242,7 +242,10 @@ int exchange_gemm_build(afqmc_engine *e, int b, ExGemmBlock &blk)
     blk.tOff = e->bl.tOff[b];
     // C = Aflat Aflat^T over the vectors, Aflat(c, g) = A_g(a, i), c = a + Ns i
     zd *C = nullptr;
-    if (cudaMalloc(&C, sizeof(zd) * K * K) != cudaSuccess) return engine_fail(AFQMC_ERR_CUDA, "exchange setup: alloc");
+    if (cudaMalloc(&C, sizeof(zd) * K * K) != cudaSuccess) {
+        cudaGetLastError();   // reported here: the next launch check must not see it
+        return engine_fail(AFQMC_ERR_CUDA, "exchange setup: alloc");
+    }
     ZGemmArgs g;
     g.m = (int)K; g.n = (int)K; g.k = G;
     g.opA = OP_N; g.opB = OP_T;
