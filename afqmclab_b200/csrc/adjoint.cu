@@ -235,7 +235,8 @@ struct DevBufs {
     explicit DevBufs(afqmc_engine *e_) : e(e_) {}
     ~DevBufs()
     {
-        for (void *q : p) cudaFree(q);   // waits for the work in flight
+        cudaStreamSynchronize(e->stream);   // also where a call ends with an error, work in flight
+        for (void *q : p) cudaFree(q);
     }
     template <class T> cudaError_t get(T **out, size_t count)
     {
