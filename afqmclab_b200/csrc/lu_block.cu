@@ -17,14 +17,14 @@
 // The next panel's column block is updated first, and panel warps of their own
 // factor it while the others finish this update.  The step of the panel is a
 // chain of about 25 dependent operations (a pivot search, a reciprocal, one
-// exchange through shared memory): 515 cycles with two panel warps alone on an
-// SM, about 950 beside the matrix products of two CTAs, which is what bounds
-// the kernel; the products themselves take a third of that.  Hence one warp
-// reduction per search (lb_rank) and the hardware's reciprocal start (lb_rcp);
-// with the compute warps as panel warps the registers spilled and a step took
-// 1200.  Rows that tie in the rank are told apart by all 64 bits: at once where one
-// warp holds the rows, else by one more pass over the panel (lb_again); the test
-// costs nothing up to 64 columns and 3 to 4 % on 80 and 120.
+// exchange through shared memory), which bounds the kernel: for 1024 matrices of 56
+// columns the warps spend half their time at the barriers behind it, the matrix
+// pipe is busy 22 % and the issue slots 28 % of the time.  Hence one warp reduction
+// per search (lb_rank) and the hardware's reciprocal start (lb_rcp); with the
+// compute warps as panel warps the registers spilled.  Rows that tie in the rank
+// are told apart by all 64 bits: at once where one warp holds the rows, else by
+// one more pass over the panel (lb_again); the test costs nothing up to 64 columns
+// and 3 to 4 % on 80 and 120.
 //
 // Against the element-wise kernels it replaces (us per launch, one B200): 14
 // columns, 100 matrices 35 -> 17; 16 columns, 512 matrices 31 -> 17; 56, 1024: 203

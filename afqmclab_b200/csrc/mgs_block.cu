@@ -11,9 +11,9 @@
 // in shared memory up to 40 KB (QS; always for the mixed form, whose columns
 // are rounded to fp32 only on the way out).
 //
-// Bound: instruction issue and latency of the columns' reductions (about 350
-// instructions per column and warp, a third of the issue slots) over the
-// walkers that share an SM, three at n = 128.  Against one column at a time over
+// Bound: instruction issue and latency of the columns' reductions (35 % of the
+// issue slots and 33 % of the matrix pipe busy at 128 x 56) over the walkers that
+// share an SM, three at n = 128.  Against one column at a time over
 // all later ones (us per launch, one B200): 128 x 56, 1024 walkers 568 -> 341; 200 x
 // 80, 1024: 3670 -> 1295; 288 x 120, 1024: 12600 -> 3300; 128 x 32, 2048: 349 -> 252 (fp32
 // walkers 348 -> 306); 256 x 64, 512: 1227 -> 557; 32 x 14, 100: 20 -> 16.

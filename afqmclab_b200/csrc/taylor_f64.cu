@@ -17,13 +17,14 @@
 // Bound: the FP64 matrix rate.  Per order 8 n^2 N flops per walker against
 // n^2 16 bytes of M from L2 (16 bytes per cycle and SM at n = 256, 8 at 128) and
 // 32 bytes per cycle and SM of fragment loads, both far below their limits.
-// Measured, series and one-body product, against one GEMM and one accumulation
-// launch per order up to the cap: n = 128, N = 32, 2048 walkers 7.44 -> 2.49 ms;
-// n = 64, N = 16, 512 walkers 0.761 -> 0.113; n = 90, N = 21, 300 walkers 1.17 ->
-// 0.338; n = 256, N = 64, 512 walkers 7.37 -> 5.59.  From the panels of a
-// symmetric M (and a real one-body operator): 2.49, 0.111, 0.314 and 6.01; the
-// mirrored rows cost loads here, and the M-build that writes them loses half
-// its products (2.87 -> 1.45, 0.117 -> 0.060, 0.123 -> 0.077, 5.68 -> 2.74 ms).
+// Phase times, series and one-body product, one GEMM and one accumulation launch per
+// order up to the cap against this: n = 128, N = 32, 2048 walkers 7.44 and 2.49 ms
+// (23.6 TFLOP/s at a mean order of 6.35, the matrix pipe busy 66 % of the time);
+// n = 64, N = 16, 512 walkers 0.761 and 0.109; n = 90, N = 21, 300 walkers 1.17 and
+// 0.269; n = 256, N = 64, 512 walkers 7.37 and 5.83.  These read the panels of a
+// symmetric M: the mirrored rows cost loads here (n = 256 with a full M 5.59 against
+// 6.01 then), and the M-build that writes the panels has half the products (2.87 ->
+// 1.40, 0.117 -> 0.058, 0.123 -> 0.075, 5.68 -> 2.64 ms).
 #include <cooperative_groups.h>
 #include <math_constants.h>
 

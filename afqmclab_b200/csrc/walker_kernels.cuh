@@ -118,8 +118,9 @@ void launch_taylor_accum(int W, long long wsize, const zd *term, zd *wfNew, cons
 
 // Modified Gram-Schmidt stabilisation (replaces SD::stabilize / SD2is::stabilize)
 // In panels of eight columns (mgs_block.cu); wf is zd (f32 false) or the mixed
-// form's fp32 planes (f32 true).  Returns false (nothing launched) where a
-// walker's rows do not fit one CTA (above 448; fp32: see launch_mgs_block).
+// form's fp32 planes (f32 true).  Returns false (nothing launched) above 512 rows
+// and where the panels and sums do not fit 227 KB of shared memory, which grows
+// with rows and columns (448 x 200 and 512 x 40 do not, 480 x 48 does).
 bool launch_mgs_block(int W, int n, int ncol, int nup, int ndn, int isSD2is, void *wf, bool f32, zd *logw,
                       const int *alive, int *status, cudaStream_t s);
 void launch_mgs(int W, int n, int ncol, int nup, int ndn, int isSD2is, zd *wf, zd *logw,

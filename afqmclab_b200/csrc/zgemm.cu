@@ -4,14 +4,14 @@
 // 33.9 for a bare chain of DFMAs), and its fragments take each operand value
 // from shared memory once per warp: a 32 x 16 complex warp tile reads 3 KB
 // per 512 matrix-pipe cycles, where the register-tiled DFMA form before it was
-// bound by its fragment loads.  One B200, before and after: M-build (16384 x
-// 2048 x 640, real A) 4.14 -> 2.83 ms (30.3 TFLOP/s), exchange of n = 128, 32
-// electrons, 640 vectors and 2048 walkers 17.1 -> 10.7 ms, one-body product
-// of 1024 128 x 56 walkers 0.465 -> 0.27 ms.  Without a branch between the
-// products of a warp whose tile lies inside C, 10 % more: 8704 x 2048 x 640, real A,
-// 1.58 -> 1.45 ms (31.6 TFLOP/s); 4096 x 2048 x 4096, real A, 4.65 -> 4.24 (32.5); 4096
-// x 640 x 4096, real B, 1.67 -> 1.44 (29.9).  The matrix pipe is then busy 85 % of
-// the time; what is left is barriers and the copies' address arithmetic.
+// bound by its fragment loads.  One B200, scalar tiles and the first form of
+// these: M-build (16384 x 2048 x 640, real A) 4.14 and 2.83 ms, one-body product of
+// 1024 128 x 56 walkers 0.465 and 0.27 ms.  Without a branch between the products
+// of a warp whose tile lies inside C, 10 % more.  Now 8704 x 2048 x 640, real A, takes
+// 1.43 ms (31.9 TFLOP/s, the matrix pipe busy 90 % of the time) and the force 640 x
+// 2048 x 4096 0.71 ms (30.2, 89 %); what is left is barriers and the copies' address
+// arithmetic.  Small outputs are bound by their operands too: 32 x 32 x 128, real A,
+// 2048 walkers 0.047 ms (22.8 TFLOP/s, pipe 74 %, 3.1 TB/s).
 #include "zgemm.cuh"
 
 #include <algorithm>
@@ -319,9 +319,9 @@ typedef Tile<32, 32, 16, 16, 8, 4, 4> TileS;
 typedef Tile<64, 32, 32, 16, 8, 4, 3> TileM;
 typedef Tile<64, 64, 32, 16, 16, 3, 2> TileL;
 // The largest for one real operand and a long contraction: half the products per
-// stage leave room for 32 columns of it in two stages, half the barriers (4096
-// x 2048 x 4096, real A, 4.24 -> 4.09 ms; 4096 x 640 x 4096, real B, 1.54 -> 1.48; the
-// complex form loses, 4.21 -> 4.56).
+// stage leave room for 32 columns of it in two stages, half the barriers (TileL
+// and this, in one run: 4096 x 2048 x 4096, real A, 4.24 and 4.09 ms; 4096 x 640 x 4096,
+// real B, 1.54 and 1.48; the complex form loses, 4.21 and 4.56).
 typedef Tile<64, 64, 32, 16, 32, 2, 2> TileLR;
 
 cudaError_t launch_cand(int c, const ZGemmArgs &a, cudaStream_t s)
