@@ -29,6 +29,9 @@
 // Against the element-wise kernels it replaces (us per launch, one B200): 14
 // columns, 100 matrices 35 -> 17; 16 columns, 512 matrices 31 -> 17; 56, 1024: 203
 // -> 183; 64, 512: 131 -> 109; 80, 1024: 1459 -> 822; 120, 1024: 2867 -> 1464.
+// Error against extended precision over random matrices of 4 to 120 columns, the
+// element-wise kernels' as 1 (geometric mean, 120 to 900 matrices a size): inverse
+// 1.03 to 1.2, log-determinant 0.7 to 1.1; both are some N eps.
 #include <cooperative_groups.h>
 
 #include <atomic>
